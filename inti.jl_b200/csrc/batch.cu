@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mrhs_mma(BatchArgs a) {
   constexpr int XPER = MS::XPER;
   static_assert(Sh::MT == 64 && kMmaThreads % Sh::MT == 0 && kMmaJ % (kMmaThreads / Sh::MT) == 0, "shape");
   extern __shared__ __align__(16) double smem_d[];
+  if (a.only_if && !*a.only_if) return;
   double* As = smem_d;
   double* Bs = As + Sh::MT * Sh::LDA;
   double* ssrc = Bs + Sh::kK * Sh::LDB;  // [x y z](J) [n](J) [w](J)
@@ -328,7 +329,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mrhs_mma(BatchArgs a) {
 template <bool CPLX>
 __global__ void csr_mrhs(int64_t m, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                         const double* __restrict__ val, const double* __restrict__ x, int64_t ldx, double* y,
-                        int64_t ldy, int nrhs, double ar, double ai) {
+                        int64_t ldy, int nrhs, double ar, double ai, const int* only_if) {
+  if (only_if && !*only_if) return;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int c = blockIdx.y;
   if (i >= m || c >= nrhs) return;
@@ -515,6 +517,19 @@ static void mrhs_mma_launch(inti_ctx* ctx, int pde, int kind, const BatchArgs& a
   INTI_CUDA(cudaGetLastError());
 }
 
+// The FP64 product of many columns: on the INT8 tensor path where that pays
+// (the correction rows included), with the FP64 MMA kernel standing by for
+// densities that do not fit it; else on the FP64 MMA kernel.
+static void mrhs_fp64(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, const inti_csr* corr, BatchArgs& a,
+                      double pairs, int64_t blocks) {
+  if (fx_pays(p.pde, p.kind, pairs) && fx_prepare(ctx, p, plan, a.nrhs)) {
+    const double alpha[2] = {a.ar, a.ai}, beta[2] = {a.br, a.bi};
+    fx_apply(ctx, p, plan, corr, a.x, a.ldx, a.y, a.ldy, a.nrhs, alpha, beta);
+    a.only_if = fx_flag(ctx);
+  }
+  mrhs_mma_launch(ctx, p.pde, p.kind, a, blocks);
+}
+
 void batch_apply_device(inti_batch* b, int precision, const double* x, int64_t ldx, double* y, int64_t ldy,
                         int32_t nrhs, const double* alpha, const double* beta) {
   inti_ctx* ctx = b->ctx;
@@ -547,7 +562,27 @@ void batch_apply_device(inti_batch* b, int precision, const double* x, int64_t l
     mrhs_tc_launch(b, a);
   } else if (precision == INTI_FP64) {
     ProfScope ps(ctx, "batch");
-    mrhs_mma_launch(ctx, b->pde, b->kind, a, b->nitems);
+    FxProblem p;
+    p.pde = b->pde;
+    p.kind = b->kind;
+    p.k = b->k;
+    for (int q = 0; q < 2; ++q) {
+      p.c1[q] = b->c1[q];
+      p.c2[q] = b->c2[q];
+    }
+    p.tcoords = p.coords = a.coords;
+    p.tnormals = p.normals = a.normals;
+    p.weights = a.weights;
+    double pairs = 0.0;
+    for (size_t s = 0; s + 1 < b->off.size(); ++s) {
+      const int64_t ns = b->off[s + 1] - b->off[s];
+      p.row.push_back(b->off[s]);
+      p.src.push_back(b->off[s]);
+      p.nrow.push_back(ns);
+      p.nsrc.push_back(ns);
+      pairs += (double)ns * (double)ns;
+    }
+    mrhs_fp64(ctx, p, b->fx, b->corr.get(), a, pairs, b->nitems);
   } else {
     throw Error(INTI_E_ARG, "batch precision must be FP64 or TF32");
   }
@@ -557,10 +592,10 @@ void batch_apply_device(inti_batch* b, int precision, const double* x, int64_t l
     dim3 grid((unsigned)((m + 255) / 256), (unsigned)nrhs);
     if (cplx)
       csr_mrhs<true><<<grid, 256, 0, ctx->stream>>>(m, b->corr->rowptr.as<int64_t>(), b->corr->col.as<int32_t>(),
-                                                    b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai);
+                                                    b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     else
       csr_mrhs<false><<<grid, 256, 0, ctx->stream>>>(m, b->corr->rowptr.as<int64_t>(), b->corr->col.as<int32_t>(),
-                                                     b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai);
+                                                     b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     ctx->launches++;
     INTI_CUDA(cudaGetLastError());
   }
@@ -605,17 +640,33 @@ void op_apply_mrhs(inti_op* op, const double* x, int64_t ldx, double* y, int64_t
   const int64_t blocks = (a.gm + kMrhsBlock - 1) / kMrhsBlock;
   {
     ProfScope ps(ctx, "mrhs");
-    mrhs_mma_launch(ctx, op->pde, op->kind, a, blocks);
+    FxProblem p;
+    p.pde = op->pde;
+    p.kind = op->kind;
+    p.k = op->k;
+    for (int q = 0; q < 2; ++q) {
+      p.c1[q] = op->c1[q];
+      p.c2[q] = op->c2[q];
+    }
+    p.tcoords = a.tcoords;
+    p.tnormals = a.tnormals;
+    p.coords = a.coords;
+    p.normals = a.normals;
+    p.weights = a.weights;
+    p.row = p.src = {0};
+    p.nrow = {a.gm};
+    p.nsrc = {a.gn};
+    mrhs_fp64(ctx, p, op->fx, op->corr, a, (double)a.gm * (double)a.gn, blocks);
   }
   if (op->corr) {
     const inti_csr* c = op->corr;
     dim3 grid((unsigned)((a.gm + 255) / 256), (unsigned)nrhs);
     if (cplx)
       csr_mrhs<true><<<grid, 256, 0, ctx->stream>>>(a.gm, c->rowptr.as<int64_t>(), c->col.as<int32_t>(),
-                                                    c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai);
+                                                    c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     else
       csr_mrhs<false><<<grid, 256, 0, ctx->stream>>>(a.gm, c->rowptr.as<int64_t>(), c->col.as<int32_t>(),
-                                                     c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai);
+                                                     c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     ctx->launches++;
     INTI_CUDA(cudaGetLastError());
   }
@@ -632,10 +683,10 @@ void batch_correction_rows(inti_batch* b, const double* x, int64_t ldx, double* 
   const int64_t* rp = b->corr->rowptr.as<int64_t>() + row0;  // entries keep their global positions
   if (cplx)
     csr_mrhs<true><<<grid, 256, 0, ctx->stream>>>(row1 - row0, rp, b->corr->col.as<int32_t>(),
-                                                  b->corr->val.as<double>(), x, ldx, y + 2 * row0, ldy, nrhs, ar, ai);
+                                                  b->corr->val.as<double>(), x, ldx, y + 2 * row0, ldy, nrhs, ar, ai, nullptr);
   else
     csr_mrhs<false><<<grid, 256, 0, ctx->stream>>>(row1 - row0, rp, b->corr->col.as<int32_t>(),
-                                                   b->corr->val.as<double>(), x, ldx, y + row0, ldy, nrhs, ar, ai);
+                                                   b->corr->val.as<double>(), x, ldx, y + row0, ldy, nrhs, ar, ai, nullptr);
   ctx->launches++;
   INTI_CUDA(cudaGetLastError());
 }

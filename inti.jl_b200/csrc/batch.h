@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.h"
+#include "contract_i8.h"
 
 struct inti_batch {
   inti_ctx* ctx = nullptr;
@@ -37,6 +38,7 @@ struct inti_batch {
   }
   int64_t tc_ntiles = 0;
   int tc_nitems = 0;
+  inti::FxPlan fx;  // FP64 products on the INT8 tensor path
 };
 
 namespace inti {
@@ -64,6 +66,7 @@ struct BatchArgs {
   const double* tcoords = nullptr;
   const double* tnormals = nullptr;  // adjoint double layer / hypersingular
   int64_t gm = 0, gn = 0;
+  const int* only_if = nullptr;  // when set, the kernels run only if it is nonzero
 };
 
 void mrhs_tc_launch(inti_batch* b, const BatchArgs& a);

@@ -71,6 +71,41 @@ struct DevBuf {
   }
 };
 
+// One block of up to 128 target rows and the sources they sum over.
+struct FxRows {
+  int64_t row0;    // first target (global)
+  int32_t nrows;   // valid rows
+  int32_t slot0;   // first slot of partial sums, nseg of them
+  int32_t nseg;
+  int32_t surf;
+  int32_t stage0;  // first source stage of the surface
+  int32_t nstages;
+};
+
+// A run of source stages for one row block.
+struct FxItem {
+  int32_t rows, stage, nstages, slot;
+};
+
+// Sources of one stage: src0 .. src0 + count - 1 of surface surf.
+struct FxStage {
+  int64_t src0;
+  int32_t count, surf;
+};
+
+// What a multi-column contraction (contract_i8.h) keeps between calls: work
+// lists, source records and row scales, all functions of the geometry, the
+// kernel and its coefficients.
+struct FxPlan {
+  DevBuf tables, records, tiles, rowscale, meta;
+  const FxRows* rows = nullptr;  // in tables
+  const FxStage* stages = nullptr;
+  const FxItem* items = nullptr;
+  int nrows = 0, nitems = 0, nslots = 0, nstages = 0, nsurf = 0;
+  int64_t ntargets = 0;
+  bool ready = false;
+};
+
 }  // namespace inti
 
 struct inti_ctx {
@@ -129,7 +164,15 @@ struct inti_ctx {
   // traces, Theta, its partial sums, green multipliers.
   struct {
     inti::DevBuf d_xs, g0, g1, theta, part, mu;
+    inti::FxPlan plan;
   } dimwork;
+  // Buffers of the multi-column contractions (contract_i8.cu): phase table,
+  // digit blocks of the densities, partial sums, and [flag, counters, column
+  // bounds].  Shared by the context's operators like the symmetric form's
+  // partials: live only within one product, on the context's one stream.
+  struct {
+    inti::DevBuf tab, bdig, partial, work;
+  } fx;
 };
 
 struct inti_quad {

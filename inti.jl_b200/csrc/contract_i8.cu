@@ -1,0 +1,1356 @@
+// Multi-column pair contractions Y = K X with FP64 accuracy on the INT8
+// tensor path (tcgen05 kind::i8): the product of an operator with many
+// densities, the batched operators, and the Theta product of the
+// density-interpolation correction.
+//
+// tcgen05 has no FP64 kind, and the FP64 MMA (mma.sync, fp64_mma.cuh) shares
+// the 64-lane FP64 datapath with the kernel evaluation: 64 complex columns
+// cost 256 FMA lanes a pair next to about 45 for the kernel value.  Here both
+// factors are written as 64-bit fixed-point numbers in eight signed base-256
+// digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer.
+// Algorithms 59 (2012), with integer digits), the digit products run on the
+// tensor cores with exact 32-bit integer sums, and the sums are put together
+// in FP64 once per item.  What is left on the FP64 pipe is one kernel
+// evaluation per pair and column group and four instructions per value that
+// cut it into digits.
+//
+// Accuracy.  Row i of A = K is scaled by a power of two that puts a bound of
+// |K_i.| just below 2^63, column c of B = diag(w) X by one for max |w x_c|;
+// both are rounded to integers (error 1/2 in 2^62..2^63) and the digit
+// products with p + q <= 7 are kept (p, q = 0 the leading digits; what is
+// dropped is below 2^-61 of the product of the two bounds per pair).  Sums
+// carry no rounding.  An FP64 accumulation of n terms rounds n times at
+// 2^-53 of the running sum, so the result is closer to the exact product of
+// the FP64 kernel values than the FP64 MMA's (measured against 64-bit
+// references in tests/test_gpu_contract.py).
+//
+// Work.  A persistent CTA per SM takes items (128 targets, a run of source
+// stages) from a counter, the longest first.  A stage is 64 K elements: NA
+// values per pair (1 real, 2 complex, 2 or 4 for the (S, D) pair of Theta)
+// of 64/NA sources.  Warp roles as in mrhs_tc.cu:
+//   * 16 generator warps: thread (row, quarter) evaluates 64/(4 NA) sources
+//     for its row and writes eight 16-byte chunks (one per digit, 16 K
+//     elements) of the A operand to shared memory: 128 rows x 16 B contiguous
+//     per chunk, conflict-free;
+//   * a copy warp: source records (FP64) and digit blocks of the densities
+//     by the TMA bulk engine;
+//   * an MMA warp: the digits of B lie one after another along N, so A's
+//     digit p against B's digits 0..7-p is one wide product (N = (8-p) NC,
+//     at most 256 per instruction) whose columns start at diagonal p of the
+//     accumulators: eight diagonals of NC columns, all 512 tensor-memory
+//     columns for NC = 64.  Reading each A digit once per 256 columns keeps
+//     the operand traffic of shared memory below the MMA time.
+// Generation of one stage runs beside the MMAs of the one before (two A
+// buffers), but only its integer, memory and conversion instructions overlap
+// them: on the B200 FP64 FMAs make no progress while INT8 MMAs are in flight
+// (16 warps of independent FMAs next to an MMA loop: 1.5% of their rate
+// alone, and the MMAs at 92% of theirs).  A stage therefore costs about the
+// sum of both: DL with 64 columns 2,333 cycles of MMAs (the full INT8 rate)
+// and 4,250 of generation, of which 2,500 are FP64 issue.  The 32-bit sums
+// hold 127 stages (8 * 255 * 128 * 8,128 < 2^31); then, or at the end of the
+// item, the generators read the diagonals and add them up in FP64.
+//
+// Measured (B200, against the FP64 MMA kernels, device time): 64 complex
+// columns of a Helmholtz DL at 13,872 nodes 5.63 -> 2.47 ms; eight surfaces of
+// 2,646 .. 21,600 nodes, combined field, 64 columns 26.9 -> 15.6 ms; the
+// correction of a 43,200-node surface (18 complex columns) 33.6 -> 16.0 ms.
+//
+// e^{ikd} comes from a 128-entry table in eight copies, one per lane of a
+// quarter-warp, so the gathers never conflict (a shared 1024-entry table
+// costs about 12 wavefronts a warp, and shared memory is as busy here as the
+// FP64 pipe), with one more term in each series.
+//
+// Every wait is bounded, as in mrhs_tc.cu.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "common.h"
+#include "contract_i8.h"
+#include "device_common.cuh"
+#include "internal.h"
+
+namespace inti {
+
+constexpr int FX_D = 8;                              // digits
+constexpr int FX_K = 64;                             // K elements per stage
+constexpr int FX_M = 128;                            // targets per item
+constexpr int FX_NMAX = 64;                          // real columns per pass
+constexpr int FX_GEN = 16;                           // generator warps
+constexpr int FX_THREADS = 32 * (FX_GEN + 2);
+constexpr int FX_FLUSH = 127;                        // stages a 32-bit sum holds
+constexpr int FX_A_DIGIT = FX_M * FX_K;              // bytes of one digit of A
+constexpr int FX_A_BYTES = FX_D * FX_A_DIGIT;        // 64 KB
+constexpr int FX_B_BYTES = FX_D * FX_NMAX * FX_K;    // 32 KB
+constexpr int FX_NS = 4;                             // source-record ring
+constexpr int FX_ND = 4;                             // MMA completion ring
+constexpr int FX_REC = 6;                            // doubles per source record
+constexpr int FX_TAB = 128, FX_REP = 8;              // phase table, copies
+
+template <int PDE, int KIND>
+struct FxShape {
+  static constexpr bool theta = KIND == FX_THETA || KIND == FX_THETA_D;
+  static constexpr bool cplx = PDE == HELMHOLTZ;
+  static constexpr int NA = (cplx ? 2 : 1) * (theta ? 2 : 1);
+  static constexpr int J = FX_K / NA;        // sources per stage
+  static constexpr int JT = J / 4;           // sources per generator thread and stage
+  static constexpr bool tnormal = KIND == ADL || KIND == HS || KIND == FX_THETA_D;
+  static constexpr int S_BYTES = J * FX_REC * 8;
+  static constexpr int OFF_B = 2 * FX_A_BYTES;
+  static constexpr int OFF_T = OFF_B + 2 * FX_B_BYTES;
+  static constexpr int OFF_S = OFF_T + (cplx ? FX_TAB * FX_REP * 16 : 0);
+  static constexpr int SMEM = OFF_S + FX_NS * S_BYTES;
+  static_assert(SMEM <= 230 * 1024, "shared memory");
+};
+
+static int fx_na(int pde, int kind) {
+  return (pde == HELMHOLTZ ? 2 : 1) * (kind >= FX_THETA ? 2 : 1);
+}
+
+// Per-launch constants of the kernel values.
+struct FxConst {
+  double k, kT, c1r, c1i, c2r, c2i, kc1r, kc1i;
+};
+
+// e^{i d k}, kT = k FX_TAB / (2 pi): the table value of the nearest multiple
+// of delta = 2 pi / FX_TAB times the Taylor series of the rest (|f delta| <=
+// pi/128: sin to r^7, cos to r^6, truncation below 4e-18).
+__device__ __forceinline__ void fx_expi(double d, double kT, const double2* __restrict__ tab, double& c, double& s) {
+  constexpr double D = 2.0 * kPi / FX_TAB, D2 = D * D;
+  constexpr double C2 = -D2 / 2, C4 = D2 * D2 / 24, C6 = -D2 * D2 * D2 / 720;
+  constexpr double S3 = -D2 * D / 6, S5 = D2 * D2 * D / 120, S7 = -D2 * D2 * D2 * D / 5040;
+  const double t = fma(d, kT, kRoundShift);
+  const double f = fma(d, kT, -(t - kRoundShift));
+  const double f2 = f * f;
+  const double cp = fma(f2, fma(f2, fma(f2, C6, C4), C2), 1.0);
+  const double sp = f * fma(f2, fma(f2, fma(f2, S7, S5), S3), D);
+  const double2 e = tab[(__double2loint(t) & (FX_TAB - 1)) * FX_REP];
+  c = fma(cp, e.x, -sp * e.y);
+  s = fma(sp, e.x, cp * e.y);
+}
+
+// The NA values of one pair without the 1/(4 pi), times the row's scale p:
+// (Re, Im) of the kernel, Theta: the S value(s), then the D value(s).  nx is
+// the target normal times p.  rec = x y z nx ny nz of the
+// source; e^{ikd}(1/d - ik)(r.n)/d^2 is formed as e^{ikd}(Q - ik P) with
+// P = (r.n)/d^2, Q = P/d.
+template <int PDE, int KIND>
+__device__ __forceinline__ void fx_values(const double (&x)[3], const double (&nx)[3], double pr,
+                                          const double* __restrict__ rec, const FxConst& c, const double2* __restrict__ tab,
+                                          double (&v)[FxShape<PDE, KIND>::NA]) {
+  const double2 s01 = reinterpret_cast<const double2*>(rec)[0], s23 = reinterpret_cast<const double2*>(rec)[1];
+  const double r0 = x[0] - s01.x, r1 = x[1] - s01.y, r2 = x[2] - s23.x;
+  const double d2 = fma(r2, r2, fma(r1, r1, r0 * r0));
+  const double ri = pair_keep(d2) ? rsqrt_fast(d2) : 0.0;  // self pair: every value 0
+  double rny = 0.0, rnx = 0.0, nn = 0.0;
+  if (KIND != SL) {
+    const double2 s45 = reinterpret_cast<const double2*>(rec)[2];
+    if (KIND != ADL) rny = fma(r2, s45.y, fma(r1, s45.x, r0 * s23.y));
+    if (FxShape<PDE, KIND>::tnormal) rnx = fma(r2, nx[2], fma(r1, nx[1], r0 * nx[0]));
+    if (KIND == HS || KIND == FX_THETA_D) nn = fma(nx[2], s45.y, fma(nx[1], s45.x, nx[0] * s23.y));
+  }
+  const double id2 = ri * ri;
+  if constexpr (PDE == LAPLACE) {
+    const double ri3 = id2 * ri;
+    if constexpr (KIND == SL)
+      v[0] = pr * ri;
+    else if constexpr (KIND == DL)
+      v[0] = pr * rny * ri3;
+    else if constexpr (KIND == ADL)
+      v[0] = -rnx * ri3;
+    else if constexpr (KIND == HS)
+      v[0] = fma(-3.0 * rnx * rny, id2, nn) * ri3;
+    else if constexpr (KIND == CF)
+      v[0] = pr * fma(c.c2r, ri, c.c1r * (rny * ri3));
+    else if constexpr (KIND == FX_THETA) {
+      const double pri = pr * ri;
+      v[0] = pri;
+      v[1] = rny * (pri * id2);
+    } else {
+      v[0] = -rnx * ri3;
+      v[1] = fma(-3.0 * rnx * rny, id2, nn) * ri3;
+    }
+  } else {
+    const double d = d2 * ri;
+    double cs, sn;
+    fx_expi(d, c.kT, tab, cs, sn);
+    auto times_e = [&](double wr, double wi, double& re, double& im) {
+      re = fma(cs, wr, -sn * wi);
+      im = fma(cs, wi, sn * wr);
+    };
+    auto layer = [&](double rn, double& re, double& im) {
+      const double P = rn * id2;
+      times_e(P * ri, -c.k * P, re, im);
+    };
+    auto hyper = [&](double& re, double& im) {
+      // [(1/d - ik) p + (k^2 d^2 - 3 + 3ikd) s5], p = nn/d^2, s5 = rnx rny/d^5
+      const double kd = c.k * d;
+      const double p = nn * id2, s5 = (rnx * rny) * (id2 * id2 * ri);
+      times_e(fma(ri, p, fma(kd, kd, -3.0) * s5), fma(-c.k, p, 3.0 * kd * s5), re, im);
+    };
+    if constexpr (KIND == SL) {
+      const double pri = pr * ri;
+      v[0] = pri * cs;
+      v[1] = pri * sn;
+    } else if constexpr (KIND == DL) {
+      layer(pr * rny, v[0], v[1]);
+    } else if constexpr (KIND == ADL) {
+      layer(-rnx, v[0], v[1]);
+    } else if constexpr (KIND == HS) {
+      hyper(v[0], v[1]);
+    } else if constexpr (KIND == CF) {
+      const double P = rny * id2, Q = P * ri;
+      const double cp = pr * cs, sp = pr * sn;
+      const double wr = fma(c.c2r, ri, fma(c.c1r, Q, c.kc1i * P)), wi = fma(c.c2i, ri, fma(c.c1i, Q, -c.kc1r * P));
+      v[0] = fma(cp, wr, -sp * wi);
+      v[1] = fma(cp, wi, sp * wr);
+    } else if constexpr (KIND == FX_THETA) {
+      const double pri = pr * ri;
+      v[0] = pri * cs;
+      v[1] = pri * sn;
+      layer(pr * rny, v[2], v[3]);
+    } else {
+      layer(-rnx, v[0], v[1]);
+      hyper(v[2], v[3]);
+    }
+  }
+}
+
+// Power of two p with |v| p < 2^63 (1 - 2^-5) for |v| <= cur: eight balanced
+// digits reach 0.498 * 2^64.  0 for cur = 0.
+__device__ __forceinline__ double fx_scale(double cur) {
+  if (!(cur > 0.0)) return 0.0;
+  const long long b = __double_as_longlong(cur);
+  const int e = (int)(b >> 52) - 1023;
+  const bool high = (b & 0xFFFFFFFFFFFFFLL) > 0xE666666666666LL;  // mantissa above 1.9
+  return __longlong_as_double((long long)(1023 + (high ? 61 : 62) - e) << 52);
+}
+// 0, or a magnitude whose scale and products of scales stay normal numbers.
+__device__ __forceinline__ bool fx_fits(double cur) { return cur == 0.0 || (cur > 1e-120 && cur < 1e120); }
+
+// Digits of A: the bytes of v rounded to a 64-bit integer, the leading one
+// signed, the others unsigned (the MMA takes the signedness of A per
+// instruction, so nothing has to be balanced).  The conversion runs on the
+// otherwise idle conversion unit; cutting v with rounding additions took four
+// FP64 instructions.
+__device__ __forceinline__ uint2 fx_bytes(double v) {
+  const long long w = __double2ll_rn(v);
+  return make_uint2((uint32_t)w, (uint32_t)(w >> 32));
+}
+
+// Digits of B are balanced (-128 .. 127): the bytes of the integer plus 0x80
+// in every byte, each minus 128.  Their mean is zero, and so is that of what
+// is dropped.
+__device__ __forceinline__ uint2 fx_digits(double v) {
+  const unsigned long long w = ((unsigned long long)__double2ll_rn(v) + 0x8080808080808080ULL) ^ 0x8080808080808080ULL;
+  return make_uint2((uint32_t)w, (uint32_t)(w >> 32));
+}
+
+// Digits of four values as one word per digit (value e in byte e), leading
+// digit first.
+__device__ __forceinline__ void fx_pack4(const uint2 (&a)[4], uint32_t (&w)[FX_D]) {
+  auto four = [](uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t& b0, uint32_t& b1, uint32_t& b2,
+                 uint32_t& b3) {
+    const uint32_t l0 = __byte_perm(a0, a1, 0x5140), l1 = __byte_perm(a2, a3, 0x5140);
+    const uint32_t h0 = __byte_perm(a0, a1, 0x7362), h1 = __byte_perm(a2, a3, 0x7362);
+    b0 = __byte_perm(l0, l1, 0x5410);
+    b1 = __byte_perm(l0, l1, 0x7632);
+    b2 = __byte_perm(h0, h1, 0x5410);
+    b3 = __byte_perm(h0, h1, 0x7632);
+  };
+  four(a[0].x, a[1].x, a[2].x, a[3].x, w[7], w[6], w[5], w[4]);
+  four(a[0].y, a[1].y, a[2].y, a[3].y, w[3], w[2], w[1], w[0]);
+}
+
+// ---------------------------------------------------------------------------
+// tensor-core primitives
+// ---------------------------------------------------------------------------
+// K-major, no swizzle: 8-row x 16-byte core matrices, `lbo` bytes between
+// K chunks, 128 bytes between 8-row groups.
+__device__ __forceinline__ uint64_t fx_desc(uint32_t saddr, uint32_t lbo) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)((lbo >> 4) & 0x3FFF) << 16 | (uint64_t)(128 >> 4) << 32 |
+         (uint64_t)1 << 46;
+}
+
+// S32 accumulate, 8-bit A (signed or not) and signed B, both K-major, M = 128
+__host__ __device__ constexpr uint32_t fx_idesc(int n, bool a_signed) {
+  return (2u << 4) | ((a_signed ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(FX_M >> 4) << 24);
+}
+
+__device__ __forceinline__ void fx_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+__device__ __forceinline__ bool fx_elect() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.b32 %0, 1, 0, P;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
+__device__ __forceinline__ void fx_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void fx_fence_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void fx_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__device__ __forceinline__ void fx_ld4(uint32_t taddr, int32_t (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void fx_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+struct FxArgs {
+  const FxRows* rows;
+  const FxItem* items;
+  int nitems;
+  int nc;                   // real columns of this pass (fx_width)
+  const double* tcoords;
+  const double* tnormals;
+  const double* rowscale;   // per target
+  const double* records;    // source records, J per stage
+  const unsigned char* bdig;  // digit blocks, nc * 512 bytes per stage
+  const double2* tab;       // FX_TAB phase table
+  double* partial;          // [slot][column][128]
+  FxConst c;
+  int* counter;
+  const int* flag;
+  int* err;
+};
+
+// The MMAs of one stage: A digit p against the digits 0 .. 7-p of B, in equal
+// parts of at most 256 columns, for each K slab of 32 elements.  Digit 0 covers every
+// accumulator column, so its first slab may overwrite them (accumulate 0).
+// For odd NC/8 a product of an odd number of digits is rounded up by eight
+// columns: they read the digit after and add to the columns past the last
+// diagonal, which nothing reads.
+// Unrolled, so that every offset is an immediate: the issuing lane competes
+// with the generators for its issue slots, and a loop that reads them from
+// shared memory took about 330 cycles per MMA, three times the MMA's own.
+template <int NC>
+__device__ __forceinline__ void fx_issue(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t accumulate) {
+#pragma unroll
+  for (int slab = 0; slab < 2; ++slab) {
+#pragma unroll
+    for (int p = 0; p < FX_D; ++p) {
+      const int total = ((FX_D - p) * NC + 15) / 16 * 16, parts = (total + 255) / 256;
+      const int w = (total / parts + 15) / 16 * 16;
+      static_assert(NC % 8 == 0 && 8 * NC + (NC % 16 ? 8 : 0) <= 512, "tensor memory");
+#pragma unroll
+      for (int part = 0; part < parts; ++part) {
+        const int n0 = part * w, n = min(w, total - n0);
+        fx_mma(tmem + p * NC + n0, ad + ((p * FX_A_DIGIT + slab * 2 * FX_M * 16) >> 4),
+               bd + ((slab * 2 * NC * FX_D * 16 + n0 * 16) >> 4), fx_idesc(n, p == 0),
+               slab == 0 && p == 0 ? accumulate : 1u);
+      }
+    }
+  }
+}
+
+// Sum of the diagonals of one accumulator element in units of 256^7.
+__device__ __forceinline__ double fx_sum(const int32_t (&d)[FX_D][4], int e) {
+  const long long hi = ((long long)d[0][e] << 24) + ((long long)d[1][e] << 16) + ((long long)d[2][e] << 8) + d[3][e];
+  const long long lo = ((long long)d[4][e] << 24) + ((long long)d[5][e] << 16) + ((long long)d[6][e] << 8) + d[7][e];
+  return fma((double)hi, 4294967296.0, (double)lo);
+}
+
+template <int PDE, int KIND>
+__global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
+  using SH = FxShape<PDE, KIND>;
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ __align__(8) uint64_t fullS[FX_NS], fullB[2], aFull[2], mmaDone[FX_ND], drainBar;
+  __shared__ uint32_t tmem_base_sh;
+  __shared__ int item_sh;
+  if (*a.flag) return;  // densities or kernel values out of range: the FP64 kernels run
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nc = a.nc;
+  const uint32_t bstage = (uint32_t)nc * (FX_D * FX_K), blbo = (uint32_t)nc * (FX_D * 16);
+  if (tid == 0) {
+    for (int q = 0; q < FX_NS; ++q) mbar_init(&fullS[q], 1);
+    for (int q = 0; q < FX_ND; ++q) mbar_init(&mmaDone[q], 1);
+    for (int q = 0; q < 2; ++q) {
+      mbar_init(&fullB[q], 1);
+      mbar_init(&aFull[q], FX_GEN);
+    }
+    mbar_init(&drainBar, 1);
+    mbar_fence_init();
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (SH::cplx) {
+    double2* tab = reinterpret_cast<double2*>(sm + SH::OFF_T);
+    for (int q = tid; q < FX_TAB * FX_REP; q += FX_THREADS) tab[q] = a.tab[q / FX_REP];
+  }
+  fx_fence_before();
+  __syncthreads();
+  fx_fence_after();
+  const uint32_t tmem = tmem_base_sh, sbase = smem_u32(sm);
+
+  uint32_t g = 0;           // stages done by this CTA (same in every thread)
+  uint32_t nS = 0, nB = 0;  // copy warp: copies issued
+  uint32_t nC = 0;          // MMA warp: groups committed
+  bool ok = true;
+
+  for (;;) {
+    if (tid == 0) item_sh = atomicAdd(a.counter, 1);
+    __syncthreads();
+    const int it = item_sh;
+    if (it >= a.nitems) break;
+    const FxItem item = a.items[it];
+    const FxRows rb = a.rows[item.rows];
+    for (int done = 0; done < item.nstages; done += FX_FLUSH) {
+      const uint32_t T = (uint32_t)min(FX_FLUSH, item.nstages - done);
+      const int64_t st0 = (int64_t)rb.stage0 + item.stage + done;
+      if (warp == 0) {
+        for (uint32_t t = 0; t < T; ++t) {
+          const uint32_t gg = g + t, bb = gg & 1;
+          ok = mbar_wait_bounded(&aFull[bb], (gg >> 1) & 1) && mbar_wait_bounded(&fullB[bb], (gg >> 1) & 1);
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+          }
+          fx_fence_after();
+          if (fx_elect()) {
+            const uint64_t ad = fx_desc(sbase + bb * FX_A_BYTES, FX_M * 16);
+            const uint64_t bd = fx_desc(sbase + SH::OFF_B + bb * FX_B_BYTES, blbo);
+            const uint32_t acc = t > 0 ? 1u : 0u;
+            switch (nc) {
+              case 16: fx_issue<16>(tmem, ad, bd, acc); break;
+              case 24: fx_issue<24>(tmem, ad, bd, acc); break;
+              case 32: fx_issue<32>(tmem, ad, bd, acc); break;
+              case 40: fx_issue<40>(tmem, ad, bd, acc); break;
+              case 48: fx_issue<48>(tmem, ad, bd, acc); break;
+              case 56: fx_issue<56>(tmem, ad, bd, acc); break;
+              default: fx_issue<64>(tmem, ad, bd, acc); break;
+            }
+            fx_commit(&mmaDone[gg % FX_ND]);
+          }
+          __syncwarp();
+          ++nC;
+        }
+      } else if (warp == 1) {
+        auto copyS = [&](uint32_t t) {
+          const uint32_t b = (g + t) % FX_NS;
+          if (fx_elect()) {
+            mbar_arrive_expect_tx(&fullS[b], SH::S_BYTES);
+            bulk_copy_g2s(sm + SH::OFF_S + b * SH::S_BYTES, a.records + (st0 + t) * (SH::J * FX_REC), SH::S_BYTES,
+                          &fullS[b]);
+          }
+          __syncwarp();
+          ++nS;
+        };
+        auto copyB = [&](uint32_t t) {
+          const uint32_t b = (g + t) & 1;
+          if (fx_elect()) {
+            mbar_arrive_expect_tx(&fullB[b], bstage);
+            bulk_copy_g2s(sm + SH::OFF_B + b * FX_B_BYTES, a.bdig + (size_t)(st0 + t) * bstage, bstage, &fullB[b]);
+          }
+          __syncwarp();
+          ++nB;
+        };
+        // the buffers of the run before are free: its MMAs were waited for
+        for (uint32_t t = 0; t < FX_NS - 1 && t < T; ++t) copyS(t);
+        copyB(0);
+        for (uint32_t t = 0; t + 1 < T; ++t) {
+          // MMA group gg-1 read the B buffer of stage gg+1 and, through its A
+          // tile, the source records of stage gg-1
+          const uint32_t gg = g + t;
+          if (t > 0) ok = mbar_wait_bounded(&mmaDone[(gg - 1) % FX_ND], ((gg - 1) / FX_ND) & 1);
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+          }
+          copyB(t + 1);
+          if (t + FX_NS - 1 < T) copyS(t + FX_NS - 1);
+        }
+      } else {
+        const int gw = warp - 2, quarter = gw >> 2;
+        const int r = 32 * (warp & 3) + lane;  // target row = tensor-memory lane
+        const int64_t row = rb.row0 + min(r, rb.nrows - 1);
+        double x[3], nx[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[c] = a.tcoords[3 * row + c];
+        if (SH::tnormal) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) nx[c] = a.tnormals[3 * row + c] * a.rowscale[row];
+        }
+        const double scale = a.rowscale[row];
+        const double2* tab = reinterpret_cast<const double2*>(sm + SH::OFF_T) + (lane & (FX_REP - 1));
+        for (uint32_t t = 0; t < T; ++t) {
+          const uint32_t gg = g + t, sb = gg % FX_NS;
+          bool w = mbar_wait_bounded(&fullS[sb], (gg / FX_NS) & 1);
+          // A buffer gg & 1 was last read by MMA group gg-2
+          if (w && t >= 2) w = mbar_wait_bounded(&mmaDone[(gg - 2) % FX_ND], ((gg - 2) / FX_ND) & 1);
+          if (!__all_sync(0xffffffffu, w)) {
+            ok = false;
+            break;
+          }
+          const double* S = reinterpret_cast<const double*>(sm + SH::OFF_S + sb * SH::S_BYTES) +
+                            quarter * SH::JT * FX_REC;
+          unsigned char* A = sm + (gg & 1) * FX_A_BYTES + quarter * (FX_M * 16) + r * 16;
+          // Groups of four sources, NA words each.  The octets of a warp take
+          // them in rotated order, so that their stores of NA words at a
+          // stride of 16 bytes fall on distinct banks; storing each group at
+          // once keeps the registers for evaluations in flight.
+          constexpr int G = SH::JT / 4;
+#pragma unroll
+          for (int q = 0; q < G; ++q) {
+            const int grp = (q + (lane >> 3)) & (G - 1);
+            const double* Sg = S + grp * (4 * FX_REC);
+            uint2 dg[SH::NA][4];
+            {
+              double v[4][SH::NA];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) fx_values<PDE, KIND>(x, nx, scale, Sg + e * FX_REC, a.c, tab, v[e]);
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int n = 0; n < SH::NA; ++n) dg[n][e] = fx_bytes(v[e][n]);
+            }
+            uint32_t wd[SH::NA][FX_D];
+#pragma unroll
+            for (int n = 0; n < SH::NA; ++n) fx_pack4(dg[n], wd[n]);
+            unsigned char* Ag = A + grp * (4 * SH::NA);
+#pragma unroll
+            for (int p = 0; p < FX_D; ++p) {
+              if constexpr (SH::NA == 1)
+                *reinterpret_cast<uint32_t*>(Ag + p * FX_A_DIGIT) = wd[0][p];
+              else if constexpr (SH::NA == 2)
+                *reinterpret_cast<uint2*>(Ag + p * FX_A_DIGIT) = make_uint2(wd[0][p], wd[1][p]);
+              else
+                *reinterpret_cast<uint4*>(Ag + p * FX_A_DIGIT) = make_uint4(wd[0][p], wd[1][p], wd[2][p], wd[3][p]);
+            }
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&aFull[gg & 1]);
+        }
+        if (ok) {
+          const uint32_t gl = g + T - 1;
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&mmaDone[gl % FX_ND], (gl / FX_ND) & 1));
+        }
+        if (ok) {
+          fx_fence_after();
+          const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+          double* out = a.partial + (size_t)item.slot * nc * FX_M + r;
+          for (int c = 4 * quarter; c < nc; c += FX_GEN) {
+            int32_t d[FX_D][4];
+#pragma unroll
+            for (int s = 0; s < FX_D; ++s) fx_ld4(lane_addr + s * nc + c, d[s]);
+            fx_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              double v = fx_sum(d, e);
+              double* o = out + (size_t)(c + e) * FX_M;
+              if (done > 0) v += *o;  // the runs of an item add up in the same thread
+              *o = v;
+            }
+          }
+        }
+      }
+      g += T;
+      fx_fence_before();
+      // accumulators read (or the run abandoned) before the next run's MMAs
+      if (__syncthreads_or(!ok)) goto fail;
+      fx_fence_after();
+    }
+  }
+  goto done;
+fail:
+  if (tid == 0) atomicExch(a.err, kErrWaitTimeout);
+  // Everything this CTA put in flight must land before it leaves (each copy
+  // alone on its barrier; one more commit tracks every MMA issued).
+  if (warp == 1 && lane == 0) {
+    for (uint32_t q = nS > FX_NS ? nS - FX_NS : 0; q < nS; ++q) mbar_wait_bounded(&fullS[q % FX_NS], (q / FX_NS) & 1);
+    for (uint32_t q = nB > 2 ? nB - 2 : 0; q < nB; ++q) mbar_wait_bounded(&fullB[q & 1], (q >> 1) & 1);
+  }
+  if (warp == 0) {
+    if (nC > 0 && fx_elect()) {
+      fx_commit(&drainBar);
+      mbar_wait_bounded(&drainBar, 0);
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+done:
+  fx_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    fx_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// plan kernels
+// ---------------------------------------------------------------------------
+// Centre and radius of each stage's sources (double4) and their records; the
+// largest normal of all sources (bits in meta[0]).
+__global__ void fx_plan_sources(int nstages, int J, const FxStage* __restrict__ stages,
+                                const double* __restrict__ coords, const double* __restrict__ normals,
+                                double* __restrict__ records, double4* __restrict__ tiles,
+                                unsigned long long* __restrict__ meta) {
+  const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (s >= nstages) return;
+  const FxStage st = stages[s];
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY}, n2 = 0.0;
+  for (int j = lane; j < J; j += 32) {
+    double v[FX_REC] = {0, 0, 0, 0, 0, 0};
+    if (j < st.count) {
+      const int64_t i = st.src0 + j;
+      for (int c = 0; c < 3; ++c) {
+        v[c] = coords[3 * i + c];
+        lo[c] = fmin(lo[c], v[c]);
+        hi[c] = fmax(hi[c], v[c]);
+        if (normals) v[3 + c] = normals[3 * i + c];
+      }
+      n2 = fmax(n2, v[3] * v[3] + v[4] * v[4] + v[5] * v[5]);
+    }
+    for (int c = 0; c < FX_REC; ++c) records[((int64_t)s * J + j) * FX_REC + c] = v[c];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+      hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+    }
+    n2 = fmax(n2, __shfl_xor_sync(0xffffffffu, n2, o));
+  }
+  if (lane == 0) {
+    const double a = hi[0] - lo[0], b = hi[1] - lo[1], c = hi[2] - lo[2];
+    tiles[s] = make_double4((lo[0] + hi[0]) / 2, (lo[1] + hi[1]) / 2, (lo[2] + hi[2]) / 2,
+                            0.5 * sqrt(a * a + b * b + c * c) * (1 + 1e-12));
+    atomicMax(meta, (unsigned long long)__double_as_longlong(sqrt(n2)));
+  }
+}
+
+// Bound of |K(x, y)| over the NA values from the modulus of the kernel (no
+// phase), with the distance d, id = 1/d, |r.n_x|, |r.n_y| and |n_x.n_y| given.
+template <int PDE, int KIND>
+__device__ __forceinline__ double fx_modulus(double d, double id, double rnx, double rny, double nn,
+                                             const FxConst& c) {
+  const double id2 = id * id;
+  const double k = PDE == HELMHOLTZ ? fabs(c.k) : 0.0;
+  const double f = (id + k) * id2;  // |e^{ikd}(1/d - ik)|/d^2 at most
+  const double h = f * nn + ((k * d) * (k * d) + 3.0 + 3.0 * k * d) * rnx * rny * (id2 * id2 * id);
+  if (KIND == SL) return id;
+  if (KIND == DL) return f * rny;
+  if (KIND == ADL) return f * rnx;
+  if (KIND == HS) return h;
+  if (KIND == CF) return (fabs(c.c1r) + fabs(c.c1i)) * f * rny + (fabs(c.c2r) + fabs(c.c2i)) * id;
+  if (KIND == FX_THETA) return fmax(id, f * rny);
+  return fmax(f * rnx, h);
+}
+
+// Scale of each target row: a bound of its kernel values.  One warp per eight
+// consecutive rows, which lie close together: it takes the values of their
+// nearest tiles, then of every tile whose values may exceed one of the bounds
+// so far (|K| from the distance to the tile alone); the others add nothing to
+// the maximum.  (One thread per row left the device almost empty, 4.0 ms at
+// 13,872 rows; one warp per row read the tiles 43,200 times, 2.1 ms there.)
+constexpr int kPlanRows = 8;
+
+template <int PDE, int KIND>
+__global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __restrict__ rows,
+                                                    const double* __restrict__ tc, const double* __restrict__ tn,
+                                                    const FxStage* __restrict__ stages,
+                                                    const double4* __restrict__ tiles,
+                                                    const double* __restrict__ records, FxConst c,
+                                                    double* __restrict__ rowscale,
+                                                    unsigned long long* __restrict__ meta) {
+  using SH = FxShape<PDE, KIND>;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int JL = SH::J < 32 ? SH::J : 32;  // lanes along the sources of a tile
+  constexpr int RP = 32 / JL;                  // rows per pass
+  constexpr int NP = kPlanRows / RP;           // passes
+  __shared__ double sx[8][kPlanRows][8];       // x, n_x, |n_x| of a warp's rows
+  const int wid = blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (wid / (FX_M / kPlanRows) >= nrb) return;
+  const FxRows rb = rows[wid / (FX_M / kPlanRows)];
+  const int r0 = wid % (FX_M / kPlanRows) * kPlanRows;
+  if (r0 >= rb.nrows) return;
+  const double snorm = __longlong_as_double((long long)meta[0]);
+  double (*rx)[8] = sx[threadIdx.x >> 5];
+  if (lane < kPlanRows) {
+    const int64_t row = rb.row0 + min(r0 + lane, rb.nrows - 1);
+    double n2 = 0.0;
+    for (int q = 0; q < 3; ++q) {
+      const double nq = SH::tnormal ? tn[3 * row + q] : 0.0;
+      rx[lane][q] = tc[3 * row + q];
+      rx[lane][3 + q] = nq;
+      n2 += nq * nq;
+    }
+    rx[lane][6] = SH::tnormal ? sqrt(n2) : 1.0;
+  }
+  __syncwarp();
+  auto centre2 = [&](int q, const double4& t) {  // squared distance of row q to the tile's centre
+    const double a = rx[q][0] - t.x, b = rx[q][1] - t.y, e = rx[q][2] - t.z;
+    return a * a + b * b + e * e;
+  };
+  const int s0 = rb.stage0, s1 = rb.stage0 + rb.nstages;
+  double best[NP] = {};  // of rows RP * pass + lane / JL, this lane's sources
+  auto tile = [&](int s) {
+    const int cnt = stages[s].count;
+    for (int j = lane % JL; j < cnt; j += JL) {
+      const double* y = records + ((int64_t)s * SH::J + j) * FX_REC;
+      const double y0 = y[0], y1 = y[1], y2 = y[2], n0 = y[3], n1 = y[4], n2 = y[5];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const double* t = rx[RP * p + lane / JL];
+        const double a = t[0] - y0, b = t[1] - y1, e = t[2] - y2;
+        const double d2 = a * a + b * b + e * e;
+        if (!(d2 > 0.99 * kSamePointTol2)) continue;
+        const double id = rsqrt_fast(d2);
+        const double rnx = fabs(a * t[3] + b * t[4] + e * t[5]), rny = fabs(a * n0 + b * n1 + e * n2);
+        const double nn = fabs(t[3] * n0 + t[4] * n1 + t[5] * n2);
+        best[p] = fmax(best[p], fx_modulus<PDE, KIND>(d2 * id, id, rnx, rny, nn, c));
+      }
+    }
+  };
+  auto bound = [&](int q) {  // the largest value of row q so far, in every lane
+    double v = 0.0;
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+      if (p == q / RP && lane / JL == q % RP) v = best[p];
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(kAll, v, o));
+    return v;
+  };
+  int last = -1;
+  for (int q = 0; q < kPlanRows; ++q) {
+    double dn = INFINITY;
+    int near = s0;
+    for (int s = s0 + lane; s < s1; s += 32) {
+      const double d = centre2(q, tiles[s]);
+      if (d < dn) {
+        dn = d;
+        near = s;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double d = __shfl_xor_sync(kAll, dn, o);
+      const int s = __shfl_xor_sync(kAll, near, o);
+      if (d < dn || (d == dn && s < near)) {
+        dn = d;
+        near = s;
+      }
+    }
+    if (near != last) tile(near);
+    last = near;
+  }
+  // Sources at least `reach` away cannot exceed the bound: the crude bound
+  // falls with the distance, so the first of 64 distances (powers of sqrt 2,
+  // two per lane) at which it is low enough will do.  Kept with the row.
+  for (int q = 0; q < kPlanRows; ++q) {
+    const double cur = bound(q), tnorm = rx[q][6], unit = tiles[last].w + sqrt(centre2(q, tiles[last]));
+    double reach = INFINITY;
+    for (int h = 1; h >= 0; --h) {
+      const double d = exp2(0.5 * (lane + 32 * h) - 24.0) * unit;
+      const unsigned ok =
+          __ballot_sync(kAll, fx_modulus<PDE, KIND>(d, 1.0 / d, d * tnorm, d * snorm, tnorm * snorm, c) <= cur);
+      if (ok) reach = __shfl_sync(kAll, d, __ffs(ok) - 1);
+    }
+    if (lane == 0) rx[q][7] = reach;
+  }
+  __syncwarp();
+  for (int b = s0; b < s1; b += 32) {
+    const int s = b + lane;
+    bool want = false;
+    if (s < s1) {
+      const double4 t = tiles[s];
+#pragma unroll
+      for (int q = 0; q < kPlanRows; ++q) {
+        const double rr = (rx[q][7] + t.w) * (1 + 1e-9);
+        want |= centre2(q, t) < rr * rr;
+      }
+    }
+    for (unsigned m = __ballot_sync(kAll, want); m; m &= m - 1) tile(b + __ffs(m) - 1);
+  }
+  for (int q = 0; q < kPlanRows; ++q) {
+    const double v = bound(q) * (1 + 1e-9);  // the values' own rounding
+    if (lane == 0 && r0 + q < rb.nrows) {
+      if (!fx_fits(v)) atomicExch(meta + 1, 1ULL);  // NaN too
+      rowscale[rb.row0 + r0 + q] = fx_fits(v) ? fx_scale(v) : 0.0;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// densities: column bounds and digit blocks
+// ---------------------------------------------------------------------------
+// colmax[surf * ncol + c]: bits of max |w x| over the (Re, Im) parts of column c.  Non-negative doubles
+// order as their bits; a NaN's exceed every number's.
+constexpr int kMaxRun = 8;  // stages per warp
+
+template <bool CPLX>
+__global__ void fx_colmax(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
+                          const double* __restrict__ x, int64_t ldx, int ncol, unsigned long long* colmax) {
+  const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, c = blockIdx.y;
+  const int s0 = run * kMaxRun, s1 = min(nstages, s0 + kMaxRun);
+  unsigned long long best = 0;
+  int surf = -1;
+  auto flush = [&]() {
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+      best = other > best ? other : best;
+    }
+    if (lane == 0 && surf >= 0) atomicMax(&colmax[(int64_t)surf * ncol + c], best);
+    best = 0;
+  };
+  for (int s = s0; s < s1; ++s) {
+    const FxStage st = stages[s];
+    if (st.surf != surf) {
+      flush();
+      surf = st.surf;
+    }
+    for (int j = lane; j < st.count; j += 32) {
+      const int64_t i = st.src0 + j;
+      const int64_t q = (int64_t)c * ldx + i;
+      double m;
+      if (CPLX) {
+        const double2 v = reinterpret_cast<const double2*>(x)[q];
+        const double re = fabs(w[i] * v.x), im = fabs(w[i] * v.y);
+        m = re > im || re != re ? re : im;
+      } else {
+        m = fabs(w[i] * x[q]);
+      }
+      const unsigned long long b = (unsigned long long)__double_as_longlong(m);
+      best = b > best ? b : best;
+    }
+  }
+  flush();
+}
+
+// Sets the flag when a row or column bound does not fit (one block).
+__global__ void fx_check(int count, const unsigned long long* __restrict__ colmax,
+                         const unsigned long long* __restrict__ meta, int* flag) {
+  bool bad = meta[1] != 0;
+  for (int q = threadIdx.x; q < count; q += blockDim.x) bad |= !fx_fits(__longlong_as_double((long long)colmax[q]));
+  if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
+}
+
+// Digit blocks: stage s, digit q of column n at [chunk][q * nc + n][16 bytes].
+// One thread per (chunk of a stage, column c of the pass).  A chunk holds
+// groups of four sources, each value 0, then value 1; complex columns
+// (2c, 2c + 1) have values (Re x, -Im x) and (Im x, Re x).
+template <bool CPLX>
+__global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
+                        const double* __restrict__ x, int64_t ldx, int c0, int ncol, int nall, int nc,
+                        const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
+                        unsigned char* __restrict__ out) {
+  constexpr int JT = CPLX ? 8 : 16;  // sources of a chunk
+  const int per = CPLX ? nc / 2 : nc;
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(id % per), chunk = (int)(id / per % 4);
+  const int64_t s = id / per / 4;
+  if (s >= nstages || *flag) return;
+  const FxStage st = stages[s];
+  const bool live = c < ncol;
+  const double p =
+      live ? fx_scale(__longlong_as_double((long long)colmax[(int64_t)st.surf * nall + c0 + c])) : 0.0;
+  uint4* o = reinterpret_cast<uint4*>(out + s * ((int64_t)nc * FX_D * FX_K) + (int64_t)chunk * (nc * FX_D * 16));
+  uint32_t re[JT / 4][FX_D], im[CPLX ? 2 : 1][FX_D], mi[CPLX ? 2 : 1][FX_D];
+#pragma unroll
+  for (int h = 0; h < JT / 4; ++h) {
+    uint2 a[4], b[4], m[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int j = chunk * JT + 4 * h + e;
+      double vr = 0.0, vi = 0.0;
+      if (live && j < st.count) {
+        const int64_t i = st.src0 + j, q = (int64_t)(c0 + c) * ldx + i;
+        if (CPLX) {
+          const double2 v = reinterpret_cast<const double2*>(x)[q];
+          vr = w[i] * v.x;
+          vi = w[i] * v.y;
+        } else {
+          vr = w[i] * x[q];
+        }
+      }
+      a[e] = fx_digits(vr * p);
+      if (CPLX) {
+        b[e] = fx_digits(vi * p);
+        m[e] = fx_digits(-vi * p);
+      }
+    }
+    fx_pack4(a, re[h]);
+    if constexpr (CPLX) {
+      fx_pack4(b, im[h]);
+      fx_pack4(m, mi[h]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < FX_D; ++q) {
+    if constexpr (CPLX) {
+      o[q * nc + 2 * c] = make_uint4(re[0][q], mi[0][q], re[1][q], mi[1][q]);
+      o[q * nc + 2 * c + 1] = make_uint4(im[0][q], re[0][q], im[1][q], re[1][q]);
+    } else {
+      o[q * nc + c] = make_uint4(re[0][q], re[1][q], re[2][q], re[3][q]);
+    }
+  }
+}
+
+// Theta: column bounds over the traces (both arrays share a column's scale,
+// since their products share the accumulators).
+__global__ void fx_theta_max(int64_t n, int ns, bool cplx, const double* __restrict__ w, const double2* __restrict__ g0,
+                             const double2* __restrict__ g1, unsigned long long* colmax) {
+  // a block takes 256 consecutive nodes; thread t the entries t, t + 256, ... of their rows
+  __shared__ unsigned long long best[32];
+  if (threadIdx.x < 32) best[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t j0 = blockIdx.x * (int64_t)256, j1 = min(n, j0 + 256);
+  for (int64_t e = j0 * ns + threadIdx.x; e < j1 * ns; e += blockDim.x) {
+    const int64_t j = e / ns;
+    const double2 a = g0[e], b = g1[e];
+    const double v[4] = {a.x, b.x, cplx ? a.y : 0.0, cplx ? b.y : 0.0};
+    unsigned long long m = 0;
+    for (int q = 0; q < 4; ++q) {
+      const unsigned long long t = (unsigned long long)__double_as_longlong(fabs(w[j] * v[q]));
+      m = t > m ? t : m;
+    }
+    atomicMax(&best[(int)(e - j * ns)], m);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < ns) atomicMax(&colmax[threadIdx.x], best[threadIdx.x]);
+}
+
+// Digit blocks of the traces: values (S; D), complex (Sr, Si; Dr, Di), against
+// (g1; -g0), complex columns (Re, Im): (g1r, g1i), (-g1i, g1r), (-g0r, -g0i),
+// (g0i, -g0r).
+template <bool CPLX>
+__global__ void fx_theta_pack(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
+                              const double2* __restrict__ g0, const double2* __restrict__ g1, int ns, int nc,
+                              const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
+                              unsigned char* __restrict__ out) {
+  constexpr int JT = CPLX ? 4 : 8;
+  const int per = CPLX ? nc / 2 : nc;
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(id % per), chunk = (int)(id / per % 4);
+  const int64_t s = id / per / 4;
+  if (s >= nstages || *flag) return;
+  const FxStage st = stages[s];
+  const bool live = c < ns;
+  const double p = live ? fx_scale(__longlong_as_double((long long)colmax[c])) : 0.0;
+  uint4* o = reinterpret_cast<uint4*>(out + s * ((int64_t)nc * FX_D * FX_K) + (int64_t)chunk * (nc * FX_D * 16));
+  double2 a[JT], b[JT];
+#pragma unroll
+  for (int e = 0; e < JT; ++e) {
+    const int j = chunk * JT + e;
+    a[e] = b[e] = make_double2(0.0, 0.0);
+    if (live && j < st.count) {
+      const int64_t i = st.src0 + j, q = i * ns + c;
+      const double wj = w[i];
+      const double2 u = g0[q], v = g1[q];
+      a[e] = make_double2(wj * u.x, wj * u.y);
+      b[e] = make_double2(wj * v.x, wj * v.y);
+    }
+  }
+  auto pack = [&](auto get, uint32_t (&wd)[FX_D]) {
+    uint2 d[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[e] = fx_digits(get(e) * p);
+    fx_pack4(d, wd);
+  };
+  uint32_t wd[CPLX ? 6 : 4][FX_D];
+  if constexpr (CPLX) {
+    pack([&](int e) { return b[e].x; }, wd[0]);
+    pack([&](int e) { return b[e].y; }, wd[1]);
+    pack([&](int e) { return -b[e].y; }, wd[2]);
+    pack([&](int e) { return -a[e].x; }, wd[3]);
+    pack([&](int e) { return -a[e].y; }, wd[4]);
+    pack([&](int e) { return a[e].y; }, wd[5]);
+#pragma unroll
+    for (int q = 0; q < FX_D; ++q) {
+      o[q * nc + 2 * c] = make_uint4(wd[0][q], wd[2][q], wd[3][q], wd[5][q]);
+      o[q * nc + 2 * c + 1] = make_uint4(wd[1][q], wd[0][q], wd[4][q], wd[3][q]);
+    }
+  } else {
+    pack([&](int e) { return b[e].x; }, wd[0]);
+    pack([&](int e) { return b[e + 4].x; }, wd[1]);
+    pack([&](int e) { return -a[e].x; }, wd[2]);
+    pack([&](int e) { return -a[e + 4].x; }, wd[3]);
+#pragma unroll
+    for (int q = 0; q < FX_D; ++q) o[q * nc + c] = make_uint4(wd[0][q], wd[2][q], wd[1][q], wd[3][q]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// results
+// ---------------------------------------------------------------------------
+// Sum of the slots of (row block, real column), unscaled.
+__device__ __forceinline__ double fx_total(const FxRows& rb, const double* __restrict__ partial, int nc, int col,
+                                           int r) {
+  double s = 0.0;
+  for (int q = 0; q < rb.nseg; ++q) s += partial[((size_t)(rb.slot0 + q) * nc + col) * FX_M + r];
+  return s;
+}
+
+constexpr double kFxUnit = 72057594037927936.0;  // 256^7
+
+// 1/p for a power of two p (0 for 0)
+__device__ __forceinline__ double fx_inverse(double p) {
+  return p > 0.0 ? __longlong_as_double((2046LL << 52) - __double_as_longlong(p)) : 0.0;
+}
+
+struct FxOut {
+  const FxRows* rows;
+  const double* partial;
+  const double* rowscale;
+  const unsigned long long* colmax;
+  const int* flag;
+  const int64_t* rowptr;  // correction, null when there is none
+  const int32_t* col;
+  const double* val;
+  const double* x;
+  double* y;
+  int64_t ldx, ldy;
+  int c0, ncol, nall, nc;
+  double scale, ar, ai, br, bi;
+  bool beta_zero;
+};
+
+template <bool CPLX>
+__global__ void __launch_bounds__(FX_M) fx_finish(FxOut o) {
+  if (*o.flag) return;
+  const FxRows rb = o.rows[blockIdx.x];
+  const int r = threadIdx.x, c = blockIdx.y, cg = o.c0 + c;
+  if (r >= rb.nrows) return;
+  const int64_t row = rb.row0 + r;
+  const double pb = fx_scale(__longlong_as_double((long long)o.colmax[(int64_t)rb.surf * o.nall + cg]));
+  // sums are in units of 256^7 / (pa pb)
+  const double u = fx_inverse(o.rowscale[row]) * fx_inverse(pb) * (o.scale * kFxUnit);
+  double sr, si = 0.0;
+  if (CPLX) {
+    sr = u * fx_total(rb, o.partial, o.nc, 2 * c, r);
+    si = u * fx_total(rb, o.partial, o.nc, 2 * c + 1, r);
+  } else {
+    sr = u * fx_total(rb, o.partial, o.nc, c, r);
+  }
+  if (o.rowptr) {
+    for (int64_t p = o.rowptr[row]; p < o.rowptr[row + 1]; ++p) {
+      const int64_t j = (int64_t)cg * o.ldx + o.col[p];
+      if (CPLX) {
+        const double2 v = reinterpret_cast<const double2*>(o.val)[p], xv = reinterpret_cast<const double2*>(o.x)[j];
+        sr = fma(v.x, xv.x, fma(-v.y, xv.y, sr));
+        si = fma(v.x, xv.y, fma(v.y, xv.x, si));
+      } else {
+        sr = fma(o.val[p], o.x[j], sr);
+      }
+    }
+  }
+  const int64_t q = (int64_t)cg * o.ldy + row;
+  if (CPLX) {
+    double2* Y = reinterpret_cast<double2*>(o.y);
+    double yr = o.ar * sr - o.ai * si, yi = o.ar * si + o.ai * sr;
+    if (!o.beta_zero) {
+      const double2 yo = Y[q];
+      yr += o.br * yo.x - o.bi * yo.y;
+      yi += o.br * yo.y + o.bi * yo.x;
+    }
+    Y[q] = make_double2(yr, yi);
+  } else {
+    double v = o.ar * sr;
+    if (!o.beta_zero) v += o.br * o.y[q];
+    o.y[q] = v;
+  }
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(FX_M) fx_theta_finish(const FxRows* __restrict__ rows,
+                                                        const double* __restrict__ partial,
+                                                        const double* __restrict__ rowscale,
+                                                        const unsigned long long* __restrict__ colmax, int ns, int nc,
+                                                        const int* __restrict__ flag, double2* __restrict__ out) {
+  if (*flag) return;
+  const FxRows rb = rows[blockIdx.x];
+  const int r = threadIdx.x, c = blockIdx.y;
+  if (r >= rb.nrows) return;
+  const int64_t row = rb.row0 + r;
+  const double u = fx_inverse(rowscale[row]) *
+                   fx_inverse(fx_scale(__longlong_as_double((long long)colmax[c]))) * (1.0 / (4 * kPi) * kFxUnit);
+  double2 v = make_double2(0.0, 0.0);
+  if (CPLX) {
+    v.x = u * fx_total(rb, partial, nc, 2 * c, r);
+    v.y = u * fx_total(rb, partial, nc, 2 * c + 1, r);
+  } else {
+    v.x = u * fx_total(rb, partial, nc, c, r);
+  }
+  out[row * ns + c] = v;
+}
+
+// ---------------------------------------------------------------------------
+// host
+// ---------------------------------------------------------------------------
+template <class F>
+static void fx_dispatch(int pde, int kind, F&& f) {
+  auto by = [&](auto pc) {
+    constexpr int P = decltype(pc)::value;
+    switch (kind) {
+      case SL: return f(pc, std::integral_constant<int, SL>());
+      case DL: return f(pc, std::integral_constant<int, DL>());
+      case ADL: return f(pc, std::integral_constant<int, ADL>());
+      case HS: return f(pc, std::integral_constant<int, HS>());
+      case CF: return f(pc, std::integral_constant<int, CF>());
+      case FX_THETA: return f(pc, std::integral_constant<int, FX_THETA>());
+      default: return f(pc, std::integral_constant<int, FX_THETA_D>());
+    }
+    (void)P;
+  };
+  if (pde == HELMHOLTZ)
+    by(std::integral_constant<int, HELMHOLTZ>());
+  else
+    by(std::integral_constant<int, LAPLACE>());
+}
+
+static FxConst fx_const(const FxProblem& p) {
+  return FxConst{p.k,     p.k * FX_TAB / (2 * kPi), p.c1[0], p.c1[1], p.c2[0], p.c2[1],
+                 p.k * p.c1[0], p.k * p.c1[1]};
+}
+
+const int* fx_flag(const inti_ctx* ctx) { return ctx->fx.work.as<int>(); }
+
+// Where the contraction is the faster form.  Below about 2e6 pairs (1,400
+// nodes squared) the FP64 MMA kernel's single launch is as fast: 8 complex
+// columns at 1,200 nodes take 123 us either way, at 1,728 nodes 170 us against
+// 64 us here (64 columns 407 against 125 us).  Theta pays for its plan (row
+// bounds, work lists) every time, about 0.1 ms: real values break even near
+// 5e7 pairs (7,000 nodes), complex ones near 2e7.
+bool fx_pays(int pde, int kind, double pairs) {
+  if (kind < FX_THETA) return pairs >= 2e6;
+  return pairs >= (pde == HELMHOLTZ ? 2e7 : 5e7);
+}
+
+// Columns of one pass: a multiple of eight, at least 16, at most 64.
+static int fx_width(int real_columns) { return std::min(FX_NMAX, std::max(16, (real_columns + 7) / 8 * 8)); }
+// work: [flag, counter per pass (up to 63) | column bounds]
+constexpr int FX_COUNTERS = 64;
+static size_t fx_work_bytes(int nsurf, int ncols) {
+  return sizeof(int) * FX_COUNTERS + sizeof(unsigned long long) * (size_t)nsurf * ncols;
+}
+
+static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
+  const int J = FX_K / fx_na(p.pde, p.kind);
+  const int nsurf = (int)p.row.size();
+  std::vector<FxRows> rows;
+  std::vector<FxItem> items;
+  std::vector<FxStage> stages;
+  plan.ntargets = 0;
+  double total = 0.0;
+  for (int s = 0; s < nsurf; ++s)
+    total += (double)((p.nrow[s] + FX_M - 1) / FX_M) * (double)((p.nsrc[s] + J - 1) / J);
+  // Runs of about a sixth of an SM's share of the stages (a short tail), at
+  // least four stages (an item costs about one stage in hand-over).
+  const int run = (int)std::max(4.0, std::ceil(total / (6.0 * ctx->num_sms)));
+  plan.nslots = 0;
+  for (int s = 0; s < nsurf; ++s) {
+    const int stage0 = (int)stages.size(), nst = (int)((p.nsrc[s] + J - 1) / J);
+    for (int t = 0; t < nst; ++t)
+      stages.push_back(FxStage{p.src[s] + (int64_t)t * J, (int32_t)std::min<int64_t>(J, p.nsrc[s] - (int64_t)t * J), s});
+    const int nseg = std::max(1, (nst + run - 1) / run);
+    for (int64_t r = 0; r < p.nrow[s]; r += FX_M) {
+      const int rb = (int)rows.size();
+      rows.push_back(FxRows{p.row[s] + r, (int32_t)std::min<int64_t>(FX_M, p.nrow[s] - r), plan.nslots, nseg, s, stage0,
+                            nst});
+      for (int q = 0; q < nseg; ++q) {
+        const int a = (int)((int64_t)nst * q / nseg), b = (int)((int64_t)nst * (q + 1) / nseg);
+        items.push_back(FxItem{rb, a, b - a, plan.nslots + q});
+      }
+      plan.nslots += nseg;
+    }
+    plan.ntargets = std::max(plan.ntargets, p.row[s] + p.nrow[s]);
+  }
+  std::stable_sort(items.begin(), items.end(), [](const FxItem& a, const FxItem& b) { return a.nstages > b.nstages; });
+  plan.nrows = (int)rows.size();
+  plan.nitems = (int)items.size();
+  plan.nstages = (int)stages.size();
+  plan.nsurf = nsurf;
+  // one upload (rows | stages | items): each copy from pageable memory waits
+  // for the stream, and a correction builds its plan every time
+  const size_t b_rows = sizeof(FxRows) * rows.size(), b_stages = sizeof(FxStage) * stages.size(),
+               b_items = sizeof(FxItem) * items.size();
+  std::vector<unsigned char> h(b_rows + b_stages + b_items);
+  std::memcpy(h.data(), rows.data(), b_rows);
+  std::memcpy(h.data() + b_rows, stages.data(), b_stages);
+  std::memcpy(h.data() + b_rows + b_stages, items.data(), b_items);
+  plan.tables.ensure(h.size());
+  INTI_CUDA(cudaMemcpyAsync(plan.tables.p, h.data(), h.size(), cudaMemcpyHostToDevice, ctx->stream));
+  plan.rows = plan.tables.as<FxRows>();
+  plan.stages = reinterpret_cast<const FxStage*>(plan.tables.as<unsigned char>() + b_rows);
+  plan.items = reinterpret_cast<const FxItem*>(plan.tables.as<unsigned char>() + b_rows + b_stages);
+  plan.records.ensure(sizeof(double) * FX_REC * J * stages.size());
+  plan.tiles.ensure(sizeof(double4) * stages.size());
+  plan.rowscale.ensure(sizeof(double) * std::max<int64_t>(plan.ntargets, 1));
+  plan.meta.ensure(sizeof(unsigned long long) * 2);
+  INTI_CUDA(cudaMemsetAsync(plan.meta.p, 0, sizeof(unsigned long long) * 2, ctx->stream));
+  fx_plan_sources<<<(plan.nstages + 7) / 8, 256, 0, ctx->stream>>>(
+      plan.nstages, J, plan.stages, p.coords, p.normals, plan.records.as<double>(),
+      plan.tiles.as<double4>(), plan.meta.as<unsigned long long>());
+  fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
+    constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
+    fx_plan_rows<P, K><<<(unsigned)plan.nrows * (FX_M / kPlanRows / 8), 256, 0, ctx->stream>>>(
+        plan.nrows, plan.rows, p.tcoords, p.tnormals, plan.stages, plan.tiles.as<double4>(),
+        plan.records.as<double>(), fx_const(p), plan.rowscale.as<double>(), plan.meta.as<unsigned long long>());
+    INTI_CUDA(cudaFuncSetAttribute(fx_contract_kernel<P, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   FxShape<P, K>::SMEM));
+  });
+  ctx->launches += 2;
+  INTI_CUDA(cudaGetLastError());
+  if (!ctx->fx.tab.p) {
+    std::vector<double2> t(FX_TAB);
+    const long double d = (long double)(2.0 * kPi / FX_TAB);
+    for (int m = 0; m < FX_TAB; ++m) t[m] = make_double2((double)cosl(m * d), (double)sinl(m * d));
+    ctx->fx.tab.ensure(sizeof(double2) * FX_TAB);
+    INTI_CUDA(cudaMemcpyAsync(ctx->fx.tab.p, t.data(), sizeof(double2) * FX_TAB, cudaMemcpyHostToDevice, ctx->stream));
+  }
+  plan.ready = true;
+}
+
+bool fx_prepare(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, int ncols) {
+  const int nc = fx_width(ncols * (p.pde == HELMHOLTZ ? 2 : 1));
+  auto digits = [&] { return (size_t)plan.nstages * nc * FX_D * FX_K; };
+  auto partial = [&] { return sizeof(double) * (size_t)plan.nslots * nc * FX_M; };
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  INTI_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return false;
+  try {
+    if (!plan.ready) fx_plan(ctx, p, plan);
+    ctx->fx.bdig.ensure(digits());
+    ctx->fx.partial.ensure(partial());
+    ctx->fx.work.ensure(fx_work_bytes(plan.nsurf, ncols));
+  } catch (const Error& e) {
+    if (e.code != INTI_E_NOMEM) throw;
+    return false;
+  }
+  return true;
+}
+
+static unsigned long long* fx_colmax_ptr(inti_ctx* ctx) {
+  return reinterpret_cast<unsigned long long*>(ctx->fx.work.as<int>() + FX_COUNTERS);
+}
+
+static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc, int* counter) {
+  FxArgs a;
+  a.rows = plan.rows;
+  a.items = plan.items;
+  a.nitems = plan.nitems;
+  a.nc = nc;
+  a.tcoords = p.tcoords;
+  a.tnormals = p.tnormals;
+  a.rowscale = plan.rowscale.as<double>();
+  a.records = plan.records.as<double>();
+  a.bdig = ctx->fx.bdig.as<unsigned char>();
+  a.tab = ctx->fx.tab.as<double2>();
+  a.partial = ctx->fx.partial.as<double>();
+  a.c = fx_const(p);
+  a.counter = counter;
+  a.flag = fx_flag(ctx);
+  a.err = ctx->err_flag.as<int>();
+  ctx->flag_armed = true;
+  fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
+    constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
+    fx_contract_kernel<P, K><<<std::min(ctx->num_sms, plan.nitems), FX_THREADS, FxShape<P, K>::SMEM, ctx->stream>>>(a);
+  });
+  ctx->launches++;
+  INTI_CUDA(cudaGetLastError());
+}
+
+void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_csr* corr, const double* x,
+              int64_t ldx, double* y, int64_t ldy, int nrhs, const double* alpha, const double* beta) {
+  const bool cplx = p.pde == HELMHOLTZ;
+  const int comps = cplx ? 2 : 1;
+  const int width = FX_NMAX / comps;  // columns per pass
+  INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(plan.nsurf, nrhs), ctx->stream));
+  int* flag = ctx->fx.work.as<int>();
+  unsigned long long* colmax = fx_colmax_ptr(ctx);
+  const FxStage* st = plan.stages;
+  const unsigned long long* meta = plan.meta.as<unsigned long long>();
+  auto by_type = [&](auto cc) {
+    constexpr bool C = decltype(cc)::value;
+    const int runs = (plan.nstages + kMaxRun - 1) / kMaxRun;
+    fx_colmax<C><<<dim3((runs + 7) / 8, nrhs), 256, 0, ctx->stream>>>(plan.nstages, st, p.weights, x, ldx, nrhs, colmax);
+    fx_check<<<1, 256, 0, ctx->stream>>>(plan.nsurf * nrhs, colmax, meta, flag);
+    ctx->launches += 2;
+    int pass = 0;
+    for (int c0 = 0; c0 < nrhs; c0 += width, ++pass) {
+      const int ncol = std::min(width, nrhs - c0), nc = fx_width(ncol * comps);
+      const int64_t threads = (int64_t)plan.nstages * 4 * (nc / comps);
+      fx_pack<C><<<(unsigned)((threads + 127) / 128), 128, 0, ctx->stream>>>(
+          plan.nstages, st, p.weights, x, ldx, c0, ncol, nrhs, nc, colmax, flag, ctx->fx.bdig.as<unsigned char>());
+      ctx->launches++;
+      const int slot = 1 + pass % (FX_COUNTERS - 1);
+      if (pass >= FX_COUNTERS - 1) INTI_CUDA(cudaMemsetAsync(flag + slot, 0, sizeof(int), ctx->stream));
+      fx_run(ctx, p, plan, nc, flag + slot);
+      FxOut o;
+      o.rows = plan.rows;
+      o.partial = ctx->fx.partial.as<double>();
+      o.rowscale = plan.rowscale.as<double>();
+      o.colmax = colmax;
+      o.flag = flag;
+      o.rowptr = corr ? corr->rowptr.as<int64_t>() : nullptr;
+      o.col = corr ? corr->col.as<int32_t>() : nullptr;
+      o.val = corr ? corr->val.as<double>() : nullptr;
+      o.x = x;
+      o.y = y;
+      o.ldx = ldx;
+      o.ldy = ldy;
+      o.c0 = c0;
+      o.ncol = ncol;
+      o.nall = nrhs;
+      o.nc = nc;
+      o.scale = 1.0 / (4 * kPi);
+      o.ar = alpha ? alpha[0] : 1.0;
+      o.ai = alpha ? alpha[1] : 0.0;
+      o.br = beta ? beta[0] : 0.0;
+      o.bi = beta ? beta[1] : 0.0;
+      o.beta_zero = o.br == 0.0 && o.bi == 0.0;
+      fx_finish<C><<<dim3(plan.nrows, ncol), FX_M, 0, ctx->stream>>>(o);
+      ctx->launches++;
+    }
+  };
+  if (cplx)
+    by_type(std::true_type());
+  else
+    by_type(std::false_type());
+  INTI_CUDA(cudaGetLastError());
+}
+
+void fx_theta(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const double2* g0, const double2* g1, int ns,
+              double2* out) {
+  const bool cplx = p.pde == HELMHOLTZ;
+  const int nc = fx_width(ns * (cplx ? 2 : 1));
+  INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(plan.nsurf, ns), ctx->stream));
+  int* flag = ctx->fx.work.as<int>();
+  unsigned long long* colmax = fx_colmax_ptr(ctx);
+  const int64_t n = p.nsrc[0];
+  fx_theta_max<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(n, ns, cplx, p.weights, g0, g1, colmax);
+  fx_check<<<1, 32, 0, ctx->stream>>>(ns, colmax, plan.meta.as<unsigned long long>(), flag);
+  const int64_t threads = (int64_t)plan.nstages * 4 * (cplx ? nc / 2 : nc);
+  auto by_type = [&](auto cc) {
+    constexpr bool C = decltype(cc)::value;
+    fx_theta_pack<C><<<(unsigned)((threads + 127) / 128), 128, 0, ctx->stream>>>(
+        plan.nstages, plan.stages, p.weights, g0, g1, ns, nc, colmax, flag,
+        ctx->fx.bdig.as<unsigned char>());
+    fx_run(ctx, p, plan, nc, flag + 1);
+    fx_theta_finish<C><<<dim3(plan.nrows, ns), FX_M, 0, ctx->stream>>>(
+        plan.rows, ctx->fx.partial.as<double>(), plan.rowscale.as<double>(), colmax, ns, nc, flag, out);
+  };
+  if (cplx)
+    by_type(std::true_type());
+  else
+    by_type(std::false_type());
+  ctx->launches += 4;
+  INTI_CUDA(cudaGetLastError());
+}
+
+}  // namespace inti

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "common.h"
+#include "contract_i8.h"
 #include "device_common.cuh"
 #include "fp64_mma.cuh"
 #include "internal.h"
@@ -275,7 +276,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) dim_theta_mma(
     const double* __restrict__ x,
     const double* __restrict__ nrm, const double* __restrict__ w, const double2* __restrict__ g0,
     const double2* __restrict__ g1, double k, double kT, double delta, const double2* __restrict__ tab_g,
-    int tiles_per_split, double2* __restrict__ partial) {
+    int tiles_per_split, double2* __restrict__ partial, const int* __restrict__ only_if) {
+  if (only_if && !*only_if) return;
   using TM = ThetaMma<PDE, WIDE>;
   using Sh = typename TM::Sh;
   constexpr bool CPLX = PDE == HELMHOLTZ;
@@ -399,12 +401,15 @@ __global__ void __launch_bounds__(kMmaThreads, 2) dim_theta_mma(
   }
 }
 
-// theta[i,k] = mu_i * B(x_i, xs_k) + sum_s partial[s][i][k]
+// theta[i,k] = mu_i * B(x_i, xs_k) + sum_s partial[s][i][k]; one slot when the
+// product came from the contraction (its flag is set and zero)
 template <int PDE, int DIM, bool DERIV>
 __global__ void dim_theta_reduce(int64_t m, int ns, int split, const double* __restrict__ tx,
                                  const double* __restrict__ tn, const double* __restrict__ xs,
                                  const double* __restrict__ mu, double k,
-                                 const double2* __restrict__ partial, double2* __restrict__ theta) {
+                                 const double2* __restrict__ partial, double2* __restrict__ theta,
+                                 const int* __restrict__ only_if) {
+  if (only_if && !*only_if) split = 1;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= m * ns) return;
   const int64_t i = t / ns;
@@ -765,13 +770,35 @@ static void dim_theta_run(inti_ctx* ctx, int pde, double k_re, const inti_quad* 
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         });
         ProfScope pd(ctx, "dim");
+        // on the INT8 tensor path where that pays; this kernel then stands by
+        // for traces that do not fit it
+        const int* only_if = nullptr;
+        FxProblem fp;
+        fp.pde = P;
+        fp.kind = DV ? FX_THETA_D : FX_THETA;
+        fp.k = k_re;
+        fp.tcoords = tx;
+        fp.tnormals = tn;
+        fp.coords = X;
+        fp.normals = NR;
+        fp.weights = W;
+        fp.row = fp.src = {0};
+        fp.nrow = {m};
+        fp.nsrc = {n};
+        FxPlan& plan = ctx->dimwork.plan;
+        plan.ready = false;  // another geometry
+        if (fx_pays(P, fp.kind, (double)m * (double)n) && fx_prepare(ctx, fp, plan, ns)) {
+          fx_theta(ctx, fp, plan, wk.g0.as<double2>(), wk.g1.as<double2>(), ns, wk.part.as<double2>());
+          only_if = fx_flag(ctx);
+        }
         kern<<<dim3((unsigned)blocks, (unsigned)split), kMmaThreads, smem, ctx->stream>>>(
             m, n, ns, tx, tn, X, NR, W, wk.g0.as<double2>(), wk.g1.as<double2>(), k_re,
             k_re * kExpiTable / (2 * kPi), 2 * kPi / kExpiTable, P == HELMHOLTZ ? expi_table_f64(ctx) : nullptr, tps,
-            wk.part.as<double2>());
+            wk.part.as<double2>(), only_if);
         ctx->launches++;
         dim_theta_reduce<P, D, DV><<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(
-            m, ns, split, tx, tn, wk.d_xs.as<double>(), mu, k_re, wk.part.as<double2>(), wk.theta.as<double2>());
+            m, ns, split, tx, tn, wk.d_xs.as<double>(), mu, k_re, wk.part.as<double2>(), wk.theta.as<double2>(),
+            only_if);
         ctx->launches++;
       };
       auto mma_d = [&](auto wide_c) {
@@ -810,7 +837,7 @@ static void dim_theta_run(inti_ctx* ctx, int pde, double k_re, const inti_quad* 
           wk.part.as<double2>());
       ctx->launches++;
       dim_theta_reduce<P, D, DV><<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(
-          m, ns, split, tx, tn, wk.d_xs.as<double>(), mu, k_re, wk.part.as<double2>(), wk.theta.as<double2>());
+          m, ns, split, tx, tn, wk.d_xs.as<double>(), mu, k_re, wk.part.as<double2>(), wk.theta.as<double2>(), nullptr);
       ctx->launches++;
     };
     auto by_ns = [&](auto deriv_c) {

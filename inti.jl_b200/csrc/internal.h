@@ -34,6 +34,7 @@ struct inti_op {
   inti::DevBuf tpartial, tpacked, tones;  // A^T: partials, packed target records, unit weights
   inti::DevBuf gpartial;  // source gradients: split x n x (2 dim + 2)
   inti::DevBuf mx, my;    // staging of host columns for multi-column applies
+  inti::FxPlan fx;        // multi-column products on the INT8 tensor path
   int split = 1;
   int tpt = 4;  // targets per thread of the pair kernel (autotuned with split)
   int tsplit = 1, ttpt = 4;  // A^T launch shape
