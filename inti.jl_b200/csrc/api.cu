@@ -132,6 +132,7 @@ PairLaunch make_launch(inti_op* op, const double* xdev) {
     L.symm = true;
     L.sym_nb = op->sym_nb;
     L.sym_nitems = op->sym_nitems;
+    L.sym_sub = op->sym_sub;
     L.sym_items = op->sym_tab.as<int32_t>();
     L.sym_rowptr = L.sym_items + 3 * op->sym_nitems;
     L.sym_rowitems = L.sym_rowptr + op->sym_nb + 1;
@@ -171,7 +172,7 @@ void op_apply_device(inti_op* op, const double* x, double* y, const double* alph
     // (with panels pair_launch clears them before each panel)
     if (L.sym_npanels <= 1) {
       const size_t pb = (size_t)pair_partial_bytes(op->pde, op->precision);
-      INTI_CUDA(cudaMemsetAsync(L.partial, 0, pb * op->sym_nitems * pair_symm_block(op->tpt), op->ctx->stream));
+      INTI_CUDA(cudaMemsetAsync(L.partial, 0, pb * op->sym_nitems * op->sym_sub * pair_symm_block(op->tpt), op->ctx->stream));
       INTI_CUDA(cudaMemsetAsync(L.zpart, 0, pb * op->sym_nb * op->n_tiles * pair_tile(op->precision),
                                 op->ctx->stream));
     }

@@ -254,6 +254,7 @@ struct PairLaunch {
   // (I, J0, J1), per row block the list of its items, column partials
   bool symm = false;
   int sym_nb = 0, sym_nitems = 0;
+  int sym_sub = 1;                        // CTAs (and row-partial slots) per item
   const int32_t* sym_items = nullptr;     // 3 x nitems
   const int32_t* sym_rowptr = nullptr;    // nb + 1
   const int32_t* sym_rowitems = nullptr;  // nitems
@@ -301,6 +302,9 @@ int pair_symm_block(int tpt);
 void pair_symm_plan(int64_t n, int tpt, int ch, int pcols, std::vector<int32_t>& table,
                     std::vector<SymPanel>& panels, int& nb, int& nitems);
 int pair_symm_default_ch(const inti_ctx* ctx, int pde, int kind, int dim, int precision, int64_t n, int tpt);
+// CTAs per item: small operators, whose items (one source block each) do not
+// fill the device, give every item's block to several CTAs.
+int pair_symm_sub(const inti_ctx* ctx, int tpt, int ch, int nitems);
 // Choose the split for a problem on this device.
 int pair_plan_split(const inti_ctx* ctx, int pde, int kind, int dim, int precision, int64_t m,
                     int64_t n, int tpt = 4);

@@ -42,7 +42,7 @@ struct inti_op {
   // column partials; split holds the source blocks per work item
   bool small = false;  // applies in the single-launch form (pair_small)
   bool symm = false;
-  int sym_nb = 0, sym_nitems = 0;
+  int sym_nb = 0, sym_nitems = 0, sym_sub = 1;
   inti::DevBuf sym_tab;
   // panels of the work items (one unless the column partials of the whole
   // operator would pass the partial budget); the partials and running sums

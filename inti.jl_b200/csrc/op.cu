@@ -234,7 +234,8 @@ void op_symm_configure(inti_op* op, int tpt, int ch) {
   const bool panels = op->sym_panels.size() > 1;
   op->sym_zld = panels ? (int64_t)pcols * pair_symm_block(tpt) : npad;
   inti_ctx* ctx = op->ctx;
-  const size_t yb = (size_t)pb * nitems * pair_symm_block(tpt);
+  op->sym_sub = panels ? 1 : pair_symm_sub(ctx, tpt, ch_eff, nitems);
+  const size_t yb = (size_t)pb * nitems * op->sym_sub * pair_symm_block(tpt);
   if (ctx->sym_ypart.bytes < yb) ctx->sym_ypart.ensure(yb + yb / 4);
   ctx->sym_zpart.ensure((size_t)pb * nb * op->sym_zld);
   if (panels) ctx->sym_acc.ensure(sizeof(double) * (op->pde == INTI_HELMHOLTZ ? 2 : 1) * op->source->n);
@@ -339,6 +340,10 @@ void op_autotune(inti_op* op, bool measure) {
     int warmed = 0;
     for (auto& c : cand) {
       op_symm_configure(op, c.first, c.second);
+      // FP32C: the columns' sums over a row block are FP32, so the targets per
+      // thread decide the results' last digits; the choice is made on whole
+      // blocks, independent of how their parts are spread
+      if (op->precision == INTI_FP32C) op->sym_sub = 1;
       PairLaunch L = make_launch(op, op->xbuf.as<double>());
       if (c.first != warmed) {  // one warm-up per kernel (targets per thread); the others reuse it
         pair_launch(ctx, L);

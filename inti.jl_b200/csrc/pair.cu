@@ -735,6 +735,7 @@ struct SymArgs {
   int64_t npad;           // packed records: nb * BT (zero charges past n)
   const int32_t* items;   // (I, J0, J1) per CTA
   const int32_t* ids;     // row-partial slot of each CTA's item (NULL: the CTA index)
+  int sub;                // CTAs per item: an equal part of its (one) source block each
   const void* packed;
   void* ypart;            // [item][BT]
   void* zpart;            // [nb][zld]: node j of the panel's columns at j - zcol0
@@ -976,7 +977,10 @@ __device__ __forceinline__ void put_partial(double2* p, double r, double i) { *p
 __device__ __forceinline__ void put_partial(float2* p, float r, float) { *p = make_float2(r, 0.f); }
 __device__ __forceinline__ void put_partial(float4* p, float r, float i) { *p = make_float4(r, 0.f, i, 0.f); }
 
-template <int PDE, int KIND, int DIM, class R, int TILE, int TPT>
+// SUB: several CTAs share an item's source block (a.sub > 1).  Without it the
+// tile length is a constant: made a variable it cost 4% at 62,208 nodes, and
+// up to 38 registers.
+template <int PDE, int KIND, int DIM, class R, int TILE, int TPT, bool SUB>
 __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
   using RC = SymRec<PDE, KIND, DIM, R>;
   constexpr bool CPLX = RC::cplx;
@@ -993,11 +997,25 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
   R* stage1 = reinterpret_cast<R*>(smem_raw + kStageBytes);
   R2* tab = reinterpret_cast<R2*>(smem_raw + 2 * kStageBytes);  // Helmholtz only
   R* zsm = reinterpret_cast<R*>(smem_raw + 2 * kStageBytes + (CPLX ? kExpiTable * sizeof(R2) : 0));
-  __shared__ __align__(8) uint64_t full[2];
+  __shared__ __align__(8) uint64_t full[2], tab_full;
+  constexpr bool TMA_TAB = SUB && CPLX && sizeof(R) == 8;  // (FP32 takes the hardware sine and cosine)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int I = a.items[3 * blockIdx.x], J0 = a.items[3 * blockIdx.x + 1], J1 = a.items[3 * blockIdx.x + 2];
+  // SUB: this CTA takes part `part` of the item's one source block
+  const int item = SUB ? blockIdx.x / a.sub : blockIdx.x, part = SUB ? blockIdx.x % a.sub : 0;
+  const int I = a.items[3 * item], J0 = a.items[3 * item + 1], J1 = a.items[3 * item + 2];
+  const int ps = SUB ? BT / a.sub : 0;                           // sources of a part
+  const int64_t j0 = SUB ? (int64_t)J0 * BT + part * ps : 0;     // tile t starts at source j0 + t * TILE
+  auto bytes = [&](int64_t t) {
+    return (SUB ? (uint32_t)min((int64_t)TILE, ps - t * TILE) : (uint32_t)TILE) * (uint32_t)(kStageBytes / TILE);
+  };
   const R* src = static_cast<const R*>(a.packed);
+  if (TMA_TAB && tid == 0) {  // the table's copy does not wait for the kernel before
+    mbar_init(&tab_full, 1);
+    mbar_fence_init();
+    mbar_arrive_expect_tx(&tab_full, kExpiTable * sizeof(R2));
+    bulk_copy_g2s(tab, a.expi, kExpiTable * sizeof(R2), &tab_full);
+  }
   R tg[TPT][NU];
   Acc<R, CPLX> acc[TPT];
 #pragma unroll
@@ -1007,7 +1025,7 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
     for (int c = 0; c < NU; ++c) tg[u][c] = src[i * RC::n + c];
   }
   const R k = R(a.k), kT = R(a.kT), delta = R(a.delta);
-  if (CPLX) {
+  if (CPLX && !TMA_TAB) {
     const R2* g = static_cast<const R2*>(a.expi);
     for (int q = tid; q < kExpiTable; q += kBlock) tab[q] = g[q];
   }
@@ -1017,33 +1035,36 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
     mbar_fence_init();
   }
   __syncthreads();
-  const int64_t t0 = (int64_t)J0 * TPB, t1 = (int64_t)J1 * TPB;
+  const int64_t t0 = SUB ? 0 : (int64_t)J0 * TPB, t1 = SUB ? (ps + TILE - 1) / TILE : (int64_t)J1 * TPB;
   int64_t issued = t0;
   if (tid == 0) {
     for (int s = 0; s < 2 && issued < t1; ++s, ++issued) {
-      mbar_arrive_expect_tx(&full[s], kStageBytes);
-      bulk_copy_g2s(s ? stage1 : stage0, src + issued * TILE * RC::n, kStageBytes, &full[s]);
+      mbar_arrive_expect_tx(&full[s], bytes(issued));
+      bulk_copy_g2s(s ? stage1 : stage0, src + (j0 + issued * TILE) * RC::n, bytes(issued), &full[s]);
     }
   }
   for (int64_t t = t0; t < t1; ++t) {
     const int st = (int)((t - t0) & 1);
     const uint32_t parity = (uint32_t)(((t - t0) >> 1) & 1);
-    const bool ok = mbar_wait_bounded(&full[st], parity);
+    bool ok = mbar_wait_bounded(&full[st], parity);
+    if (TMA_TAB && t == t0) ok = mbar_wait_bounded(&tab_full, 0) && ok;
     if (!__syncthreads_and(ok)) {
       if (tid == 0) {
         atomicExch(a.err, kErrWaitTimeout);
+        if (TMA_TAB) mbar_wait_bounded(&tab_full, 0);
         for (int64_t q = t + 1; q < issued; ++q)
           mbar_wait_bounded(&full[(q - t0) & 1], (uint32_t)(((q - t0) >> 1) & 1));
       }
       return;
     }
     const R* sp = st ? stage1 : stage0;
-    const bool diag = t / TPB == I;
+    const bool diag = SUB ? J0 == I : t / TPB == I;
+    const int cnt = SUB ? (int)min((int64_t)TILE, ps - t * TILE) : TILE;
     R* zb = zsm + st * (kWarps * TILE * 2);
     if (diag) {
 #pragma unroll 1
-      for (int g = 0; g < TILE; g += kGroup) {
-#pragma unroll 2
+      for (int g = 0; g < cnt; g += kGroup) {
+#pragma unroll(SUB ? 8 / TPT : 2)
         for (int s = 0; s < kGroup; ++s) {
           const R* rec = sp + (g + s) * RC::n;
 #pragma unroll
@@ -1065,7 +1086,7 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
       }
     } else {
 #pragma unroll 1
-      for (int g = 0; g < TILE; g += kGroup) {
+      for (int g = 0; g < cnt; g += kGroup) {
 #pragma unroll 1
         for (int s = 0; s < kGroup; s += 4) {
           R zr[4], zi[4];
@@ -1092,8 +1113,8 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
     }
     __syncthreads();  // the stage is read and this tile's column sums are in zb
     if (!diag) {
-      P* zp = static_cast<P*>(a.zpart) + (int64_t)I * a.zld + (t * TILE - a.zcol0);
-      for (int s = tid; s < TILE; s += kBlock) {
+      P* zp = static_cast<P*>(a.zpart) + (int64_t)I * a.zld + (j0 + t * TILE - a.zcol0);
+      for (int s = tid; s < cnt; s += kBlock) {
         R vr = zb[s * 2], vi = zb[s * 2 + 1];
 #pragma unroll
         for (int w = 1; w < kWarps; ++w) {
@@ -1105,12 +1126,12 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
     }
     if (tid == 0 && issued < t1) {
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&full[st], kStageBytes);
-      bulk_copy_g2s(st ? stage1 : stage0, src + issued * TILE * RC::n, kStageBytes, &full[st]);
+      mbar_arrive_expect_tx(&full[st], bytes(issued));
+      bulk_copy_g2s(st ? stage1 : stage0, src + (j0 + issued * TILE) * RC::n, bytes(issued), &full[st]);
       ++issued;
     }
   }
-  P* out = static_cast<P*>(a.ypart) + (int64_t)(a.ids ? a.ids[blockIdx.x] : (int)blockIdx.x) * BT;
+  P* out = static_cast<P*>(a.ypart) + (int64_t)((a.ids ? a.ids[item] : item) * (SUB ? a.sub : 1) + part) * BT;
 #pragma unroll
   for (int u = 0; u < TPT; ++u) store_partial(out + u * kBlock + tid, acc[u]);
 }
@@ -1195,7 +1216,7 @@ __device__ __forceinline__ void pair_x2_step(const float2 (&t)[RecX2<KIND>::vals
   }
 }
 
-template <int KIND, int TPT>
+template <int KIND, int TPT, bool SUB>
 __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
   constexpr int TILE = kTile32;
   constexpr int NR = RecX2<KIND>::n, NV = RecX2<KIND>::vals;
@@ -1211,7 +1232,14 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
   __shared__ __align__(8) uint64_t full[2];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int I = a.items[3 * blockIdx.x], J0 = a.items[3 * blockIdx.x + 1], J1 = a.items[3 * blockIdx.x + 2];
+  // SUB: this CTA takes part `part` of the item's one source block
+  const int item = SUB ? blockIdx.x / a.sub : blockIdx.x, part = SUB ? blockIdx.x % a.sub : 0;
+  const int I = a.items[3 * item], J0 = a.items[3 * item + 1], J1 = a.items[3 * item + 2];
+  const int ps = SUB ? BT / a.sub : 0;                           // sources of a part
+  const int64_t j0 = SUB ? (int64_t)J0 * BT + part * ps : 0;     // tile t starts at source j0 + t * TILE
+  auto bytes = [&](int64_t t) {
+    return (SUB ? (uint32_t)min((int64_t)TILE, ps - t * TILE) : (uint32_t)TILE) * (uint32_t)(kStageBytes / TILE);
+  };
   const float* src = static_cast<const float*>(a.packed);
   float2 tg[NP][NV];  // (target 2p, target 2p + 1), value c
   float2 g[NP];       // group sums per lane
@@ -1238,12 +1266,12 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
     mbar_fence_init();
   }
   __syncthreads();
-  const int64_t t0 = (int64_t)J0 * TPB, t1 = (int64_t)J1 * TPB;
+  const int64_t t0 = SUB ? 0 : (int64_t)J0 * TPB, t1 = SUB ? (ps + TILE - 1) / TILE : (int64_t)J1 * TPB;
   int64_t issued = t0;
   if (tid == 0) {
     for (int s = 0; s < 2 && issued < t1; ++s, ++issued) {
-      mbar_arrive_expect_tx(&full[s], kStageBytes);
-      bulk_copy_g2s(s ? stage1 : stage0, src + issued * TILE * NR, kStageBytes, &full[s]);
+      mbar_arrive_expect_tx(&full[s], bytes(issued));
+      bulk_copy_g2s(s ? stage1 : stage0, src + (j0 + issued * TILE) * NR, bytes(issued), &full[s]);
     }
   }
   for (int64_t t = t0; t < t1; ++t) {
@@ -1259,11 +1287,12 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
       return;
     }
     const float* sp = st ? stage1 : stage0;
-    const bool diag = t / TPB == I;
+    const bool diag = SUB ? J0 == I : t / TPB == I;
+    const int cnt = SUB ? (int)min((int64_t)TILE, ps - t * TILE) : TILE;
     float* zb = zsm + st * (kWarps * TILE * 2);
     if (diag) {
 #pragma unroll 1
-      for (int gq = 0; gq < TILE; gq += kGroup) {
+      for (int gq = 0; gq < cnt; gq += kGroup) {
 #pragma unroll 2
         for (int s = 0; s < kGroup; ++s) {
           const float2* rec = reinterpret_cast<const float2*>(sp + (gq + s) * NR);
@@ -1275,7 +1304,7 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
       }
     } else {
 #pragma unroll 1
-      for (int gq = 0; gq < TILE; gq += kGroup) {
+      for (int gq = 0; gq < cnt; gq += kGroup) {
 #pragma unroll 1
         for (int s = 0; s < kGroup; s += 4) {
           float zr[4];
@@ -1300,8 +1329,8 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
     }
     __syncthreads();  // the stage is read and this tile's column sums are in zb
     if (!diag) {
-      float2* zp = static_cast<float2*>(a.zpart) + (int64_t)I * a.zld + (t * TILE - a.zcol0);
-      for (int s = tid; s < TILE; s += kBlock) {
+      float2* zp = static_cast<float2*>(a.zpart) + (int64_t)I * a.zld + (j0 + t * TILE - a.zcol0);
+      for (int s = tid; s < cnt; s += kBlock) {
         float vr = zb[s * 2];
 #pragma unroll
         for (int w = 1; w < kWarps; ++w) vr += zb[(w * TILE + s) * 2];
@@ -1310,12 +1339,12 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
     }
     if (tid == 0 && issued < t1) {
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&full[st], kStageBytes);
-      bulk_copy_g2s(st ? stage1 : stage0, src + issued * TILE * NR, kStageBytes, &full[st]);
+      mbar_arrive_expect_tx(&full[st], bytes(issued));
+      bulk_copy_g2s(st ? stage1 : stage0, src + (j0 + issued * TILE) * NR, bytes(issued), &full[st]);
       ++issued;
     }
   }
-  float2* out = static_cast<float2*>(a.ypart) + (int64_t)(a.ids ? a.ids[blockIdx.x] : (int)blockIdx.x) * BT;
+  float2* out = static_cast<float2*>(a.ypart) + (int64_t)((a.ids ? a.ids[item] : item) * (SUB ? a.sub : 1) + part) * BT;
 #pragma unroll
   for (int u = 0; u < TPT; ++u) out[u * kBlock + tid] = make_float2(hr[u], lr[u]);
 }
@@ -1386,31 +1415,82 @@ __global__ void __launch_bounds__(kFoldNodes * kFoldSlices) pair_symm_fold_kerne
 
 struct SymEpi {
   int64_t npad;
-  int bt;
+  int bt, lsub;             // block, log2 of the slots per item
   const int32_t* rowptr;    // nb + 1
   const int32_t* rowitems;  // items of each row block
   const void* zpart;
 };
 
+// Row i of the product.  Eight threads per node, each summing every eighth
+// of its partials (the slots of its block's items, then the column partials
+// of the blocks above) and of its correction row's entries; the eight sums
+// are added in a fixed order.  One thread per node summed them one after
+// another, with 12 blocks of 256 threads at 3,072 nodes.
+constexpr int kEpiNodes = 32, kEpiSlices = 8;
+
 template <class P, bool CPLX>
-__global__ void pair_symm_epilogue_kernel(EpiArgs e, SymEpi s) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= e.m) return;
-  const int B = (int)(i / s.bt), il = (int)(i % s.bt);
-  const P* yp = static_cast<const P*>(e.partial);
-  const P* zp = static_cast<const P*>(s.zpart);
-  double sr = 0.0, si = 0.0;
-  for (int q = s.rowptr[B]; q < s.rowptr[B + 1]; ++q) {
-    const double2 v = load_partial(yp + (int64_t)s.rowitems[q] * s.bt + il);
-    sr += v.x;
-    si += v.y;
+__global__ void __launch_bounds__(kEpiNodes * kEpiSlices) pair_symm_epilogue_kernel(EpiArgs e, SymEpi s) {
+  __shared__ double4 part[kEpiSlices][kEpiNodes];
+  __shared__ int32_t list[kEpiNodes * kEpiSlices];
+  const int tn = threadIdx.x % kEpiNodes, sl = threadIdx.x / kEpiNodes;
+  const int64_t i0 = blockIdx.x * (int64_t)kEpiNodes, i = i0 + tn;
+  const bool live = i < e.m;
+  double4 c = make_double4(0.0, 0.0, 0.0, 0.0);  // pair sum, correction sum
+  if (live && e.rowptr) {
+    for (int64_t p = e.rowptr[i] + sl, p1 = e.rowptr[i + 1]; p < p1; p += kEpiSlices) {
+      const int32_t j = e.col[p];
+      if (CPLX) {
+        const double2 v = reinterpret_cast<const double2*>(e.val)[p];
+        const double2 xv = reinterpret_cast<const double2*>(e.x)[j];
+        c.z = fma(v.x, xv.x, fma(-v.y, xv.y, c.z));
+        c.w = fma(v.x, xv.y, fma(v.y, xv.x, c.w));
+      } else {
+        c.z = fma(e.val[p], e.x[j], c.z);
+      }
+    }
   }
-  for (int r = 0; r < B; ++r) {
-    const double2 v = load_partial(zp + (int64_t)r * s.npad + i);
-    sr += v.x;
-    si += v.y;
+  // the nodes of a CTA lie in one row block
+  const int B = (int)(i0 / s.bt), il = (int)(i - (int64_t)B * s.bt);
+  const P* yp = static_cast<const P*>(e.partial) + il;
+  const P* zp = static_cast<const P*>(s.zpart) + i;
+  const int q0 = s.rowptr[B], q1 = s.rowptr[B + 1];
+  for (int qc = q0; qc < q1; qc += kEpiNodes * kEpiSlices) {
+    const int cnt = min(q1 - qc, kEpiNodes * kEpiSlices);
+    __syncthreads();
+    if ((int)threadIdx.x < cnt) list[threadIdx.x] = s.rowitems[qc + threadIdx.x];
+    __syncthreads();
+    if (live) {
+#pragma unroll 4
+      for (int q = sl; q < cnt << s.lsub; q += kEpiSlices) {
+        const int64_t slot = ((int64_t)list[q >> s.lsub] << s.lsub) + (q & ((1 << s.lsub) - 1));
+        const double2 v = load_partial(yp + slot * s.bt);
+        c.x += v.x;
+        c.y += v.y;
+      }
+    }
   }
-  epilogue_finish<CPLX>(e, i, sr, si);
+  if (live) {
+#pragma unroll 4
+    for (int r = sl; r < B; r += kEpiSlices) {
+      const double2 v = load_partial(zp + (int64_t)r * s.npad);
+      c.x += v.x;
+      c.y += v.y;
+    }
+  }
+  part[sl][tn] = c;
+  __syncthreads();
+  if (sl != 0 || i >= e.m) return;
+#pragma unroll
+  for (int q = 1; q < kEpiSlices; ++q) {
+    const double4 v = part[q][tn];
+    c.x += v.x;
+    c.y += v.y;
+    c.z += v.z;
+    c.w += v.w;
+  }
+  const double sc = e.rowscale ? e.scale * e.rowscale[i] : e.scale;
+  epilogue_store<CPLX>(e, i, fma(c.x, sc, c.z), fma(c.y, sc, c.w),
+                       e.beta_zero ? make_double2(0.0, 0.0) : epilogue_y_old<CPLX>(e, i));
 }
 
 // ---------------------------------------------------------------------------
@@ -1699,16 +1779,16 @@ int pair_symm_default_ch(const inti_ctx* ctx, int pde, int kind, int dim, int pr
       size_t sm;
       if (precision == INTI_FP32C) {
         if constexpr (symm_x2<T, float>()) {
-          fn = tpt == 2 ? (const void*)&pair_symm_x2<T::kind, 2> : (const void*)&pair_symm_x2<T::kind, 4>;
+          fn = tpt == 2 ? (const void*)&pair_symm_x2<T::kind, 2, false> : (const void*)&pair_symm_x2<T::kind, 4, false>;
           sm = symm_x2_smem<T>();
         } else {
-          fn = tpt == 2 ? (const void*)&pair_symm<T::pde, T::kind, T::dim, float, kTile32, 2>
-                        : (const void*)&pair_symm<T::pde, T::kind, T::dim, float, kTile32, 4>;
+          fn = tpt == 2 ? (const void*)&pair_symm<T::pde, T::kind, T::dim, float, kTile32, 2, false>
+                        : (const void*)&pair_symm<T::pde, T::kind, T::dim, float, kTile32, 4, false>;
           sm = symm_smem<T, float>();
         }
       } else {
-        fn = tpt == 2 ? (const void*)&pair_symm<T::pde, T::kind, T::dim, double, kTile64, 2>
-                      : (const void*)&pair_symm<T::pde, T::kind, T::dim, double, kTile64, 4>;
+        fn = tpt == 2 ? (const void*)&pair_symm<T::pde, T::kind, T::dim, double, kTile64, 2, false>
+                      : (const void*)&pair_symm<T::pde, T::kind, T::dim, double, kTile64, 4, false>;
         sm = symm_smem<T, double>();
       }
       INTI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1721,6 +1801,17 @@ int pair_symm_default_ch(const inti_ctx* ctx, int pde, int kind, int dim, int pr
   const int64_t pairs = nb * (nb + 1) / 2;         // block pairs J >= I
   const int64_t want = (int64_t)ctx->num_sms * occ * 8;  // about 8 waves of items
   return (int)std::max<int64_t>(1, std::min<int64_t>(nb, (pairs + want - 1) / want));
+}
+
+int pair_symm_sub(const inti_ctx* ctx, int tpt, int ch, int nitems) {
+  // Parts of at least 32 sources (one FP32C group) until there are 16 CTAs
+  // per SM: four waves of the four resident ones, so that the last, partly
+  // filled one weighs little.  With whole blocks (78 CTAs at 3,072 nodes) a
+  // Helmholtz SL took 64 us in the pair kernel; 27 us with eight parts.
+  if (ch != 1) return 1;
+  int sub = 1;
+  while (sub < pair_symm_block(tpt) / kGroup && (int64_t)nitems * sub < (int64_t)16 * ctx->num_sms) sub *= 2;
+  return sub;
 }
 
 int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
@@ -1740,20 +1831,15 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
         bool done = false;
         if constexpr (symm_x2<T, R>()) {
           if (L.symm) {
-            pack_sources_x2<T::kind><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x,
-                                                               L.c1[0], L.c2[0], static_cast<float*>(L.packed));
+            pack_sources_x2<T::kind><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x, L.c1[0], L.c2[0], static_cast<float*>(L.packed));
             done = true;
           }
         }
         if (done) {
         } else if (L.symm && (T::kind == ADL || T::kind == HS)) {
-          pack_sym_normal<T::pde, T::dim, R><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals,
-                                                                         L.sweights, L.x,
-                                                                         static_cast<R*>(L.packed));
+          pack_sym_normal<T::pde, T::dim, R><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x, static_cast<R*>(L.packed));
         } else {
-          pack_sources<T::pde, T::kind, T::dim, R><<<gp, pb, 0, ctx->stream>>>(
-              L.n, npad, L.scoords, L.snormals, L.sweights, L.x, make_double2(L.c1[0], L.c1[1]),
-              make_double2(L.c2[0], L.c2[1]), static_cast<R*>(L.packed));
+          pack_sources<T::pde, T::kind, T::dim, R><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x, make_double2(L.c1[0], L.c1[1]), make_double2(L.c2[0], L.c2[1]), static_cast<R*>(L.packed));
         }
       }
       if constexpr (symm_kind<T>()) {
@@ -1762,6 +1848,7 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
           a.npad = npad;
           a.items = L.sym_launch ? L.sym_launch : L.sym_items;
           a.ids = L.sym_launch ? L.sym_launch_ids : nullptr;
+          a.sub = L.sym_sub;
           a.packed = L.packed;
           a.ypart = L.partial;
           a.zpart = L.zpart;
@@ -1775,18 +1862,25 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
           void (*fn)(SymArgs);
           if constexpr (symm_x2<T, R>()) {
             sm = symm_x2_smem<T>();
-            fn = L.tpt == 2 ? &pair_symm_x2<T::kind, 2> : &pair_symm_x2<T::kind, 4>;
+            if (L.sym_sub > 1)
+              fn = L.tpt == 2 ? &pair_symm_x2<T::kind, 2, true> : &pair_symm_x2<T::kind, 4, true>;
+            else
+              fn = L.tpt == 2 ? &pair_symm_x2<T::kind, 2, false> : &pair_symm_x2<T::kind, 4, false>;
           } else {
             sm = symm_smem<T, R>();
-            fn = L.tpt == 2 ? &pair_symm<T::pde, T::kind, T::dim, R, TILE, 2>
-                            : &pair_symm<T::pde, T::kind, T::dim, R, TILE, 4>;
+            if (L.sym_sub > 1)
+              fn = L.tpt == 2 ? &pair_symm<T::pde, T::kind, T::dim, R, TILE, 2, true>
+                              : &pair_symm<T::pde, T::kind, T::dim, R, TILE, 4, true>;
+            else
+              fn = L.tpt == 2 ? &pair_symm<T::pde, T::kind, T::dim, R, TILE, 2, false>
+                              : &pair_symm<T::pde, T::kind, T::dim, R, TILE, 4, false>;
           }
           INTI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
           a.zld = npad;
           a.zcol0 = 0;
           if (L.sym_npanels <= 1) {
             ProfScope pp(ctx, "pair");
-            const int grid = L.sym_launch ? L.sym_launch_items : L.sym_nitems;
+            const int grid = (L.sym_launch ? L.sym_launch_items : L.sym_nitems) * L.sym_sub;
             if (grid > 0) fn<<<(unsigned)grid, kBlock, sm, ctx->stream>>>(a);
             launches = 2;
             return;
@@ -1910,22 +2004,26 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
     return 1;
   }
   if (L.symm) {
+    const unsigned gs = (unsigned)((L.m + kEpiNodes - 1) / kEpiNodes);
+    const unsigned ts = kEpiNodes * kEpiSlices;
     SymEpi se;
     se.npad = L.n_tiles * pair_tile(L.precision);
     se.bt = pair_symm_block(L.tpt);
+    se.lsub = 0;
+    while ((1 << se.lsub) < L.sym_sub) ++se.lsub;
     se.rowptr = L.sym_rowptr;
     se.rowitems = L.sym_rowitems;
     se.zpart = L.zpart;
     if (L.precision == INTI_FP32C) {
       if (cplx)
-        pair_symm_epilogue_kernel<float4, true><<<gb, tb, 0, ctx->stream>>>(e, se);
+        pair_symm_epilogue_kernel<float4, true><<<gs, ts, 0, ctx->stream>>>(e, se);
       else
-        pair_symm_epilogue_kernel<float2, false><<<gb, tb, 0, ctx->stream>>>(e, se);
+        pair_symm_epilogue_kernel<float2, false><<<gs, ts, 0, ctx->stream>>>(e, se);
     } else {
       if (cplx)
-        pair_symm_epilogue_kernel<double2, true><<<gb, tb, 0, ctx->stream>>>(e, se);
+        pair_symm_epilogue_kernel<double2, true><<<gs, ts, 0, ctx->stream>>>(e, se);
       else
-        pair_symm_epilogue_kernel<double, false><<<gb, tb, 0, ctx->stream>>>(e, se);
+        pair_symm_epilogue_kernel<double, false><<<gs, ts, 0, ctx->stream>>>(e, se);
     }
     INTI_CUDA(cudaGetLastError());
     ctx->launches += 1;
