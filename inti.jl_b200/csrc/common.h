@@ -9,6 +9,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/inti_b200.h"
@@ -33,6 +34,23 @@ struct Error : std::runtime_error {
     if (_e != cudaSuccess)                                                           \
       throw ::inti::Error(INTI_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
   } while (0)
+
+// Launch that may overlap the end of the kernel before it in the stream (see
+// pdl_wait in device_common.cuh).
+template <class... P, class... A>
+void launch_pdl(cudaStream_t stream, dim3 grid, unsigned block, size_t smem, void (*kernel)(P...), A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  INTI_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...));
+}
 
 // Device blocks are taken from, and given back to, a per-device CUDA memory
 // pool that keeps released memory (devmem.cu): creating and destroying

@@ -144,6 +144,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// Programmatic dependent launch (launch_pdl): a kernel may start while the one
+// before it in the stream is finishing.  What it does before pdl_wait() must
+// not touch anything that one writes or reads; pdl_wait() returns when the
+// grid before has completed and its writes are visible (at once when the
+// launch had no such attribute).  pdl_trigger() lets the next one start.
+// Every kernel launched this way waits, so completion carries over a chain.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Error codes written to the context's device flag.
 constexpr int kErrWaitTimeout = 1;
 

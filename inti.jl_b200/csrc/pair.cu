@@ -111,6 +111,8 @@ __global__ void pack_sources(int64_t n, int64_t npad, const double* __restrict__
                              R* __restrict__ out) {
   using RC = Rec<PDE, KIND, DIM, R>;
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (j >= npad) return;
   R rec[RC::n];
   build_record<PDE, KIND, DIM, R>(j, n, xs, ns, w, sigma, c1, c2, rec);
@@ -377,6 +379,7 @@ __global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
   const int64_t t1 = min(a.n_tiles, t0 + a.tiles_per_split);
   const R* src = static_cast<const R*>(a.packed);
 
+  pdl_trigger();
   Target<R, DIM, RC::tnormal> tg[TPT];
   Acc<R, CPLX> acc[TPT];
 #pragma unroll
@@ -403,6 +406,7 @@ __global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
     mbar_fence_init();
   }
   __syncthreads();
+  pdl_wait();  // the packed records; the partials of the product before are consumed
   int64_t issued = t0;  // next tile to issue (meaningful in thread 0)
   if (tid == 0) {
     for (int s = 0; s < 2 && issued < t1; ++s, ++issued) {
@@ -534,6 +538,8 @@ __device__ __forceinline__ void epilogue_finish(const EpiArgs& e, int64_t i, dou
 template <class P, bool CPLX>
 __global__ void pair_epilogue_kernel(EpiArgs e) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (i >= e.m) return;
   if (e.err && *e.err) {  // the partial sums are incomplete: make the failure visible in y
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
@@ -768,6 +774,8 @@ __global__ void pack_sym_normal(int64_t n, int64_t npad, const double* __restric
                                 const double* __restrict__ sigma, R* __restrict__ out) {
   constexpr int NR = SymRec<PDE, HS, DIM, R>::n;
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (j >= npad) return;
   R rec[NR];
 #pragma unroll
@@ -1010,12 +1018,14 @@ __global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
     return (SUB ? (uint32_t)min((int64_t)TILE, ps - t * TILE) : (uint32_t)TILE) * (uint32_t)(kStageBytes / TILE);
   };
   const R* src = static_cast<const R*>(a.packed);
+  pdl_trigger();
   if (TMA_TAB && tid == 0) {  // the table's copy does not wait for the kernel before
     mbar_init(&tab_full, 1);
     mbar_fence_init();
     mbar_arrive_expect_tx(&tab_full, kExpiTable * sizeof(R2));
     bulk_copy_g2s(tab, a.expi, kExpiTable * sizeof(R2), &tab_full);
   }
+  pdl_wait();  // the packed records; the partials of the product before are consumed
   R tg[TPT][NU];
   Acc<R, CPLX> acc[TPT];
 #pragma unroll
@@ -1161,6 +1171,8 @@ __global__ void pack_sources_x2(int64_t n, int64_t npad, const double* __restric
                                 float* __restrict__ out) {
   constexpr int NR = RecX2<KIND>::n;
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (j >= npad) return;
   float v[RecX2<KIND>::vals];
 #pragma unroll
@@ -1241,6 +1253,8 @@ __global__ void __launch_bounds__(kBlock) pair_symm_x2(SymArgs a) {
     return (SUB ? (uint32_t)min((int64_t)TILE, ps - t * TILE) : (uint32_t)TILE) * (uint32_t)(kStageBytes / TILE);
   };
   const float* src = static_cast<const float*>(a.packed);
+  pdl_trigger();
+  pdl_wait();  // the packed records; the partials of the product before are consumed
   float2 tg[NP][NV];  // (target 2p, target 2p + 1), value c
   float2 g[NP];       // group sums per lane
   float hr[TPT], lr[TPT];
@@ -1435,6 +1449,8 @@ __global__ void __launch_bounds__(kEpiNodes * kEpiSlices) pair_symm_epilogue_ker
   const int tn = threadIdx.x % kEpiNodes, sl = threadIdx.x / kEpiNodes;
   const int64_t i0 = blockIdx.x * (int64_t)kEpiNodes, i = i0 + tn;
   const bool live = i < e.m;
+  pdl_trigger();
+  pdl_wait();
   double4 c = make_double4(0.0, 0.0, 0.0, 0.0);  // pair sum, correction sum
   if (live && e.rowptr) {
     for (int64_t p = e.rowptr[i] + sl, p1 = e.rowptr[i + 1]; p < p1; p += kEpiSlices) {
@@ -1831,15 +1847,19 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
         bool done = false;
         if constexpr (symm_x2<T, R>()) {
           if (L.symm) {
-            pack_sources_x2<T::kind><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x, L.c1[0], L.c2[0], static_cast<float*>(L.packed));
+            launch_pdl(ctx->stream, gp, pb, 0, &pack_sources_x2<T::kind>, L.n, npad, L.scoords, L.snormals, L.sweights,
+                       L.x, L.c1[0], L.c2[0], static_cast<float*>(L.packed));
             done = true;
           }
         }
         if (done) {
         } else if (L.symm && (T::kind == ADL || T::kind == HS)) {
-          pack_sym_normal<T::pde, T::dim, R><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x, static_cast<R*>(L.packed));
+          launch_pdl(ctx->stream, gp, pb, 0, &pack_sym_normal<T::pde, T::dim, R>, L.n, npad, L.scoords, L.snormals,
+                     L.sweights, L.x, static_cast<R*>(L.packed));
         } else {
-          pack_sources<T::pde, T::kind, T::dim, R><<<gp, pb, 0, ctx->stream>>>(L.n, npad, L.scoords, L.snormals, L.sweights, L.x, make_double2(L.c1[0], L.c1[1]), make_double2(L.c2[0], L.c2[1]), static_cast<R*>(L.packed));
+          launch_pdl(ctx->stream, gp, pb, 0, &pack_sources<T::pde, T::kind, T::dim, R>, L.n, npad, L.scoords, L.snormals,
+                     L.sweights, L.x, make_double2(L.c1[0], L.c1[1]), make_double2(L.c2[0], L.c2[1]),
+                     static_cast<R*>(L.packed));
         }
       }
       if constexpr (symm_kind<T>()) {
@@ -1881,7 +1901,7 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
           if (L.sym_npanels <= 1) {
             ProfScope pp(ctx, "pair");
             const int grid = (L.sym_launch ? L.sym_launch_items : L.sym_nitems) * L.sym_sub;
-            if (grid > 0) fn<<<(unsigned)grid, kBlock, sm, ctx->stream>>>(a);
+            if (grid > 0) launch_pdl(ctx->stream, (unsigned)grid, kBlock, sm, fn, a);
             launches = 2;
             return;
           }
@@ -1956,7 +1976,7 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
       INTI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
       dim3 grid((unsigned)((L.m + kBlock * L.tpt - 1) / (kBlock * L.tpt)), (unsigned)L.split);
       ProfScope pp(ctx, "pair");
-      fn<<<grid, kBlock, sm, ctx->stream>>>(a);
+      launch_pdl(ctx->stream, grid, kBlock, sm, fn, a);
       launches = 2;
     };
     if (L.precision == INTI_FP32C)
@@ -1996,9 +2016,9 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
     e.partial = L.sym_acc;
     e.split = 1;
     if (cplx)
-      pair_epilogue_kernel<double2, true><<<gb, tb, 0, ctx->stream>>>(e);
+      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double2, true>, e);
     else
-      pair_epilogue_kernel<double, false><<<gb, tb, 0, ctx->stream>>>(e);
+      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double, false>, e);
     INTI_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return 1;
@@ -2016,14 +2036,14 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
     se.zpart = L.zpart;
     if (L.precision == INTI_FP32C) {
       if (cplx)
-        pair_symm_epilogue_kernel<float4, true><<<gs, ts, 0, ctx->stream>>>(e, se);
+        launch_pdl(ctx->stream, gs, ts, 0, &pair_symm_epilogue_kernel<float4, true>, e, se);
       else
-        pair_symm_epilogue_kernel<float2, false><<<gs, ts, 0, ctx->stream>>>(e, se);
+        launch_pdl(ctx->stream, gs, ts, 0, &pair_symm_epilogue_kernel<float2, false>, e, se);
     } else {
       if (cplx)
-        pair_symm_epilogue_kernel<double2, true><<<gs, ts, 0, ctx->stream>>>(e, se);
+        launch_pdl(ctx->stream, gs, ts, 0, &pair_symm_epilogue_kernel<double2, true>, e, se);
       else
-        pair_symm_epilogue_kernel<double, false><<<gs, ts, 0, ctx->stream>>>(e, se);
+        launch_pdl(ctx->stream, gs, ts, 0, &pair_symm_epilogue_kernel<double, false>, e, se);
     }
     INTI_CUDA(cudaGetLastError());
     ctx->launches += 1;
@@ -2031,14 +2051,14 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
   }
   if (L.precision == INTI_FP32C) {
     if (cplx)
-      pair_epilogue_kernel<float4, true><<<gb, tb, 0, ctx->stream>>>(e);
+      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<float4, true>, e);
     else
-      pair_epilogue_kernel<float2, false><<<gb, tb, 0, ctx->stream>>>(e);
+      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<float2, false>, e);
   } else {
     if (cplx)
-      pair_epilogue_kernel<double2, true><<<gb, tb, 0, ctx->stream>>>(e);
+      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double2, true>, e);
     else
-      pair_epilogue_kernel<double, false><<<gb, tb, 0, ctx->stream>>>(e);
+      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double, false>, e);
   }
   INTI_CUDA(cudaGetLastError());
   ctx->launches += 1;
