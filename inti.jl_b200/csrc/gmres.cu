@@ -17,16 +17,18 @@
 // reductions.  The small Hessenberg least-squares problem (Givens rotations)
 // runs on the host from one device->host copy per step.  Small systems
 // (n <= 8192 unknowns by default) take a whole step after the operator application in
-// one single-CTA kernel (both CGS passes, the norm, the new basis vector and
+// one single-cluster kernel (both CGS passes, the norm, the new basis vector and
 // the Givens update on the device) and the host looks at the residuals once
 // per kArnoldiBatch steps, so a step costs two or three launches and no
 // round trip.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <complex>
+#include <cstring>
 #include <memory>
 #include <vector>
 
@@ -172,28 +174,69 @@ __device__ __forceinline__ double2 load_c(const double* v, int64_t i) {
   return C ? reinterpret_cast<const double2*>(v)[i] : make_double2(v[i], 0.0);
 }
 
+// Warp sums of eight values, reduce-scattered (as warp_sum4 of the pair
+// kernels): 9 shuffles instead of 40.  Lane l returns the sum of v[l >> 2].
+__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
+  double a[4], b[2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    a[q] = (lane & 16 ? v[q + 4] : v[q]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? v[q] : v[q + 4], 16);
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    b[q] = (lane & 8 ? a[q + 2] : a[q]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a[q] : a[q + 2], 8);
+  double k = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 2);
+  k += __shfl_xor_sync(0xffffffffu, k, 1);
+  return k;
+}
+
 // Step j of a small-system cycle, after w = sum_t coef_t A_t v_j (the shift
 // is added here, w += shift * v_j, saving a launch per step): w is orthogonalised
 // against v_0..v_j twice (CGS2; sums in a fixed order), v_{j+1} = w/|w|,
 // and thread 0 applies the earlier rotations to the new Hessenberg column,
 // forms rotation j, and records |g[j+1]|.  A stopped cycle leaves later
-// steps as no-ops.  Dynamic shared memory: 2 * (restart + 1) double2.
+// steps as no-ops.
+//
+// One cluster of up to eight CTAs, each with an equal run of the rows (one
+// row per thread at 8,192 unknowns).  The step reads the basis four times, and
+// one CTA was bound by what its SM draws from L2 (at 6,912 complex unknowns 47 us a
+// step, averaged over 20; eight CTAs: 19 us).  The one-CTA case, up to 1,024
+// unknowns, gains from warp_sum8 (a solve on 1,000 nodes 606 -> 501 us).  The CTAs' partial sums meet in
+// distributed shared memory: every CTA adds all of them in CTA order, three
+// cluster barriers per step (two passes and the norm), each with buffers of
+// its own.  Thread 0 of CTA 0 finds the rotations in shared memory.
+// Dynamic shared memory: 6 * (restart + 1) double2.
 template <bool C>
 __global__ void __launch_bounds__(kArnoldiThreads) arnoldi_small_step(int64_t n, int j, int restart, double* V,
                                                                       double* w, double2 shift, double tol_abs,
                                                                       ArnoldiState st) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 hbuf[];
   __shared__ double2 red[kArnoldiThreads / 32][8];
-  __shared__ double hn_s;
-  if (st.flags[0]) return;
+  __shared__ double norm2[1];
+  pdl_trigger();
+  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int comps = C ? 2 : 1;
-  double2* hsum = hbuf;               // [restart + 1]
-  double2* hp = hbuf + restart + 1;   // [restart + 1]
-  for (int k = tid; k <= j; k += kArnoldiThreads) hsum[k] = make_double2(0.0, 0.0);
+  const int comps = C ? 2 : 1, ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  if (st.flags[0]) return;  // the same in every CTA: written by earlier kernels only
+  const int64_t per = (n + ncta - 1) / ncta;
+  const int64_t i0 = rank * per, i1 = min(n, i0 + per);
+  double2* hsum = hbuf;                    // [restart + 1] each
+  double2* hp = hbuf + (restart + 1);
+  double2* part = hbuf + 2 * (restart + 1);  // this CTA's sums: pass 0, pass 1
+  double2* rc = hbuf + 4 * (restart + 1);    // rotations so far
+  double2* rs = hbuf + 5 * (restart + 1);
+  for (int k = tid; k <= j; k += kArnoldiThreads) {
+    hsum[k] = make_double2(0.0, 0.0);
+    if (rank == 0 && k < j) {
+      rc[k] = st.cs[k];
+      rs[k] = st.sn[k];
+    }
+  }
   if (shift.x != 0.0 || shift.y != 0.0) {  // each thread its own entries, as in the passes below
     const double* vj = V + (int64_t)comps * n * j;
-    for (int64_t i = tid; i < n; i += kArnoldiThreads) {
+    for (int64_t i = i0 + tid; i < i1; i += kArnoldiThreads) {
       if (C) {
         const double2 a = reinterpret_cast<const double2*>(w)[i];
         const double2 p = cm(shift, reinterpret_cast<const double2*>(vj)[i]);
@@ -204,67 +247,80 @@ __global__ void __launch_bounds__(kArnoldiThreads) arnoldi_small_step(int64_t n,
     }
   }
   for (int pass = 0; pass < 2; ++pass) {
+    double2* mine = part + pass * (restart + 1);
     for (int k0 = 0; k0 <= j; k0 += 8) {
-      double2 acc[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) acc[u] = make_double2(0.0, 0.0);
-      for (int64_t i = tid; i < n; i += kArnoldiThreads) {
+      double ax[8] = {}, ay[8] = {};
+      for (int64_t i = i0 + tid; i < i1; i += kArnoldiThreads) {
         const double2 wi = load_c<C>(w, i);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-          if (k0 + u <= j) acc[u] = c_add(acc[u], cjm(load_c<C>(V + (int64_t)comps * n * (k0 + u), i), wi));
+          if (k0 + u <= j) {
+            const double2 v = load_c<C>(V + (int64_t)comps * n * (k0 + u), i);
+            ax[u] = fma(v.x, wi.x, ax[u]);
+            if (C) {
+              ax[u] = fma(v.y, wi.y, ax[u]);
+              ay[u] = fma(v.x, wi.y, fma(-v.y, wi.x, ay[u]));
+            }
+          }
       }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        acc[u].x = warp_sum(acc[u].x);
-        acc[u].y = warp_sum(acc[u].y);
-      }
-      if (lane == 0)
-#pragma unroll
-        for (int u = 0; u < 8; ++u) red[warp][u] = acc[u];
+      const double sx = warp_sum8(ax, lane), sy = C ? warp_sum8(ay, lane) : 0.0;
+      if ((lane & 3) == 0) red[warp][lane >> 2] = make_double2(sx, sy);
       __syncthreads();
-      if (tid < 8 && k0 + tid <= j) {
-        double2 t = make_double2(0.0, 0.0);
-        for (int q = 0; q < kArnoldiThreads / 32; ++q) t = c_add(t, red[q][tid]);
-        hp[k0 + tid] = t;
+      if (warp < 8 && k0 + warp <= j) {
+        double2 t = red[lane][warp];
+        t.x = warp_sum(t.x);
+        if (C) t.y = warp_sum(t.y);
+        if (lane == 0) mine[k0 + warp] = t;
       }
       __syncthreads();
     }
+    cl.sync();  // every CTA's sums of this pass are in its shared memory
+    for (int k = tid; k <= j; k += kArnoldiThreads) {
+      double2 t = make_double2(0.0, 0.0);
+      for (int r = 0; r < ncta; ++r) t = c_add(t, cl.map_shared_rank(mine, r)[k]);
+      hp[k] = t;
+      hsum[k] = c_add(hsum[k], t);
+    }
+    __syncthreads();
     // w -= V hp (each thread updates the entries it reads)
-    for (int64_t i = tid; i < n; i += kArnoldiThreads) {
+    for (int64_t i = i0 + tid; i < i1; i += kArnoldiThreads) {
       double2 a = load_c<C>(w, i);
+#pragma unroll 4
       for (int k = 0; k <= j; ++k) {
-        const double2 p = cm(load_c<C>(V + (int64_t)comps * n * k, i), hp[k]);
-        a.x -= p.x;
-        a.y -= p.y;
+        const double2 v = load_c<C>(V + (int64_t)comps * n * k, i), h = hp[k];
+        a.x = fma(-v.x, h.x, a.x);
+        if (C) {
+          a.x = fma(v.y, h.y, a.x);
+          a.y = fma(-v.x, h.y, fma(-v.y, h.x, a.y));
+        }
       }
       if (C)
         reinterpret_cast<double2*>(w)[i] = a;
       else
         w[i] = a.x;
     }
-    for (int k = tid; k <= j; k += kArnoldiThreads) hsum[k] = c_add(hsum[k], hp[k]);
     __syncthreads();
   }
   double s2 = 0.0;
-  for (int64_t i = tid; i < n; i += kArnoldiThreads) {
+  for (int64_t i = i0 + tid; i < i1; i += kArnoldiThreads) {
     const double2 a = load_c<C>(w, i);
     s2 = fma(a.x, a.x, fma(a.y, a.y, s2));
   }
   s2 = warp_sum(s2);
   if (lane == 0) red[warp][0].x = s2;
   __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-    for (int q = 0; q < kArnoldiThreads / 32; ++q) t += red[q][0].x;
-    hn_s = sqrt(fmax(t, 0.0));
+  if (warp == 0) {
+    const double t = warp_sum(red[lane][0].x);
+    if (lane == 0) norm2[0] = t;
   }
-  __syncthreads();
-  const double hn = hn_s;
+  cl.sync();
+  double t2 = 0.0;
+  for (int r = 0; r < ncta; ++r) t2 += *cl.map_shared_rank(norm2, r);
+  const double hn = sqrt(fmax(t2, 0.0));
   if (hn > 0.0) {
     double* vn = V + (int64_t)comps * n * (j + 1);
     const double inv = 1.0 / hn;
-    for (int64_t i = tid; i < n; i += kArnoldiThreads) {
+    for (int64_t i = i0 + tid; i < i1; i += kArnoldiThreads) {
       if (C) {
         const double2 a = reinterpret_cast<const double2*>(w)[i];
         reinterpret_cast<double2*>(vn)[i] = make_double2(a.x * inv, a.y * inv);
@@ -273,14 +329,15 @@ __global__ void __launch_bounds__(kArnoldiThreads) arnoldi_small_step(int64_t n,
       }
     }
   }
-  if (tid == 0) {
+  cl.sync();  // the peers have read this CTA's sums
+  if (tid == 0 && rank == 0) {
     double2* col = hsum;  // column j of H, then rotated in place (row j + 1 = hn)
     col[j + 1] = make_double2(hn, 0.0);
     for (int i = 0; i < j; ++i) {
-      const double2 a = col[i], b = col[i + 1], c = st.cs[i], sg = st.sn[i];
+      const double2 a = col[i], b = col[i + 1], c = rc[i], sg = rs[i];
       col[i] = c_add(cm(c_conj(c), a), cm(c_conj(sg), b));
-      const double2 t1 = cm(sg, a), t2 = cm(c, b);
-      col[i + 1] = make_double2(t2.x - t1.x, t2.y - t1.y);
+      const double2 t1 = cm(sg, a), t2c = cm(c, b);
+      col[i + 1] = make_double2(t2c.x - t1.x, t2c.y - t1.y);
     }
     const double2 a = col[j], b = col[j + 1];
     const double den = sqrt(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
@@ -295,8 +352,7 @@ __global__ void __launch_bounds__(kArnoldiThreads) arnoldi_small_step(int64_t n,
     st.g[j] = cm(c_conj(cj), gj);
     double2* Rj = st.R + (int64_t)(restart + 1) * j;
     for (int i = 0; i <= j; ++i) Rj[i] = col[i];
-    const double2 gn = st.g[j + 1];
-    const double res = sqrt(gn.x * gn.x + gn.y * gn.y);
+    const double res = sqrt(ng.x * ng.x + ng.y * ng.y);
     st.res[j] = res;
     st.flags[1] = j + 1;
     if (res <= tol_abs || hn == 0.0) st.flags[0] = 1;
@@ -404,8 +460,23 @@ struct Solver {
     INTI_CUDA(cudaMemsetAsync(st.flags, 0, 2 * sizeof(int), ctx->stream));
     const double2 g0 = make_double2(beta, 0.0);
     INTI_CUDA(cudaMemcpyAsync(st.g, &g0, sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
-    const size_t smem = sizeof(double2) * 2 * (restart + 1);
-    std::vector<double> rh(restart);
+    const size_t smem = sizeof(double2) * 6 * (restart + 1);
+    const auto step = C ? &arnoldi_small_step<true> : &arnoldi_small_step<false>;
+    INTI_CUDA(cudaFuncSetAttribute(step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n > 4096 ? 8 : n > 2048 ? 4 : n > 1024 ? 2 : 1;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(attr[0].val.clusterDim.x);
+    cfg.blockDim = dim3(kArnoldiThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    std::vector<double> rh(restart + 1);
     int flags[2] = {0, 0};
     int j = 0;
     while (j < restart && it < maxit && !done) {
@@ -413,18 +484,14 @@ struct Solver {
       for (int b = 0; b < batch; ++b) {
         apply_unshifted(fp32, V + (size_t)comps * n * (j + b), w);
         const double2 sh = make_double2(shift.real(), shift.imag());
-        if (C)
-          arnoldi_small_step<true><<<1, kArnoldiThreads, smem, ctx->stream>>>(n, j + b, restart, V, w, sh, tol_abs,
-                                                                               st);
-        else
-          arnoldi_small_step<false><<<1, kArnoldiThreads, smem, ctx->stream>>>(n, j + b, restart, V, w, sh,
-                                                                                tol_abs, st);
+        INTI_CUDA(cudaLaunchKernelEx(&cfg, step, n, j + b, restart, V, w, sh, tol_abs, st));
         ctx->launches++;
       }
-      INTI_CUDA(cudaMemcpyAsync(rh.data() + j, st.res + j, sizeof(double) * batch, cudaMemcpyDeviceToHost,
-                                ctx->stream));
-      INTI_CUDA(cudaMemcpyAsync(flags, st.flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      // the residuals and the flags behind them, in one copy
+      INTI_CUDA(cudaMemcpyAsync(rh.data() + j, st.res + j, sizeof(double) * (restart - j) + sizeof(flags),
+                                cudaMemcpyDeviceToHost, ctx->stream));
       INTI_CUDA(cudaStreamSynchronize(ctx->stream));
+      std::memcpy(flags, rh.data() + restart, sizeof(flags));
       const int now = flags[1];  // steps done in this cycle
       for (; j < now; ++j) {
         ++it;
