@@ -38,6 +38,7 @@ struct inti_batch {
   }
   int64_t tc_ntiles = 0;
   int tc_nitems = 0;
+  int tc_rows = 256;  // targets per item: 256 or 128
   inti::FxPlan fx;  // FP64 products on the INT8 tensor path
 };
 

@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "batch.h"
@@ -316,7 +317,11 @@ __device__ __forceinline__ void tc_kernel_x2(const float2 (&x)[3], const float4 
 // (Splitting aFull/mmaDone per K quarter, so that warp groups drift apart
 // without waiting for one another, measured slower: four commits per stage
 // cost more than the skew they hide.)
-template <int KIND>
+//
+// ACC = 2 accumulators (256 targets per item), or 1 (128 targets): batches
+// whose 256-target items do not fill the SMs.  A thread then takes one row
+// with the unpaired arithmetic; every value and every sum is the same.
+template <int KIND, int ACC>
 __global__ void __launch_bounds__(TC_THREADS, 1) mrhs_tc_kernel(TcArgs a) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t fullS[TC_NS], fullB[TC_NB], aFull[2], mmaDone[TC_NB], drainBar;
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mrhs_tc_kernel(TcArgs a) {
         const uint64_t bdesc = tc_smem_desc(sbase + TC_OFF_B + nb * TC_B_BYTES);
         if (elect_one()) {
           tc_mma8_ts(tmem, tmem + tc_a_col(bb, 0), bdesc, t > 0 ? 1u : 0u);
-          tc_mma8_ts(tmem + TC_N, tmem + tc_a_col(bb, 1), bdesc, t > 0 ? 1u : 0u);
+          if (ACC == 2) tc_mma8_ts(tmem + TC_N, tmem + tc_a_col(bb, 1), bdesc, t > 0 ? 1u : 0u);
           tc_commit(&mmaDone[nb]);
         }
         __syncwarp();
@@ -428,7 +433,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mrhs_tc_kernel(TcArgs a) {
       // lane quarter warp % 4 that this warp may access
       const int ra = 32 * (warp & 3) + lane;
       const int j0 = (gw >> 2) * (TC_J / 4);
-      const int64_t blk0 = (int64_t)a.item_block[item] * TC_ROWS;
+      const int64_t blk0 = (int64_t)a.item_block[item] * (128 * ACC);
       float2 xt[3];  // (row ra, row ra + 128) coordinates
       {
         const int64_t t0i = off + min(blk0 + ra, n - 1), t1i = off + min(blk0 + ra + 128, n - 1);
@@ -450,10 +455,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mrhs_tc_kernel(TcArgs a) {
         const float* S = reinterpret_cast<const float*>(sm + TC_OFF_S + sb * TC_S_BYTES);
 #pragma unroll
         for (int jq = 0; jq < TC_J / 4; jq += 4) {
-          uint32_t v[2][8];
+          uint32_t v[ACC][8];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int j = j0 + jq + e;
+            if constexpr (ACC == 1) {
+              const float4 ra4 = *reinterpret_cast<const float4*>(S + j * TC_S_FLOATS);
+              const float4 rb4 = *reinterpret_cast<const float4*>(S + j * TC_S_FLOATS + 4);
+              const float4 rc4 = *reinterpret_cast<const float4*>(S + j * TC_S_FLOATS + 8);
+              const float xr[3] = {xt[0].x, xt[1].x, xt[2].x};
+              const float2 kv = tc_kernel<KIND>(xr, make_float4(ra4.x, ra4.z, rb4.x, rb4.z),
+                                                make_float2(rc4.x, rc4.z), kc);
+              v[0][2 * e] = tf32_bits(kv.x);
+              v[0][2 * e + 1] = tf32_bits(kv.y);
+              continue;
+            }
             const float4 sa = *reinterpret_cast<const float4*>(S + j * TC_S_FLOATS);
             const float4 sb = *reinterpret_cast<const float4*>(S + j * TC_S_FLOATS + 4);
             const float4 sc = *reinterpret_cast<const float4*>(S + j * TC_S_FLOATS + 8);
@@ -461,11 +477,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mrhs_tc_kernel(TcArgs a) {
             tc_kernel_x2<KIND>(xt, sa, sb, sc, kc, k0, k1);
             v[0][2 * e] = tf32_bits(k0.x);
             v[0][2 * e + 1] = tf32_bits(k0.y);
-            v[1][2 * e] = tf32_bits(k1.x);
-            v[1][2 * e + 1] = tf32_bits(k1.y);
+            v[ACC - 1][2 * e] = tf32_bits(k1.x);
+            v[ACC - 1][2 * e + 1] = tf32_bits(k1.y);
           }
 #pragma unroll
-          for (int h = 0; h < 2; ++h) tc_st8(lane_base + tc_a_col(gg & 1, h) + 2 * (j0 + jq), v[h]);
+          for (int h = 0; h < ACC; ++h) tc_st8(lane_base + tc_a_col(gg & 1, h) + 2 * (j0 + jq), v[h]);
         }
         tc_wait_st();
         tc_fence_before();
@@ -479,14 +495,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mrhs_tc_kernel(TcArgs a) {
       if (ok) {
         tc_fence_after();
         // generator gw: accumulator (gw>>2)&1, TMEM lane quarter warp&3, column half gw>>3
-        const int acc = (gw >> 2) & 1, half = gw >> 3;
+        // (one accumulator: column quarter gw>>2)
+        const int acc = ACC == 2 ? (gw >> 2) & 1 : 0, part = ACC == 2 ? gw >> 3 : gw >> 2;
+        constexpr int kPart = TC_R / (ACC == 2 ? 2 : 4);
         const int64_t row_loc = blk0 + acc * 128 + ra;
         const bool active = row_loc < n;
         const uint32_t lane_addr = lane_base + acc * TC_N;
         const double sc = 1.0 / (4 * kPi);
         const int c0 = cg * TC_R;
         double2* Y = reinterpret_cast<double2*>(a.y);
-        for (int m = half * (TC_R / 2); m < (half + 1) * (TC_R / 2); m += 16) {
+        for (int m = part * kPart; m < (part + 1) * kPart; m += 16) {
           float re[16], im[16];
           tc_ld16(lane_addr + m, re);
           tc_ld16(lane_addr + TC_R + m, im);
@@ -684,9 +702,25 @@ static void tc_setup(inti_batch* b) {
   std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
     return b->off[p + 1] - b->off[p] > b->off[q + 1] - b->off[q];
   });
+  // Items of 128 targets where they finish earlier: greedy schedules of both
+  // lists over the SMs; an item costs its sources, a 128-target one 0.8 of a
+  // 256-target one (unpaired generation).  Four surfaces of 1,350 .. 7,776
+  // nodes are 70 items of 256 targets, 345 us, or 140 of 128, 273 us.
+  auto makespan = [&](int rows, double cost) {
+    std::vector<double> load(ctx->num_sms, 0.0);
+    std::make_heap(load.begin(), load.end(), std::greater<double>());
+    for (int s : order)
+      for (int64_t t = 0; t * rows < b->off[s + 1] - b->off[s]; ++t) {
+        std::pop_heap(load.begin(), load.end(), std::greater<double>());
+        load.back() += cost * (double)(b->off[s + 1] - b->off[s]);
+        std::push_heap(load.begin(), load.end(), std::greater<double>());
+      }
+    return *std::max_element(load.begin(), load.end());
+  };
+  b->tc_rows = makespan(128, 0.8) < makespan(TC_ROWS, 1.0) ? 128 : TC_ROWS;
   std::vector<int32_t> isurf, iblk;
   for (int s : order)
-    for (int64_t t = 0; t * TC_ROWS < b->off[s + 1] - b->off[s]; ++t) {
+    for (int64_t t = 0; t * b->tc_rows < b->off[s + 1] - b->off[s]; ++t) {
       isurf.push_back(s);
       iblk.push_back((int32_t)t);
     }
@@ -741,8 +775,10 @@ static void tc_setup(inti_batch* b) {
       b->kind == SL ? nullptr : b->normals.as<double>(), b->tc_src.as<float>());
   ctx->launches++;
   b->tc_counter.ensure(sizeof(int));
-  for (const void* kern : {(const void*)mrhs_tc_kernel<SL>, (const void*)mrhs_tc_kernel<DL>,
-                           (const void*)mrhs_tc_kernel<CF>, (const void*)mrhs_tc_kernel<CFI>})
+  for (const void* kern :
+       {(const void*)mrhs_tc_kernel<SL, 2>, (const void*)mrhs_tc_kernel<DL, 2>, (const void*)mrhs_tc_kernel<CF, 2>,
+        (const void*)mrhs_tc_kernel<CFI, 2>, (const void*)mrhs_tc_kernel<SL, 1>, (const void*)mrhs_tc_kernel<DL, 1>,
+        (const void*)mrhs_tc_kernel<CF, 1>, (const void*)mrhs_tc_kernel<CFI, 1>})
     INTI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
 }
 
@@ -765,7 +801,7 @@ static void tc_pack(inti_batch* b, const double* x, int64_t ldx, int nrhs, int64
 
 // The tensor-core kernel over nitems work items (item_surf[i], item_block[i]).
 static void tc_run(inti_batch* b, const BatchArgs& a, const int32_t* item_surf, const int32_t* item_block,
-                   int nitems) {
+                   int nitems, int rows) {
   inti_ctx* ctx = b->ctx;
   TcArgs t;
   t.off = b->d_off.as<int64_t>();
@@ -800,14 +836,21 @@ static void tc_run(inti_batch* b, const BatchArgs& a, const int32_t* item_surf, 
     ProfScope pk(ctx, "batch_tc");
     kern<<<ctx->num_sms, TC_THREADS, TC_SMEM, ctx->stream>>>(t);
   };
-  if (b->kind == SL)
-    launch(mrhs_tc_kernel<SL>);
-  else if (b->kind == DL)
-    launch(mrhs_tc_kernel<DL>);
-  else if (b->c1[0] == 1.0 && b->c1[1] == 0.0 && b->c2[0] == 0.0)
-    launch(mrhs_tc_kernel<CFI>);
+  auto by_kind = [&](auto acc) {
+    constexpr int A = decltype(acc)::value;
+    if (b->kind == SL)
+      launch(mrhs_tc_kernel<SL, A>);
+    else if (b->kind == DL)
+      launch(mrhs_tc_kernel<DL, A>);
+    else if (b->c1[0] == 1.0 && b->c1[1] == 0.0 && b->c2[0] == 0.0)
+      launch(mrhs_tc_kernel<CFI, A>);
+    else
+      launch(mrhs_tc_kernel<CF, A>);
+  };
+  if (rows == 128)
+    by_kind(std::integral_constant<int, 1>());
   else
-    launch(mrhs_tc_kernel<CF>);
+    by_kind(std::integral_constant<int, 2>());
   ctx->launches++;
   INTI_CUDA(cudaGetLastError());
 }
@@ -815,7 +858,7 @@ static void tc_run(inti_batch* b, const BatchArgs& a, const int32_t* item_surf, 
 void mrhs_tc_launch(inti_batch* b, const BatchArgs& a) {
   tc_setup(b);
   tc_pack(b, a.x, a.ldx, a.nrhs, 0, b->tc_ntiles);
-  tc_run(b, a, b->tc_items.as<int32_t>(), b->tc_items.as<int32_t>() + b->tc_nitems, b->tc_nitems);
+  tc_run(b, a, b->tc_items.as<int32_t>(), b->tc_items.as<int32_t>() + b->tc_nitems, b->tc_nitems, b->tc_rows);
 }
 
 void batch_apply_host_tf32(inti_batch* b, const double* x, int64_t ldx, double* y, int64_t ldy, int32_t nrhs,
@@ -872,7 +915,7 @@ void batch_apply_host_tf32(inti_batch* b, const double* x, int64_t ldx, double* 
     // compute: this group's density tiles, items and correction rows
     tc_pack(b, a.x, ldx, nrhs, toff[s0], toff[s1]);
     const int i0 = b->grp_item[g], i1 = b->grp_item[g + 1];
-    tc_run(b, a, gs + i0, gb + i0, i1 - i0);
+    tc_run(b, a, gs + i0, gb + i0, i1 - i0, TC_ROWS);
     batch_correction_rows(b, a.x, ldx, a.y, ldy, nrhs, a.ar, a.ai, r0, r0 + rows);
     INTI_CUDA(cudaEventRecord(b->ev[2 * g + 1], ctx->stream));
     // out: Y rows of this group
