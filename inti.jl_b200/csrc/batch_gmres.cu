@@ -25,36 +25,63 @@
 namespace inti {
 
 using cplx = std::complex<double>;
-constexpr int kSegBlock = 256;
+constexpr int kSegBlock = 1024;
 
-// h[sys*hs + k] = sum_{i in seg(s)} conj(V_k[r][i]) W[r][i], sys = s*R + r
+// Warp sums of eight values, reduce-scattered: lane l returns the sum of
+// v[l >> 2] (9 shuffles instead of 40).
+__device__ __forceinline__ double seg_sum8(const double (&v)[8], int lane) {
+  double a[4], b[2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    a[q] = (lane & 16 ? v[q + 4] : v[q]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? v[q] : v[q + 4], 16);
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    b[q] = (lane & 8 ? a[q + 2] : a[q]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a[q] : a[q + 2], 8);
+  double k = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 2);
+  k += __shfl_xor_sync(0xffffffffu, k, 1);
+  return k;
+}
+
+// h[sys*hs + k] = sum_{i in seg(s)} conj(V_k[r][i]) W[r][i], sys = s*R + r.
+// Eight vectors per sweep over W and 1,024 threads: with 256 threads, one
+// vector at a time and a block reduction each, it waited on its reductions
+// and on too few loads in flight (42 us on average for 256 systems of
+// 1,350 .. 7,776 nodes and five vectors; the solve they belong to 28.9 ms with
+// 512 threads, 27.4 with 1,024).
 __global__ void __launch_bounds__(kSegBlock) seg_dots(const int64_t* off, int R, int kcount, const double2* V,
                                                       int64_t vstride, int64_t ld, const double2* W, double2* h,
                                                       int hs) {
-  __shared__ double2 red[kSegBlock / 32];
-  const int sys = blockIdx.x;
+  constexpr int NW = kSegBlock / 32;
+  __shared__ double2 red[NW][8];
+  const int sys = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int s = sys / R, r = sys % R;
   const int64_t i0 = off[s], i1 = off[s + 1];
-  for (int k = 0; k < kcount; ++k) {
-    const double2* Vk = V + k * vstride + (int64_t)r * ld;
-    const double2* Wr = W + (int64_t)r * ld;
-    double sr = 0.0, si = 0.0;
+  const double2* Wr = W + (int64_t)r * ld;
+  for (int k0 = 0; k0 < kcount; k0 += 8) {
+    double ax[8] = {}, ay[8] = {};
+    const double2* Vk = V + k0 * vstride + (int64_t)r * ld;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += kSegBlock) {
-      const double2 a = Vk[i], b = Wr[i];
-      sr = fma(a.x, b.x, fma(a.y, b.y, sr));
-      si = fma(a.x, b.y, fma(-a.y, b.x, si));
+      const double2 w = Wr[i];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (k0 + u < kcount) {
+          const double2 v = Vk[u * vstride + i];
+          ax[u] = fma(v.x, w.x, fma(v.y, w.y, ax[u]));
+          ay[u] = fma(v.x, w.y, fma(-v.y, w.x, ay[u]));
+        }
     }
-    sr = warp_sum(sr);
-    si = warp_sum(si);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = make_double2(sr, si);
+    const double sx = seg_sum8(ax, lane), sy = seg_sum8(ay, lane);
+    if ((lane & 3) == 0) red[warp][lane >> 2] = make_double2(sx, sy);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double ar = 0.0, ai = 0.0;
-      for (int q = 0; q < kSegBlock / 32; ++q) {
-        ar += red[q].x;
-        ai += red[q].y;
+    if (threadIdx.x < 8 && k0 + (int)threadIdx.x < kcount) {
+      double2 t = red[0][threadIdx.x];
+#pragma unroll
+      for (int q = 1; q < NW; ++q) {
+        t.x += red[q][threadIdx.x].x;
+        t.y += red[q][threadIdx.x].y;
       }
-      h[(int64_t)sys * hs + k] = make_double2(ar, ai);
+      h[(int64_t)sys * hs + k0 + threadIdx.x] = t;
     }
     __syncthreads();
   }
@@ -68,6 +95,7 @@ __global__ void seg_axpy(int64_t n, const int32_t* node_surf, int R, int kcount,
   if (i >= n) return;
   const int sys = node_surf[i] * R + r;
   double2 acc = W[(int64_t)r * ld + i];
+#pragma unroll 4
   for (int k = 0; k < kcount; ++k) {
     const double2 v = V[k * vstride + (int64_t)r * ld + i];
     const double2 c = h[(int64_t)sys * hs + k];
@@ -102,7 +130,7 @@ struct BatchSolver {
   int64_t n, ld;
   int S, nsys;
   cplx shift;
-  DevBuf node_surf, hbuf, abuf, tmp, Vb, Wb, h1b, h2b;  // Krylov storage reused across solves
+  DevBuf node_surf, hbuf, abuf, tmp, Vb, Wb, h1b;  // Krylov storage reused across solves
   int fp64_applies = 0, lowp_applies = 0;
 
   unsigned gx() const { return (unsigned)((n + 255) / 256); }
@@ -161,8 +189,7 @@ struct BatchSolver {
     double2* V = Vb.as<double2>();
     double2* W = Wb.as<double2>();
     const int hs = restart + 2;
-    h1b.ensure(sizeof(double2) * nsys * hs);
-    h2b.ensure(sizeof(double2) * nsys * hs);
+    h1b.ensure(sizeof(double2) * nsys * hs * 2);
     int it = 0;
     bool zero = x_zero;
     std::vector<char> done(nsys, 0);
@@ -191,18 +218,21 @@ struct BatchSolver {
       for (int q = 0; q < nsys; ++q) g[q][0] = beta[q];
       int j = 0;
       bool fin = false;
-      std::vector<double2> hh1((size_t)nsys * hs), hh2((size_t)nsys * hs);
+      std::vector<double2> hh1((size_t)nsys * hs * 2);
       for (; j < restart && it < maxit; ++j) {
         apply(lowp, V + j * vs, W);
-        dots(V, vs, j + 1, W, h1b.as<double2>(), hs);
-        axpy(V, vs, j + 1, h1b.as<double2>(), hs, -1.0, W);
-        dots(V, vs, j + 1, W, h2b.as<double2>(), hs);
-        axpy(V, vs, j + 1, h2b.as<double2>(), hs, -1.0, W);
+        // both passes' coefficients, j + 2 per system, side by side: one copy of what is there
+        const int hj = j + 2;
+        double2 *h1 = h1b.as<double2>(), *h2 = h1 + (size_t)nsys * hj;
+        dots(V, vs, j + 1, W, h1, hj);
+        axpy(V, vs, j + 1, h1, hj, -1.0, W);
+        dots(V, vs, j + 1, W, h2, hj);
+        axpy(V, vs, j + 1, h2, hj, -1.0, W);
         // ||W|| into column j+1 of h2
-        dots(W, 0, 1, W, h2b.as<double2>() + (j + 1), hs);
-        INTI_CUDA(cudaMemcpyAsync(hh1.data(), h1b.p, sizeof(double2) * nsys * hs, cudaMemcpyDeviceToHost, ctx->stream));
-        INTI_CUDA(cudaMemcpyAsync(hh2.data(), h2b.p, sizeof(double2) * nsys * hs, cudaMemcpyDeviceToHost, ctx->stream));
+        dots(W, 0, 1, W, h2 + (j + 1), hj);
+        INTI_CUDA(cudaMemcpyAsync(hh1.data(), h1, sizeof(double2) * 2 * nsys * hj, cudaMemcpyDeviceToHost, ctx->stream));
         INTI_CUDA(cudaStreamSynchronize(ctx->stream));
+        const double2* hh2 = hh1.data() + (size_t)nsys * hj;
         ++it;
         bool all_done = true;
         std::vector<cplx> inv_hn(nsys);
@@ -210,8 +240,8 @@ struct BatchSolver {
           auto& Hq = H[q];
           for (int i = 0; i <= j; ++i)
             Hq[(size_t)i * restart + j] =
-                cplx(hh1[(size_t)q * hs + i].x + hh2[(size_t)q * hs + i].x, hh1[(size_t)q * hs + i].y + hh2[(size_t)q * hs + i].y);
-          const double hn = std::sqrt(std::max(hh2[(size_t)q * hs + j + 1].x, 0.0));
+                cplx(hh1[(size_t)q * hj + i].x + hh2[(size_t)q * hj + i].x, hh1[(size_t)q * hj + i].y + hh2[(size_t)q * hj + i].y);
+          const double hn = std::sqrt(std::max(hh2[(size_t)q * hj + j + 1].x, 0.0));
           Hq[(size_t)(j + 1) * restart + j] = hn;
           for (int i = 0; i < j; ++i) {
             const cplx a = Hq[(size_t)i * restart + j], c = Hq[(size_t)(i + 1) * restart + j];
@@ -254,7 +284,6 @@ struct BatchSolver {
         zero = false;
       }
       if (j > 0) {
-        h1b.ensure(sizeof(double2) * nsys * hs);
         INTI_CUDA(cudaMemcpyAsync(h1b.p, Y.data(), sizeof(double2) * nsys * hs, cudaMemcpyHostToDevice, ctx->stream));
         axpy(V, vs, j, h1b.as<double2>(), hs, +1.0, x);
       }
