@@ -50,10 +50,13 @@
 // hold 127 stages (8 * 255 * 128 * 8,128 < 2^31); then, or at the end of the
 // item, the generators read the diagonals and add them up in FP64.
 //
+// More than 64 real columns go to pairs of CTAs that share the evaluation.
+//
 // Measured (B200, against the FP64 MMA kernels, device time): 64 complex
-// columns of a Helmholtz DL at 13,872 nodes 5.63 -> 2.47 ms; eight surfaces of
-// 2,646 .. 21,600 nodes, combined field, 64 columns 26.9 -> 15.6 ms; the
-// correction of a 43,200-node surface (18 complex columns) 33.6 -> 16.0 ms.
+// columns of a Helmholtz DL at 13,872 nodes 5.63 -> 1.91 ms (2.48 without
+// pairs); eight surfaces of 2,646 .. 21,600 nodes, combined field, 64 columns
+// 26.9 -> 11.4 ms (15.7); the correction of a 43,200-node surface (18 complex
+// columns) 33.6 -> 16.0 ms.
 //
 // e^{ikd} comes from a 128-entry table in eight copies, one per lane of a
 // quarter-warp, so the gathers never conflict (a shared 1024-entry table
@@ -310,6 +313,50 @@ __device__ __forceinline__ void fx_ld4(uint32_t taddr, int32_t (&v)[4]) {
 }
 __device__ __forceinline__ void fx_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// --- pairs of CTAs ---------------------------------------------------------
+__device__ __forceinline__ uint32_t fx_peer(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void fx_st_peer(uint32_t a, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// Bulk copy from this CTA's shared memory to the peer's, completing on a
+// barrier of the peer (mapped addresses; 16-byte aligned, bytes a multiple of 16).
+__device__ __forceinline__ void fx_copy_peer(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "r"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void fx_commit_both(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void fx_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// mbar_wait_bounded for a barrier that the peer arrives at, too.
+template <int CL>
+__device__ __forceinline__ bool fx_wait(uint64_t* bar, uint32_t parity) {
+  if (CL == 1) return mbar_wait_bounded(bar, parity);
+  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
 struct FxArgs {
   const FxRows* rows;
   const FxItem* items;
@@ -319,9 +366,11 @@ struct FxArgs {
   const double* tnormals;
   const double* rowscale;   // per target
   const double* records;    // source records, J per stage
-  const unsigned char* bdig;  // digit blocks, nc * 512 bytes per stage
+  const unsigned char* bdig;  // digit blocks, nc * 512 bytes per stage, one plane per CTA of a pair
+  int nstages;                // stages of a plane
   const double2* tab;       // FX_TAB phase table
-  double* partial;          // [slot][column][128]
+  double* partial;          // [CTA of the pair][slot][column][128]
+  int nslots;
   FxConst c;
   int* counter;
   const int* flag;
@@ -364,24 +413,36 @@ __device__ __forceinline__ double fx_sum(const int32_t (&d)[FX_D][4], int e) {
   return fma((double)hi, 4294967296.0, (double)lo);
 }
 
-template <int PDE, int KIND>
+// CL = 2: a cluster of two CTAs works on the same items, each for its own
+// columns (up to 64 each).  Each evaluates half of a stage's pairs (two of the
+// four chunks) and the copy warp sends the digits to the other's A buffer (a
+// 4 KB bulk copy per digit), so that a kernel value is made once for 128
+// columns.  The MMAs of both must be done before either buffer is written
+// again: mmaDone counts two commits.  (Stores of the generators straight into
+// the peer's shared memory were twice as slow as evaluating everything twice.)
+template <int PDE, int KIND, int CL>
 __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
   using SH = FxShape<PDE, KIND>;
   extern __shared__ __align__(1024) unsigned char sm[];
-  __shared__ __align__(8) uint64_t fullS[FX_NS], fullB[2], aFull[2], mmaDone[FX_ND], drainBar;
+  __shared__ __align__(8) uint64_t fullS[FX_NS], fullB[2], aFull[2], aPeer[2], mmaDone[FX_ND], drainBar;
   __shared__ uint32_t tmem_base_sh;
-  __shared__ int item_sh;
+  __shared__ int item_sh, fail_sh;
   if (*a.flag) return;  // densities or kernel values out of range: the FP64 kernels run
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nc = a.nc;
+  const uint32_t rank = CL == 2 ? blockIdx.x & 1 : 0;  // clusters are consecutive blocks
+  const unsigned char* bdig = a.bdig + (size_t)rank * a.nstages * nc * (FX_D * FX_K);
+  double* partial = a.partial + (size_t)rank * a.nslots * nc * FX_M;
   const uint32_t bstage = (uint32_t)nc * (FX_D * FX_K), blbo = (uint32_t)nc * (FX_D * 16);
   if (tid == 0) {
     for (int q = 0; q < FX_NS; ++q) mbar_init(&fullS[q], 1);
-    for (int q = 0; q < FX_ND; ++q) mbar_init(&mmaDone[q], 1);
+    for (int q = 0; q < FX_ND; ++q) mbar_init(&mmaDone[q], CL);
     for (int q = 0; q < 2; ++q) {
       mbar_init(&fullB[q], 1);
       mbar_init(&aFull[q], FX_GEN);
+      mbar_init(&aPeer[q], 1);
     }
+    fail_sh = 0;
     mbar_init(&drainBar, 1);
     mbar_fence_init();
   }
@@ -397,16 +458,25 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
   fx_fence_before();
   __syncthreads();
   fx_fence_after();
+  if (CL == 2) fx_cluster_sync();  // the peer's barriers are there
   const uint32_t tmem = tmem_base_sh, sbase = smem_u32(sm);
 
   uint32_t g = 0;           // stages done by this CTA (same in every thread)
   uint32_t nS = 0, nB = 0;  // copy warp: copies issued
   uint32_t nC = 0;          // MMA warp: groups committed
+  uint32_t nA = 0;          // copy warp: stages sent to the peer (and awaited from it)
   bool ok = true;
 
   for (;;) {
-    if (tid == 0) item_sh = atomicAdd(a.counter, 1);
-    __syncthreads();
+    if (tid == 0 && rank == 0) {
+      const int next = atomicAdd(a.counter, 1);
+      item_sh = next;
+      if (CL == 2) fx_st_peer(fx_peer(smem_u32(&item_sh), 1), (uint32_t)next);
+    }
+    if (CL == 2)
+      fx_cluster_sync();
+    else
+      __syncthreads();
     const int it = item_sh;
     if (it >= a.nitems) break;
     const FxItem item = a.items[it];
@@ -417,7 +487,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
       if (warp == 0) {
         for (uint32_t t = 0; t < T; ++t) {
           const uint32_t gg = g + t, bb = gg & 1;
-          ok = mbar_wait_bounded(&aFull[bb], (gg >> 1) & 1) && mbar_wait_bounded(&fullB[bb], (gg >> 1) & 1);
+          ok = mbar_wait_bounded(&aFull[bb], (gg >> 1) & 1) && mbar_wait_bounded(&fullB[bb], (gg >> 1) & 1) &&
+               (CL == 1 || fx_wait<CL>(&aPeer[bb], (gg >> 1) & 1));
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
@@ -436,7 +507,10 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
               case 56: fx_issue<56>(tmem, ad, bd, acc); break;
               default: fx_issue<64>(tmem, ad, bd, acc); break;
             }
-            fx_commit(&mmaDone[gg % FX_ND]);
+            if (CL == 2)
+              fx_commit_both(&mmaDone[gg % FX_ND]);
+            else
+              fx_commit(&mmaDone[gg % FX_ND]);
           }
           __syncwarp();
           ++nC;
@@ -456,7 +530,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
           const uint32_t b = (g + t) & 1;
           if (fx_elect()) {
             mbar_arrive_expect_tx(&fullB[b], bstage);
-            bulk_copy_g2s(sm + SH::OFF_B + b * FX_B_BYTES, a.bdig + (size_t)(st0 + t) * bstage, bstage, &fullB[b]);
+            bulk_copy_g2s(sm + SH::OFF_B + b * FX_B_BYTES, bdig + (size_t)(st0 + t) * bstage, bstage, &fullB[b]);
           }
           __syncwarp();
           ++nB;
@@ -464,11 +538,30 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
         // the buffers of the run before are free: its MMAs were waited for
         for (uint32_t t = 0; t < FX_NS - 1 && t < T; ++t) copyS(t);
         copyB(0);
-        for (uint32_t t = 0; t + 1 < T; ++t) {
+        for (uint32_t t = 0; t + 1 < T || (CL == 2 && t < T); ++t) {
+          if (CL == 2) {  // this CTA's chunks of the stage to the peer
+            const uint32_t bb = (g + t) & 1;
+            ok = mbar_wait_bounded(&aFull[bb], ((g + t) >> 1) & 1);
+            if (!__all_sync(0xffffffffu, ok)) {
+              ok = false;
+              break;
+            }
+            if (fx_elect()) {
+              constexpr uint32_t kHalf = FX_A_DIGIT / 2;
+              mbar_arrive_expect_tx(&aPeer[bb], FX_D * kHalf);
+              const uint32_t src = sbase + bb * FX_A_BYTES + rank * kHalf;
+              const uint32_t dst = fx_peer(src, rank ^ 1), bar = fx_peer(smem_u32(&aPeer[bb]), rank ^ 1);
+#pragma unroll
+              for (int p = 0; p < FX_D; ++p) fx_copy_peer(dst + p * FX_A_DIGIT, src + p * FX_A_DIGIT, kHalf, bar);
+            }
+            __syncwarp();
+            ++nA;
+            if (t + 1 >= T) break;
+          }
           // MMA group gg-1 read the B buffer of stage gg+1 and, through its A
           // tile, the source records of stage gg-1
           const uint32_t gg = g + t;
-          if (t > 0) ok = mbar_wait_bounded(&mmaDone[(gg - 1) % FX_ND], ((gg - 1) / FX_ND) & 1);
+          if (t > 0) ok = fx_wait<CL>(&mmaDone[(gg - 1) % FX_ND], ((gg - 1) / FX_ND) & 1);
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
@@ -493,22 +586,26 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
           const uint32_t gg = g + t, sb = gg % FX_NS;
           bool w = mbar_wait_bounded(&fullS[sb], (gg / FX_NS) & 1);
           // A buffer gg & 1 was last read by MMA group gg-2
-          if (w && t >= 2) w = mbar_wait_bounded(&mmaDone[(gg - 2) % FX_ND], ((gg - 2) / FX_ND) & 1);
+          if (w && t >= 2) w = fx_wait<CL>(&mmaDone[(gg - 2) % FX_ND], ((gg - 2) / FX_ND) & 1);
           if (!__all_sync(0xffffffffu, w)) {
             ok = false;
             break;
           }
+          // a pair: chunks 2 rank, 2 rank + 1, half of a chunk's groups per thread
+          const int chunk = CL == 2 ? (int)rank * 2 + (quarter >> 1) : quarter;
           const double* S = reinterpret_cast<const double*>(sm + SH::OFF_S + sb * SH::S_BYTES) +
-                            quarter * SH::JT * FX_REC;
-          unsigned char* A = sm + (gg & 1) * FX_A_BYTES + quarter * (FX_M * 16) + r * 16;
+                            chunk * SH::JT * FX_REC;
+          unsigned char* A = sm + (gg & 1) * FX_A_BYTES + chunk * (FX_M * 16) + r * 16;
           // Groups of four sources, NA words each.  The octets of a warp take
           // them in rotated order, so that their stores of NA words at a
           // stride of 16 bytes fall on distinct banks; storing each group at
           // once keeps the registers for evaluations in flight.
-          constexpr int G = SH::JT / 4;
+          constexpr int G = SH::JT / 4, GQ = G / CL;  // of a chunk; of this thread
+          static_assert(GQ >= 1, "a group per thread");
+          const int g0 = CL == 2 ? (quarter & 1) * GQ : 0;
 #pragma unroll
-          for (int q = 0; q < G; ++q) {
-            const int grp = (q + (lane >> 3)) & (G - 1);
+          for (int q = 0; q < GQ; ++q) {
+            const int grp = (q + g0 + (lane >> 3)) & (G - 1);
             const double* Sg = S + grp * (4 * FX_REC);
             uint2 dg[SH::NA][4];
             {
@@ -540,12 +637,12 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
         }
         if (ok) {
           const uint32_t gl = g + T - 1;
-          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&mmaDone[gl % FX_ND], (gl / FX_ND) & 1));
+          ok = __all_sync(0xffffffffu, fx_wait<CL>(&mmaDone[gl % FX_ND], (gl / FX_ND) & 1));
         }
         if (ok) {
           fx_fence_after();
           const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-          double* out = a.partial + (size_t)item.slot * nc * FX_M + r;
+          double* out = partial + (size_t)item.slot * nc * FX_M + r;
           for (int c = 4 * quarter; c < nc; c += FX_GEN) {
             int32_t d[FX_D][4];
 #pragma unroll
@@ -563,8 +660,17 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
       }
       g += T;
       fx_fence_before();
-      // accumulators read (or the run abandoned) before the next run's MMAs
-      if (__syncthreads_or(!ok)) goto fail;
+      // accumulators read (or the run abandoned, by both CTAs) before the next run's MMAs
+      if (CL == 2) {
+        if (!ok) {
+          fail_sh = 1;
+          fx_st_peer(fx_peer(smem_u32(&fail_sh), rank ^ 1), 1u);
+        }
+        fx_cluster_sync();
+        if (*(volatile int*)&fail_sh) goto fail;
+      } else if (__syncthreads_or(!ok)) {
+        goto fail;
+      }
       fx_fence_after();
     }
   }
@@ -576,6 +682,7 @@ fail:
   if (warp == 1 && lane == 0) {
     for (uint32_t q = nS > FX_NS ? nS - FX_NS : 0; q < nS; ++q) mbar_wait_bounded(&fullS[q % FX_NS], (q / FX_NS) & 1);
     for (uint32_t q = nB > 2 ? nB - 2 : 0; q < nB; ++q) mbar_wait_bounded(&fullB[q & 1], (q >> 1) & 1);
+    for (uint32_t q = nA > 2 ? nA - 2 : 0; q < nA; ++q) mbar_wait_bounded(&aPeer[q & 1], (q >> 1) & 1);
   }
   if (warp == 0) {
     if (nC > 0 && fx_elect()) {
@@ -588,6 +695,7 @@ fail:
 done:
   fx_fence_before();
   __syncthreads();
+  if (CL == 2) fx_cluster_sync();  // neither leaves while the other may still reach its shared memory
   if (warp == 0) {
     fx_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -841,15 +949,19 @@ __global__ void fx_check(int count, const unsigned long long* __restrict__ colma
 }
 
 // Digit blocks: stage s, digit q of column n at [chunk][q * nc + n][16 bytes].
-// One thread per (chunk of a stage, column c of the pass).  A chunk holds
+// One thread per (chunk of a stage, column c of a plane).  A chunk holds
 // groups of four sources, each value 0, then value 1; complex columns
 // (2c, 2c + 1) have values (Re x, -Im x) and (Im x, Re x).
 template <bool CPLX>
 __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
-                        const double* __restrict__ x, int64_t ldx, int c0, int ncol, int nall, int nc,
+                        const double* __restrict__ x, int64_t ldx, int c0, int ncol, int half, int nall, int nc,
                         const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
                         unsigned char* __restrict__ out) {
   constexpr int JT = CPLX ? 8 : 16;  // sources of a chunk
+  // plane blockIdx.y: columns c0 + y * half and on
+  c0 += blockIdx.y * half;
+  ncol = min(half, ncol - (int)blockIdx.y * half);
+  out += (size_t)blockIdx.y * nstages * nc * (FX_D * FX_K);
   const int per = CPLX ? nc / 2 : nc;
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int c = (int)(id % per), chunk = (int)(id / per % 4);
@@ -1015,7 +1127,7 @@ struct FxOut {
   const double* x;
   double* y;
   int64_t ldx, ldy;
-  int c0, ncol, nall, nc;
+  int c0, ncol, nall, nc, half, nslots;  // half: columns per plane
   double scale, ar, ai, br, bi;
   bool beta_zero;
 };
@@ -1030,12 +1142,14 @@ __global__ void __launch_bounds__(FX_M) fx_finish(FxOut o) {
   const double pb = fx_scale(__longlong_as_double((long long)o.colmax[(int64_t)rb.surf * o.nall + cg]));
   // sums are in units of 256^7 / (pa pb)
   const double u = fx_inverse(o.rowscale[row]) * fx_inverse(pb) * (o.scale * kFxUnit);
+  const double* partial = o.partial + (size_t)(c / o.half) * o.nslots * o.nc * FX_M;
+  const int cp = c % o.half;
   double sr, si = 0.0;
   if (CPLX) {
-    sr = u * fx_total(rb, o.partial, o.nc, 2 * c, r);
-    si = u * fx_total(rb, o.partial, o.nc, 2 * c + 1, r);
+    sr = u * fx_total(rb, partial, o.nc, 2 * cp, r);
+    si = u * fx_total(rb, partial, o.nc, 2 * cp + 1, r);
   } else {
-    sr = u * fx_total(rb, o.partial, o.nc, c, r);
+    sr = u * fx_total(rb, partial, o.nc, cp, r);
   }
   if (o.rowptr) {
     for (int64_t p = o.rowptr[row]; p < o.rowptr[row + 1]; ++p) {
@@ -1133,6 +1247,20 @@ bool fx_pays(int pde, int kind, double pairs) {
 
 // Columns of one pass: a multiple of eight, at least 16, at most 64.
 static int fx_width(int real_columns) { return std::min(FX_NMAX, std::max(16, (real_columns + 7) / 8 * 8)); }
+// The next pass over `left` columns: up to 64 real ones in one plane, up to
+// 128 in two equal planes, one per CTA of a pair.
+struct FxPass {
+  int cols, planes, half, nc;  // columns, planes, columns per plane, real columns of a plane (padded)
+};
+static FxPass fx_pass(int left, int comps) {
+  const int one = FX_NMAX / comps;
+  FxPass p;
+  p.cols = std::min(left, 2 * one);
+  p.planes = p.cols > one ? 2 : 1;
+  p.half = (p.cols + p.planes - 1) / p.planes;
+  p.nc = fx_width(p.half * comps);
+  return p;
+}
 // work: [flag, counter per pass (up to 63) | column bounds]
 constexpr int FX_COUNTERS = 64;
 static size_t fx_work_bytes(int nsurf, int ncols) {
@@ -1201,8 +1329,11 @@ static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
     fx_plan_rows<P, K><<<(unsigned)plan.nrows * (FX_M / kPlanRows / 8), 256, 0, ctx->stream>>>(
         plan.nrows, plan.rows, p.tcoords, p.tnormals, plan.stages, plan.tiles.as<double4>(),
         plan.records.as<double>(), fx_const(p), plan.rowscale.as<double>(), plan.meta.as<unsigned long long>());
-    INTI_CUDA(cudaFuncSetAttribute(fx_contract_kernel<P, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    INTI_CUDA(cudaFuncSetAttribute(fx_contract_kernel<P, K, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    FxShape<P, K>::SMEM));
+    if constexpr (!FxShape<P, K>::theta)
+      INTI_CUDA(cudaFuncSetAttribute(fx_contract_kernel<P, K, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     FxShape<P, K>::SMEM));
   });
   ctx->launches += 2;
   INTI_CUDA(cudaGetLastError());
@@ -1217,9 +1348,9 @@ static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
 }
 
 bool fx_prepare(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, int ncols) {
-  const int nc = fx_width(ncols * (p.pde == HELMHOLTZ ? 2 : 1));
-  auto digits = [&] { return (size_t)plan.nstages * nc * FX_D * FX_K; };
-  auto partial = [&] { return sizeof(double) * (size_t)plan.nslots * nc * FX_M; };
+  const FxPass w = fx_pass(ncols, p.pde == HELMHOLTZ ? 2 : 1);  // the widest pass
+  auto digits = [&] { return (size_t)plan.nstages * w.planes * w.nc * FX_D * FX_K; };
+  auto partial = [&] { return sizeof(double) * (size_t)plan.nslots * w.planes * w.nc * FX_M; };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   INTI_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
   if (cap != cudaStreamCaptureStatusNone) return false;
@@ -1239,7 +1370,7 @@ static unsigned long long* fx_colmax_ptr(inti_ctx* ctx) {
   return reinterpret_cast<unsigned long long*>(ctx->fx.work.as<int>() + FX_COUNTERS);
 }
 
-static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc, int* counter) {
+static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc, int planes, int* counter) {
   FxArgs a;
   a.rows = plan.rows;
   a.items = plan.items;
@@ -1250,6 +1381,8 @@ static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc
   a.rowscale = plan.rowscale.as<double>();
   a.records = plan.records.as<double>();
   a.bdig = ctx->fx.bdig.as<unsigned char>();
+  a.nstages = plan.nstages;
+  a.nslots = plan.nslots;
   a.tab = ctx->fx.tab.as<double2>();
   a.partial = ctx->fx.partial.as<double>();
   a.c = fx_const(p);
@@ -1259,7 +1392,23 @@ static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc
   ctx->flag_armed = true;
   fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
     constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
-    fx_contract_kernel<P, K><<<std::min(ctx->num_sms, plan.nitems), FX_THREADS, FxShape<P, K>::SMEM, ctx->stream>>>(a);
+    if (planes == 1) {
+      fx_contract_kernel<P, K, 1>
+          <<<std::min(ctx->num_sms, plan.nitems), FX_THREADS, FxShape<P, K>::SMEM, ctx->stream>>>(a);
+    } else if constexpr (!FxShape<P, K>::theta) {
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(2 * std::min(ctx->num_sms / 2, plan.nitems)));
+      cfg.blockDim = dim3(FX_THREADS);
+      cfg.dynamicSmemBytes = FxShape<P, K>::SMEM;
+      cfg.stream = ctx->stream;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      INTI_CUDA(cudaLaunchKernelEx(&cfg, fx_contract_kernel<P, K, 2>, a));
+    }
   });
   ctx->launches++;
   INTI_CUDA(cudaGetLastError());
@@ -1269,7 +1418,6 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
               int64_t ldx, double* y, int64_t ldy, int nrhs, const double* alpha, const double* beta) {
   const bool cplx = p.pde == HELMHOLTZ;
   const int comps = cplx ? 2 : 1;
-  const int width = FX_NMAX / comps;  // columns per pass
   INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(plan.nsurf, nrhs), ctx->stream));
   int* flag = ctx->fx.work.as<int>();
   unsigned long long* colmax = fx_colmax_ptr(ctx);
@@ -1282,15 +1430,17 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
     fx_check<<<1, 256, 0, ctx->stream>>>(plan.nsurf * nrhs, colmax, meta, flag);
     ctx->launches += 2;
     int pass = 0;
-    for (int c0 = 0; c0 < nrhs; c0 += width, ++pass) {
-      const int ncol = std::min(width, nrhs - c0), nc = fx_width(ncol * comps);
-      const int64_t threads = (int64_t)plan.nstages * 4 * (nc / comps);
-      fx_pack<C><<<(unsigned)((threads + 127) / 128), 128, 0, ctx->stream>>>(
-          plan.nstages, st, p.weights, x, ldx, c0, ncol, nrhs, nc, colmax, flag, ctx->fx.bdig.as<unsigned char>());
+    FxPass w;
+    for (int c0 = 0; c0 < nrhs; c0 += w.cols, ++pass) {
+      w = fx_pass(nrhs - c0, comps);
+      const int64_t threads = (int64_t)plan.nstages * 4 * (w.nc / comps);
+      fx_pack<C><<<dim3((unsigned)((threads + 127) / 128), w.planes), 128, 0, ctx->stream>>>(
+          plan.nstages, st, p.weights, x, ldx, c0, w.cols, w.half, nrhs, w.nc, colmax, flag,
+          ctx->fx.bdig.as<unsigned char>());
       ctx->launches++;
       const int slot = 1 + pass % (FX_COUNTERS - 1);
       if (pass >= FX_COUNTERS - 1) INTI_CUDA(cudaMemsetAsync(flag + slot, 0, sizeof(int), ctx->stream));
-      fx_run(ctx, p, plan, nc, flag + slot);
+      fx_run(ctx, p, plan, w.nc, w.planes, flag + slot);
       FxOut o;
       o.rows = plan.rows;
       o.partial = ctx->fx.partial.as<double>();
@@ -1305,16 +1455,18 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
       o.ldx = ldx;
       o.ldy = ldy;
       o.c0 = c0;
-      o.ncol = ncol;
+      o.ncol = w.cols;
       o.nall = nrhs;
-      o.nc = nc;
+      o.nc = w.nc;
+      o.half = w.half;
+      o.nslots = plan.nslots;
       o.scale = 1.0 / (4 * kPi);
       o.ar = alpha ? alpha[0] : 1.0;
       o.ai = alpha ? alpha[1] : 0.0;
       o.br = beta ? beta[0] : 0.0;
       o.bi = beta ? beta[1] : 0.0;
       o.beta_zero = o.br == 0.0 && o.bi == 0.0;
-      fx_finish<C><<<dim3(plan.nrows, ncol), FX_M, 0, ctx->stream>>>(o);
+      fx_finish<C><<<dim3(plan.nrows, w.cols), FX_M, 0, ctx->stream>>>(o);
       ctx->launches++;
     }
   };
@@ -1341,7 +1493,7 @@ void fx_theta(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const doubl
     fx_theta_pack<C><<<(unsigned)((threads + 127) / 128), 128, 0, ctx->stream>>>(
         plan.nstages, plan.stages, p.weights, g0, g1, ns, nc, colmax, flag,
         ctx->fx.bdig.as<unsigned char>());
-    fx_run(ctx, p, plan, nc, flag + 1);
+    fx_run(ctx, p, plan, nc, 1, flag + 1);
     fx_theta_finish<C><<<dim3(plan.nrows, ns), FX_M, 0, ctx->stream>>>(
         plan.rows, ctx->fx.partial.as<double>(), plan.rowscale.as<double>(), colmax, ns, nc, flag, out);
   };
