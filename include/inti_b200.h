@@ -220,9 +220,8 @@ int inti_ctx_set_partial_budget(inti_ctx* ctx, double bytes);
 int inti_op_panels(const inti_op* op);
 /* Small FP64 operators (at most 2^20 target-source pairs and 65,536 sources,
  * e.g. the 1,000-node kite) apply in a single-launch form: one kernel per product builds the
- * source records, forms the pair sums (a cluster of up to 8 CTAs per 32
- * targets, the CTAs and their warps splitting the sources, sums in a fixed
- * order), adds the correction rows and applies alpha/beta.  Transposed
+ * source records, forms the pair sums (1 to 16 warps per target, their lanes
+ * splitting the sources, sums in a fixed order), adds the correction rows and applies alpha/beta.  Transposed
  * products of small square operators run the same kernel with the transposed
  * kernel and the transposed correction; item-sharded applies keep the tiled
  * kernels.  inti_ctx_set_single_launch(ctx,

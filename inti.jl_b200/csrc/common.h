@@ -334,7 +334,7 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
                   double* y, const double* alpha, const double* beta, const double* rowscale = nullptr);
 // Dense assembly of A.
 int pair_assemble(inti_ctx* ctx, const PairLaunch& L, double* out);
-// Single-launch form of small FP64 products (one cluster kernel: source
+// Single-launch form of small FP64 products (one kernel: source
 // records, pair sums, correction rows, alpha/beta): operators of at most
 // kSmallPairs pairs.  rowscale (nullable) scales row i's pair sum, as the
 // epilogue does for transposed products (the source weights).

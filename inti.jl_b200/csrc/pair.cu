@@ -21,7 +21,6 @@
 //    carries no O(N eps) growth.
 //  * The epilogue applies the kernel constant, alpha/beta, and the CSR
 //    correction row in the same pass (the fused near-field correction).
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -563,55 +562,59 @@ __global__ void pair_epilogue_kernel(EpiArgs e) {
 // Single-launch form for small FP64 operators (m*n up to kSmallPairs, e.g.
 // the 1,000-node kite): one kernel per product, no pack.  The tiled kernels
 // give such a problem a handful of CTAs whose threads each run a long chain
-// of dependent global loads, so the launch is latency-bound.  Here a
-// cluster of S CTAs takes 32 targets (one per lane); CTA s of the cluster
-// takes the s-th slice of the sources, builds their records in shared memory
-// from the raw nodes (build_record, kSmallTile at a time), and its warps
-// split each staged tile.  S is chosen on the host so that the clusters
-// fill the SMs.  The correction row of a target is split over the same
-// S * kSmallWarps threads (entry p0 + s*kSmallWarps + warp, then strides of
-// S*kSmallWarps); the first kSmallCorr entries of a thread are fetched before
-// the pair loop so their latency hides behind it.  The warps' pair and
-// correction sums are added in a fixed order, then the slices' sums, read
-// by CTA 0 of the cluster from its peers' shared memory (distributed shared
-// memory), in slice order; CTA 0 then applies the kernel constant to the
-// pair sum, adds the correction sum and alpha/beta.  The step is
-// pair_step's (the one-sided kernel's arithmetic).
+// of dependent global loads, so the launch is latency-bound.  Here a target
+// has k warps (1 to 16, chosen on the host so that the CTAs of 16 warps fill
+// the SMs).  A CTA builds the source records in shared memory from
+// the raw nodes (build_record, a tile at a time), the lanes of a target's
+// warps take every 32k-th record of the tile, and one correction entry each
+// (fetched before the pair loop, so that its latency hides behind it).  The
+// lanes' sums are reduced over the warp, the warps' in a fixed order, and lane
+// 0 of the target's first warp applies the kernel constant to the pair sum, adds
+// the correction sum and alpha/beta.  The step is pair_step's (the one-sided
+// kernel's arithmetic).
+//
+// What bounds it is the launch and two L2 latencies.  An earlier form gave a
+// cluster of CTAs 32 targets, one per lane, and added the slices' sums through
+// distributed shared memory.  Back to back products (start of a kernel seen in
+// steps of about 1 us): 2D DL, 1,000 nodes 8.19 -> 7.17 us, 2D SL 13.3 -> 10.2,
+// Helmholtz SL, 768 nodes 10.2 -> 8.2; eight warps per CTA 8.19, 12.3 and 8.2.
 // ---------------------------------------------------------------------------
-constexpr int kSmallWarps = 8;
-constexpr int kSmallTile = 32 * kSmallWarps;  // sources staged per pass, one per thread
-constexpr int kSmallMaxSlices = 8;            // portable cluster size
-constexpr int kSmallCorr = 2;                 // correction entries per thread fetched ahead
+constexpr int kSmallWarps = 16;
 
 struct SmallSources {
   const double *xs, *ns, *w, *sigma;
   double2 c1, c2;
 };
 
+// Records per staged tile: one or two per thread, up to 40 KB.
+template <int N>
+constexpr int small_tile() {
+  return N <= 4 ? 1024 : 512;
+}
+
 template <int PDE, int KIND, int DIM>
 __global__ void __launch_bounds__(32 * kSmallWarps) pair_small_kernel(int64_t m, int64_t n, const double* tc,
                                                                       const double* tn, SmallSources src,
                                                                       double k, double kT, double delta,
-                                                                      const double2* expi, EpiArgs e) {
-  namespace cg = cooperative_groups;
+                                                                      const double2* expi, int lk, EpiArgs e) {
   using RC = Rec<PDE, KIND, DIM, double>;
   constexpr bool CPLX = RC::cplx;
-  // the staged records; after the last tile, the warps' sums (pair, correction)
-  __shared__ __align__(16) double recs[kSmallTile * RC::n];
-  __shared__ double4 slice_sum[32];
+  constexpr int NT = 32 * kSmallWarps;
+  constexpr int TILE = small_tile<RC::n>();
+  extern __shared__ __align__(16) double recs[];  // TILE records
+  __shared__ double4 sums[kSmallWarps];
   __shared__ double2 tab[CPLX ? kExpiTable : 1];
-  static_assert(kSmallTile * RC::n >= 4 * 32 * kSmallWarps, "the sums reuse the record buffer");
-  cg::cluster_group cl = cg::this_cluster();
-  const int64_t slices = cl.num_blocks(), slice = cl.block_rank();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t i = (blockIdx.x / slices) * 32 + lane;
-  const bool lead = slice == 0 && warp == 0;
+  const int kw = 1 << lk, sub = warp & (kw - 1);  // warps of a target; this one
+  const int64_t i = (int64_t)blockIdx.x * (kSmallWarps >> lk) + (warp >> lk);
+  const bool live = i < m;
   if (CPLX)
-    for (int q = threadIdx.x; q < kExpiTable; q += 32 * kSmallWarps) tab[q] = expi[q];
+    for (int q = threadIdx.x; q < kExpiTable; q += NT) tab[q] = expi[q];
   Target<double, DIM, RC::tnormal> t;
-  int64_t p = 0, p1 = 0;  // this thread's next correction entry, row end
-  double2 yo = make_double2(0.0, 0.0);
-  if (i < m) {
+  int64_t p = 0, p1 = 0;  // this lane's next correction entry, row end
+  double2 yo = make_double2(0.0, 0.0), cv = yo;
+  int32_t cj = -1;
+  if (live) {
 #pragma unroll
     for (int c = 0; c < DIM; ++c) t.x[c] = tc[DIM * i + c];
     if constexpr (RC::tnormal) {
@@ -619,99 +622,76 @@ __global__ void __launch_bounds__(32 * kSmallWarps) pair_small_kernel(int64_t m,
       for (int c = 0; c < DIM; ++c) t.n[c] = tn[DIM * i + c];
     }
     if (e.rowptr) {
-      p = e.rowptr[i] + slice * kSmallWarps + warp;
+      p = e.rowptr[i] + sub * 32 + lane;
       p1 = e.rowptr[i + 1];
     }
-    if (lead && !e.beta_zero) yo = epilogue_y_old<CPLX>(e, i);
+    if (lane == 0 && sub == 0 && !e.beta_zero) yo = epilogue_y_old<CPLX>(e, i);
   }
-  const int64_t pstride = slices * kSmallWarps;
-  const int64_t per = (n + slices - 1) / slices;
-  const int64_t j0 = slice * per, j1 = j0 + per < n ? j0 + per : n;
-  double ar = 0.0, ai = 0.0;
-  int32_t cc[kSmallCorr];
-  double2 cv[kSmallCorr];
-  for (int64_t base = j0; base < j1; base += kSmallTile) {
-    const int cnt = (int)(j1 - base < kSmallTile ? j1 - base : kSmallTile);
-    __syncthreads();  // the previous tile is consumed
-    if (threadIdx.x < cnt) {
-      double rec[RC::n];
-      build_record<PDE, KIND, DIM, double>(base + threadIdx.x, n, src.xs, src.ns, src.w, src.sigma, src.c1,
-                                           src.c2, rec);
-      double2* o = reinterpret_cast<double2*>(recs + threadIdx.x * RC::n);
-#pragma unroll
-      for (int c = 0; c < RC::n / 2; ++c) o[c] = make_double2(rec[2 * c], rec[2 * c + 1]);
-    }
-    if (base == j0) {
-      // correction entries fetched ahead (their values are used after the pair loop)
-#pragma unroll
-      for (int u = 0; u < kSmallCorr; ++u) {
-        const int64_t pu = p + u * pstride;
-        cc[u] = pu < p1 ? e.col[pu] : -1;
-        cv[u] = pu < p1 ? (CPLX ? reinterpret_cast<const double2*>(e.val)[pu] : make_double2(e.val[pu], 0.0))
-                        : make_double2(0.0, 0.0);
-      }
-    }
-    __syncthreads();
-    if (i < m) {
-      const int pw = (cnt + kSmallWarps - 1) / kSmallWarps;
-      const int q0 = warp * pw, q1 = q0 + pw < cnt ? q0 + pw : cnt;
-      for (int q = q0; q < q1; ++q) pair_step<PDE, KIND, DIM, double>(t, recs + q * RC::n, kT, delta, k, tab, ar, ai);
-    }
-  }
-  if (j0 >= j1) {  // an empty slice still fetches its correction entries
-#pragma unroll
-    for (int u = 0; u < kSmallCorr; ++u) {
-      const int64_t pu = p + u * pstride;
-      cc[u] = pu < p1 ? e.col[pu] : -1;
-      cv[u] = pu < p1 ? (CPLX ? reinterpret_cast<const double2*>(e.val)[pu] : make_double2(e.val[pu], 0.0))
-                      : make_double2(0.0, 0.0);
-    }
-  }
-  double cr = 0.0, ci = 0.0;
-  auto corr_add = [&](int32_t j, double2 v) {
-    if (CPLX) {
-      const double2 xv = reinterpret_cast<const double2*>(e.x)[j];
-      cr = fma(v.x, xv.x, fma(-v.y, xv.y, cr));
-      ci = fma(v.x, xv.y, fma(v.y, xv.x, ci));
-    } else {
-      cr = fma(v.x, e.x[j], cr);
-    }
+  auto entry = [&]() {  // value and column of entry p
+    cj = e.col[p];
+    cv = CPLX ? reinterpret_cast<const double2*>(e.val)[p] : make_double2(e.val[p], 0.0);
   };
+  double ar = 0.0, ai = 0.0, cr = 0.0, ci = 0.0;
+  // A thread's records of a tile: all loads before the first store to shared
+  // memory (which the compiler may not move them across), the next tile's
+  // before the pairs of this one.
+  constexpr int U = TILE / NT;
+  double rec[U][RC::n];
+  auto fetch = [&](int64_t base) {
 #pragma unroll
-  for (int u = 0; u < kSmallCorr; ++u)
-    if (cc[u] >= 0) corr_add(cc[u], cv[u]);
-  for (int64_t pu = p + kSmallCorr * pstride; pu < p1; pu += pstride)
-    corr_add(e.col[pu], CPLX ? reinterpret_cast<const double2*>(e.val)[pu] : make_double2(e.val[pu], 0.0));
-  __syncthreads();  // every warp is done with the records: reuse them for the sums
-  double4* part = reinterpret_cast<double4*>(recs);  // [warp][lane]
-  part[warp * 32 + lane] = make_double4(ar, ai, cr, ci);
-  __syncthreads();
-  if (warp == 0) {
-    double4 acc = make_double4(0.0, 0.0, 0.0, 0.0);
+    for (int u = 0; u < U; ++u)
+      build_record<PDE, KIND, DIM, double>(base + threadIdx.x + u * NT, n, src.xs, src.ns, src.w, src.sigma, src.c1,
+                                           src.c2, rec[u]);
+  };
+  fetch(0);
+  for (int64_t base = 0; base < n; base += TILE) {
+    const int cnt = (int)(n - base < TILE ? n - base : TILE);
+    if (base) __syncthreads();  // the previous tile is consumed
 #pragma unroll
-    for (int w = 0; w < kSmallWarps; ++w) {
-      const double4 v = part[w * 32 + lane];
-      acc.x += v.x;
-      acc.y += v.y;
-      acc.z += v.z;
-      acc.w += v.w;
+    for (int u = 0; u < U; ++u) {
+      double2* o = reinterpret_cast<double2*>(recs + (threadIdx.x + u * NT) * RC::n);
+#pragma unroll
+      for (int c = 0; c < RC::n / 2; ++c) o[c] = make_double2(rec[u][2 * c], rec[u][2 * c + 1]);
     }
-    slice_sum[lane] = acc;
+    if (base == 0 && p < p1) entry();
+    __syncthreads();
+    if (base + TILE < n) fetch(base + TILE);
+    if (live) {
+      constexpr int UNROLL = PDE == LAPLACE && KIND == SL && DIM == 2 ? 1 : 4;  // (a log is long enough)
+#pragma unroll UNROLL
+      for (int q = sub * 32 + lane; q < cnt; q += 32 * kw)
+        pair_step<PDE, KIND, DIM, double>(t, recs + q * RC::n, kT, delta, k, tab, ar, ai);
+    }
   }
-  cl.sync();  // every slice's sums are in its shared memory
-  if (lead && i < m) {
-    double4 acc = make_double4(0.0, 0.0, 0.0, 0.0);
-    for (int r = 0; r < (int)slices; ++r) {
-      const double4 v = *cl.map_shared_rank(&slice_sum[lane], r);
-      acc.x += v.x;
-      acc.y += v.y;
-      acc.z += v.z;
-      acc.w += v.w;
+  while (cj >= 0) {
+    if (CPLX) {
+      const double2 xv = reinterpret_cast<const double2*>(e.x)[cj];
+      cr = fma(cv.x, xv.x, fma(-cv.y, xv.y, cr));
+      ci = fma(cv.x, xv.y, fma(cv.y, xv.x, ci));
+    } else {
+      cr = fma(cv.x, e.x[cj], cr);
     }
+    cj = -1;
+    p += 32 * kw;
+    if (p < p1) entry();
+  }
+  double4 acc = make_double4(warp_sum(ar), CPLX ? warp_sum(ai) : 0.0, warp_sum(cr), CPLX ? warp_sum(ci) : 0.0);
+  if (kw > 1) {
+    if (lane == 0) sums[warp] = acc;
+    __syncthreads();
+    if (sub == 0)
+      for (int w = 1; w < kw; ++w) {
+        const double4 v = sums[warp + w];
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+      }
+  }
+  if (live && lane == 0 && sub == 0) {
     const double sc = e.rowscale ? e.scale * e.rowscale[i] : e.scale;
     epilogue_store<CPLX>(e, i, fma(acc.x, sc, acc.z), fma(acc.y, sc, acc.w), yo);
   }
-  cl.sync();  // the peers' shared memory stays valid until CTA 0 has read it
 }
 
 // ---------------------------------------------------------------------------
@@ -2070,11 +2050,12 @@ bool pair_small_eligible(int precision, int64_t m, int64_t n) {
   return precision == INTI_FP64 && (double)m * (double)n <= kSmallPairs && m > 0 && n > 0 && n <= 65536;
 }
 
-static int pair_small_slices(int num_sms, int64_t m, int64_t n) {
-  const int64_t rows = (m + 31) / 32;
-  int s = 1;
-  while (s < kSmallMaxSlices && rows * 2 * s <= num_sms && n >= (int64_t)64 * 2 * s) s *= 2;
-  return s;
+// log2 of the warps per target: until the CTAs fill the SMs, while a lane
+// keeps at least four records.
+static int pair_small_warps(int num_sms, int64_t m, int64_t n) {
+  int lk = 0;
+  while ((1 << lk) < kSmallWarps && (m << (lk + 1)) <= (int64_t)num_sms * kSmallWarps && n >= (int64_t)128 << (lk + 1)) ++lk;
+  return lk;
 }
 
 int pair_small(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, const double* x, double* y,
@@ -2097,26 +2078,20 @@ int pair_small(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, const d
   e.beta_zero = (e.br == 0.0 && e.bi == 0.0);
   const SmallSources src{L.scoords, L.snormals, L.sweights, L.x, make_double2(L.c1[0], L.c1[1]),
                          make_double2(L.c2[0], L.c2[1])};
-  const int slices = pair_small_slices(ctx->num_sms, L.m, L.n);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = slices;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((L.m + 31) / 32 * slices));
-  cfg.blockDim = dim3(32 * kSmallWarps);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = ctx->stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  const int lk = pair_small_warps(ctx->num_sms, L.m, L.n);
+  const unsigned grid = (unsigned)((L.m + (kSmallWarps >> lk) - 1) / (kSmallWarps >> lk));
   const double2* expi = L.pde == HELMHOLTZ ? expi_table_f64(ctx) : nullptr;
   const double kT = L.k * kExpiTable / (2 * kPi), delta = 2 * kPi / kExpiTable;
   dispatch(L.pde, L.kind, L.dim, [&](auto tag) {
     using T = decltype(tag);
     ProfScope pp(ctx, "pair");
-    INTI_CUDA(cudaLaunchKernelEx(&cfg, pair_small_kernel<T::pde, T::kind, T::dim>, (int64_t)L.m, (int64_t)L.n,
-                                 L.tcoords, L.tnormals, src, (double)L.k, kT, delta, expi, e));
+    constexpr int N = Rec<T::pde, T::kind, T::dim, double>::n;
+    constexpr size_t sm = sizeof(double) * N * small_tile<N>();
+    if (sm + (T::pde == HELMHOLTZ ? 17408 : 1024) > 48 * 1024)
+      INTI_CUDA(cudaFuncSetAttribute(pair_small_kernel<T::pde, T::kind, T::dim>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    pair_small_kernel<T::pde, T::kind, T::dim><<<grid, 32 * kSmallWarps, sm, ctx->stream>>>(
+        L.m, L.n, L.tcoords, L.tnormals, src, L.k, kT, delta, expi, lk, e);
   });
   INTI_CUDA(cudaGetLastError());
   ctx->launches += 1;
