@@ -323,9 +323,11 @@ int pair_symm_default_ch(const inti_ctx* ctx, int pde, int kind, int dim, int pr
 // CTAs per item: small operators, whose items (one source block each) do not
 // fill the device, give every item's block to several CTAs.
 int pair_symm_sub(const inti_ctx* ctx, int tpt, int ch, int nitems);
-// Choose the split for a problem on this device.
+// Targets per thread and source chunks of a one-sided product on this device
+// (FP64: more chunks than tiles are parts of tiles).
+int pair_plan_tpt(const inti_ctx* ctx, int precision, int64_t m, int64_t n);
 int pair_plan_split(const inti_ctx* ctx, int pde, int kind, int dim, int precision, int64_t m,
-                    int64_t n, int tpt = 4);
+                    int64_t n, int tpt);
 // Enqueue pack + pair kernels (results in L.partial); returns launches.
 int pair_launch(inti_ctx* ctx, const PairLaunch& L);
 // y = alpha*(scale*rowscale_i*sum_s partial + C x) + beta*y (rowscale NULL:

@@ -65,7 +65,8 @@ inti_op* op_create(inti_ctx* ctx, int pde, int kernel, double k_re, double k_im,
   op->corr = correction;
   const int64_t tile = pair_tile(precision);
   op->n_tiles = std::max<int64_t>(1, (source->n + tile - 1) / tile);
-  op->split = pair_plan_split(ctx, pde, kernel, dim, precision, target->n, source->n);
+  op->tpt = pair_plan_tpt(ctx, precision, target->n, source->n);
+  op->split = pair_plan_split(ctx, pde, kernel, dim, precision, target->n, source->n, op->tpt);
   op_symm_init(op.get());
   if (!op->symm) {
     // the one-sided records and partials (the symmetric form packs its own
@@ -110,7 +111,8 @@ inti_op* op_create_combined(inti_ctx* ctx, int pde, double k_re, double k_im, co
   }
   const int64_t tile = pair_tile(precision);
   op->n_tiles = std::max<int64_t>(1, (source->n + tile - 1) / tile);
-  op->split = pair_plan_split(ctx, pde, CF, 3, precision, target->n, source->n);
+  op->tpt = pair_plan_tpt(ctx, precision, target->n, source->n);
+  op->split = pair_plan_split(ctx, pde, CF, 3, precision, target->n, source->n, op->tpt);
   op_symm_init(op.get());
   if (!op->symm) {
     op->packed.ensure((size_t)op->n_tiles * tile * pair_record_bytes(pde, CF, 3, precision));
@@ -140,7 +142,8 @@ inti_op* op_clone_precision(const inti_op* op, int precision) {
   }
   const int64_t tile = pair_tile(precision);
   t->n_tiles = std::max<int64_t>(1, (op->source->n + tile - 1) / tile);
-  t->split = pair_plan_split(op->ctx, op->pde, op->kind, op->dim, precision, op->target->n, op->source->n);
+  t->tpt = pair_plan_tpt(op->ctx, precision, op->target->n, op->source->n);
+  t->split = pair_plan_split(op->ctx, op->pde, op->kind, op->dim, precision, op->target->n, op->source->n, t->tpt);
   op_symm_init(t.get());
   if (!t->symm) {
     t->packed.ensure((size_t)t->n_tiles * tile * pair_record_bytes(op->pde, op->kind, op->dim, precision));
@@ -453,8 +456,8 @@ void op_prepare_transpose(inti_op* op) {
     op->ttpt = it->second.first;
     op->tsplit = it->second.second;
   } else {
-    op->ttpt = 4;
-    op->tsplit = pair_plan_split(ctx, op->pde, kt, op->dim, op->precision, m2, n2, 4);
+    op->ttpt = pair_plan_tpt(ctx, op->precision, m2, n2);
+    op->tsplit = pair_plan_split(ctx, op->pde, kt, op->dim, op->precision, m2, n2, op->ttpt);
   }
   op->tpacked.ensure((size_t)op->tn_tiles * tile * pair_record_bytes(op->pde, kt, op->dim, op->precision));
   if (op->symm)  // the symmetric form packs all npad = n_tiles * tile nodes in its own records

@@ -38,6 +38,7 @@ namespace inti {
 constexpr int kBlock = 128;  // threads per CTA
 constexpr int kTPT = 4;      // targets per thread
 constexpr int kTile64 = 128; // sources per shared-memory stage (FP64)
+constexpr int kFineTile = 32;  // sources per stage where whole tiles leave SMs idle (FP64)
 constexpr int kTile32 = 256; // sources per shared-memory stage (FP32C)
 constexpr int kGroup = 32;   // FP32C: sources summed before a compensated fold
 
@@ -343,6 +344,29 @@ __device__ __forceinline__ void store_partial(float2* p, const Acc<float, false>
 __device__ __forceinline__ void store_partial(float4* p, const Acc<float, true>& a) {
   *p = make_float4(a.hr, a.lr, a.hi, a.li);
 }
+__device__ __forceinline__ void add_partial(Acc<double, false>& a, double p) { a.r += p; }
+__device__ __forceinline__ void add_partial(Acc<double, true>& a, double2 p) {
+  a.r += p.x;
+  a.i += p.y;
+}
+
+// Slices of a CTA of pair_forward.  FP64: the four warps have the same targets
+// and a quarter of a tile's sources each, so that few targets still make many
+// CTAs and their chunks' partial sums stay four times fewer.  What bounds the
+// kernel is the FP64 pipe once an SM has some 12 CTAs; below that, idle SMs
+// and latency.  With a target block per warp and thread-per-row epilogues,
+// products back to back, Laplace DL: 51,894 sources x 4,096 / 1,000 / 100
+// targets 280 / 113 / 105 us, 3,456 x 1,000 51.2; now 248 / 70 / 20 and 12.1.
+// FP32C keeps one slice: its groups of sums are folded in the order of the
+// tile.
+template <class R>
+constexpr int fwd_slices() {
+  return std::is_same<R, float>::value ? 1 : kBlock / 32;
+}
+// Targets per CTA of pair_forward.
+static int64_t fwd_rows(int precision, int tpt) {
+  return (int64_t)tpt * kBlock / (precision == INTI_FP32C ? fwd_slices<float>() : fwd_slices<double>());
+}
 
 struct FwdArgs {
   int64_t m;
@@ -372,7 +396,9 @@ __global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
   __shared__ __align__(8) uint64_t full[2];
 
   const int tid = threadIdx.x;
-  const int64_t base = (int64_t)blockIdx.x * (kBlock * TPT);
+  constexpr int NSL = fwd_slices<R>(), kRows = kBlock / NSL;  // a slice's threads: one target each, TPT times
+  const int row = tid % kRows, slice = tid / kRows;
+  const int64_t base = (int64_t)blockIdx.x * (kRows * TPT);
   const int split = blockIdx.y;
   const int64_t t0 = (int64_t)split * a.tiles_per_split;
   const int64_t t1 = min(a.n_tiles, t0 + a.tiles_per_split);
@@ -383,7 +409,7 @@ __global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
   Acc<R, CPLX> acc[TPT];
 #pragma unroll
   for (int u = 0; u < TPT; ++u) {
-    const int64_t i = min(base + u * kBlock + tid, a.m - 1);
+    const int64_t i = min(base + u * kRows + row, a.m - 1);
 #pragma unroll
     for (int c = 0; c < DIM; ++c) tg[u].x[c] = R(a.tcoords[DIM * i + c]);
     if (RC::tnormal) {
@@ -429,10 +455,11 @@ __global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
       return;
     }
     const R* sp = st ? stage1 : stage0;
+    constexpr int kShare = TILE / NSL, kRun = kShare < kGroup ? kShare : kGroup;
 #pragma unroll 1
-    for (int g = 0; g < TILE; g += kGroup) {
+    for (int g = slice * kShare; g < (slice + 1) * kShare; g += kRun) {
 #pragma unroll 2
-      for (int s = 0; s < kGroup; ++s) {
+      for (int s = 0; s < kRun; ++s) {
         const R* rec = sp + (g + s) * RC::n;
 #pragma unroll
         for (int u = 0; u < TPT; ++u)
@@ -450,9 +477,23 @@ __global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
     }
   }
   P* out = static_cast<P*>(a.partial) + (int64_t)split * a.m;
+  if constexpr (NSL > 1) {
+    // the slices' sums, added in a fixed order (the stages are free: every
+    // tile issued was waited for)
+    static_assert((NSL - 1) * kRows * TPT * sizeof(P) <= 2 * kStageBytes, "the slices' sums fit the stages");
+    P* red = reinterpret_cast<P*>(smem_raw);
+#pragma unroll
+    for (int u = 0; u < TPT; ++u)
+      if (slice > 0) store_partial(red + ((slice - 1) * TPT + u) * kRows + row, acc[u]);
+    __syncthreads();
+    if (slice > 0) return;
+#pragma unroll
+    for (int u = 0; u < TPT; ++u)
+      for (int q = 1; q < NSL; ++q) add_partial(acc[u], red[((q - 1) * TPT + u) * kRows + row]);
+  }
 #pragma unroll
   for (int u = 0; u < TPT; ++u) {
-    const int64_t i = base + u * kBlock + tid;
+    const int64_t i = base + u * kRows + row;
     if (i < a.m) store_partial(out + i, acc[u]);
   }
 }
@@ -510,52 +551,79 @@ __device__ __forceinline__ void epilogue_store(const EpiArgs& e, int64_t i, doub
   }
 }
 
-// Kernel constant, correction row, alpha/beta and the store for row i, given
-// the row's pair sum (sr, si).
-template <bool CPLX>
-__device__ __forceinline__ void epilogue_finish(const EpiArgs& e, int64_t i, double sr, double si) {
-  const double sc = e.rowscale ? e.scale * e.rowscale[i] : e.scale;
-  sr *= sc;
-  si *= sc;
-  if (e.rowptr) {
-    const int64_t p0 = e.rowptr[i], p1 = e.rowptr[i + 1];
-    for (int64_t p = p0; p < p1; ++p) {
-      const int32_t j = e.col[p];
-      if (CPLX) {
-        const double2 v = reinterpret_cast<const double2*>(e.val)[p];
-        const double2 xv = reinterpret_cast<const double2*>(e.x)[j];
-        sr = fma(v.x, xv.x, fma(-v.y, xv.y, sr));
-        si = fma(v.x, xv.y, fma(v.y, xv.x, si));
-      } else {
-        sr = fma(e.val[p], e.x[j], sr);
-      }
-    }
-  }
-  epilogue_store<CPLX>(e, i, sr, si, e.beta_zero ? make_double2(0.0, 0.0) : epilogue_y_old<CPLX>(e, i));
-}
-
+// y_i = alpha*(scale*pair sum + correction row) + beta*y_i for `nodes` rows per
+// CTA, and for each as many threads as that leaves: thread
+// sl of a row sums every slices-th chunk and correction entry, and the sums
+// are added in a fixed order.
 template <class P, bool CPLX>
-__global__ void pair_epilogue_kernel(EpiArgs e) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__global__ void pair_epilogue_kernel(EpiArgs e, int nodes) {
+  extern __shared__ double4 epi_part[];  // slices x nodes, for more than one slice
+  const int tn = threadIdx.x % nodes, sl = threadIdx.x / nodes, slices = blockDim.x / nodes;
+  const int64_t i = blockIdx.x * (int64_t)nodes + tn;
   pdl_trigger();
   pdl_wait();
-  if (i >= e.m) return;
   if (e.err && *e.err) {  // the partial sums are incomplete: make the failure visible in y
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    if (sl > 0 || i >= e.m) return;
     if (CPLX)
       reinterpret_cast<double2*>(e.y)[i] = make_double2(nan, nan);
     else
       e.y[i] = nan;
     return;
   }
-  const P* part = static_cast<const P*>(e.partial);
-  double sr = 0.0, si = 0.0;
-  for (int s = 0; s < e.split; ++s) {
-    const double2 v = load_partial(part + (int64_t)s * e.m + i);
-    sr += v.x;
-    si += v.y;
+  double4 c = make_double4(0.0, 0.0, 0.0, 0.0);  // pair sum, correction sum
+  if (i < e.m) {
+    const P* part = static_cast<const P*>(e.partial) + i;
+#pragma unroll 4
+    for (int s = sl; s < e.split; s += slices) {
+      const double2 v = load_partial(part + (int64_t)s * e.m);
+      c.x += v.x;
+      c.y += v.y;
+    }
+    if (e.rowptr) {
+      for (int64_t p = e.rowptr[i] + sl, p1 = e.rowptr[i + 1]; p < p1; p += slices) {
+        const int32_t j = e.col[p];
+        if (CPLX) {
+          const double2 v = reinterpret_cast<const double2*>(e.val)[p];
+          const double2 xv = reinterpret_cast<const double2*>(e.x)[j];
+          c.z = fma(v.x, xv.x, fma(-v.y, xv.y, c.z));
+          c.w = fma(v.x, xv.y, fma(v.y, xv.x, c.w));
+        } else {
+          c.z = fma(e.val[p], e.x[j], c.z);
+        }
+      }
+    }
   }
-  epilogue_finish<CPLX>(e, i, sr, si);
+  if (slices > 1) {
+    epi_part[threadIdx.x] = c;
+    __syncthreads();
+    if (sl > 0) return;
+    for (int q = 1; q < slices; ++q) {
+      const double4 v = epi_part[q * nodes + tn];
+      c.x += v.x;
+      c.y += v.y;
+      c.z += v.z;
+      c.w += v.w;
+    }
+  }
+  if (i >= e.m) return;
+  const double sc = e.rowscale ? e.scale * e.rowscale[i] : e.scale;
+  epilogue_store<CPLX>(e, i, fma(c.x, sc, c.z), fma(c.y, sc, c.w),
+                       e.beta_zero ? make_double2(0.0, 0.0) : epilogue_y_old<CPLX>(e, i));
+}
+
+struct EpiShape {
+  int nodes, slices;
+  unsigned threads() const { return (unsigned)(nodes * slices); }
+  unsigned blocks(int64_t m) const { return (unsigned)((m + nodes - 1) / nodes); }
+  size_t smem() const { return slices > 1 ? sizeof(double4) * threads() : 0; }
+};
+// The rows of few chunks have enough threads with one each; with more, a
+// row's chunks are one long chain of loads and are split over 8 or 32
+// (1,000 rows: 203 chunks 31.8 us with a thread per row, 406 chunks 6.6 with 32).
+static EpiShape epi_shape(int split) {
+  if (split < 8) return {256, 1};
+  return {32, split < 64 ? 8 : 32};
 }
 
 // ---------------------------------------------------------------------------
@@ -1630,34 +1698,48 @@ static const void* fwd_kernel_ptr() {
 }
 
 template <class T, class R>
-static size_t fwd_smem() {
-  constexpr int TILE = std::is_same<R, float>::value ? kTile32 : kTile64;
+static size_t fwd_smem(int tile = std::is_same<R, float>::value ? kTile32 : kTile64) {
   const size_t table = T::pde == HELMHOLTZ ? (size_t)kExpiTable * 2 * sizeof(R) : 0;
-  return 2 * (size_t)TILE * Rec<T::pde, T::kind, T::dim, R>::n * sizeof(R) + table;
+  return 2 * (size_t)tile * Rec<T::pde, T::kind, T::dim, R>::n * sizeof(R) + table;
 }
 
+// Source chunks of a product of m targets and n sources.  FP64: chunks of
+// whole tiles until an SM has 20 CTAs; where two targets per thread and whole
+// tiles leave fewer than 10 per SM, parts of tiles (32 sources, and more chunks
+// than tiles say so) until it has 12.  Equal CTAs that nearly fill one wave
+// leave the SMs unevenly loaded, and few CTAs leave their latencies bare.
+// Products back to back, Laplace DL: 51,894 sources x 1,000 targets with 2,
+// 5.5, 11 and 22 CTAs per SM 236, 108, 72 and 70 us; 12,150 x 500 with whole
+// tiles (5) 21.4, parts at 7, 10 and 20 per SM 18.7, 15.8 and 16.4; 3,456 x
+// 1,000 whole tiles (3) 20.1, parts (6, 12) 14.0 and 12.1; but 3,456 x 4,096
+// whole tiles (11.7) 24.5, parts 24.8.
 int pair_plan_split(const inti_ctx* ctx, int pde, int kind, int dim, int precision, int64_t m,
                     int64_t n, int tpt) {
   if (tpt != 2 && tpt != 4) throw Error(INTI_E_ARG, "targets per thread must be 2 or 4");
+  if (precision == INTI_FP64) {
+    const int64_t blocks = (m + fwd_rows(precision, tpt) - 1) / fwd_rows(precision, tpt);
+    const int64_t tiles = std::max<int64_t>(1, (n + kTile64 - 1) / kTile64);
+    const int64_t units = tiles * (kTile64 / kFineTile), sms = ctx->num_sms;
+    if (tpt == 2 && blocks * tiles < 10 * sms) {
+      const int64_t per = std::max<int64_t>(1, (units * blocks + 6 * sms) / (12 * sms));
+      const int64_t split = (units + per - 1) / per;
+      if (split > tiles) return (int)split;
+    }
+    const int64_t per = std::max<int64_t>(1, tiles * blocks / (20 * sms));
+    return (int)((tiles + per - 1) / per);
+  }
   int occ = 1;
   dispatch(pde, kind, dim, [&](auto tag) {
     using T = decltype(tag);
-    const void* fn;
-    size_t sm;
-    if (precision == INTI_FP32C) {
-      fn = tpt == 2 ? fwd_kernel_ptr<T, float, 2>() : fwd_kernel_ptr<T, float, 4>();
-      sm = fwd_smem<T, float>();
-    } else {
-      fn = tpt == 2 ? fwd_kernel_ptr<T, double, 2>() : fwd_kernel_ptr<T, double, 4>();
-      sm = fwd_smem<T, double>();
-    }
+    const void* fn = tpt == 2 ? fwd_kernel_ptr<T, float, 2>() : fwd_kernel_ptr<T, float, 4>();
+    const size_t sm = fwd_smem<T, float>();
     INTI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     INTI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBlock, sm));
   });
   occ = std::max(occ, 1);
   const int64_t tile = pair_tile(precision);
   const int64_t n_tiles = std::max<int64_t>(1, (n + tile - 1) / tile);
-  const int64_t blocks = (m + kBlock * tpt - 1) / (kBlock * tpt);
+  const int64_t blocks = (m + fwd_rows(precision, tpt) - 1) / fwd_rows(precision, tpt);
   const int64_t slots = (int64_t)ctx->num_sms * occ;
   // Smallest split whose last wave is >= 90% full (or that reaches 8
   // waves), never more chunks than source tiles.  Up to kMaxSplit chunks:
@@ -1679,6 +1761,15 @@ int pair_plan_split(const inti_ctx* ctx, int pde, int kind, int dim, int precisi
     }
   }
   return best;
+}
+
+// Targets per thread: four, unless whole tiles then give an SM fewer than 12
+// CTAs (Laplace DL, 12,150 sources x 2,000 targets, 10 per SM: 55.4 us with
+// four, 38.6 with two; 51,894 x 1,000, 22 per SM: 70.1 and 71.2).
+int pair_plan_tpt(const inti_ctx* ctx, int precision, int64_t m, int64_t n) {
+  if (precision != INTI_FP64) return 4;
+  const int64_t rows = fwd_rows(precision, 4);
+  return (m + rows - 1) / rows * ((n + kTile64 - 1) / kTile64) < 12 * (int64_t)ctx->num_sms ? 2 : 4;
 }
 
 // Dynamic shared memory of the symmetric kernel: two source stages, the
@@ -1950,11 +2041,20 @@ int pair_launch(inti_ctx* ctx, const PairLaunch& L) {
       a.expi = std::is_same<R, float>::value ? (const void*)expi_table_f32(ctx) : (const void*)expi_table_f64(ctx);
       a.err = L.err_flag;
       ctx->flag_armed = true;
-      const size_t sm = fwd_smem<T, R>();
+      size_t sm = fwd_smem<T, R>();
       auto fn = L.tpt == 2 ? &pair_forward<T::pde, T::kind, T::dim, R, TILE, 2>
                            : &pair_forward<T::pde, T::kind, T::dim, R, TILE, 4>;
+      if constexpr (!std::is_same<R, float>::value) {
+        if (L.tpt == 2 && L.split > L.n_tiles) {
+          fn = &pair_forward<T::pde, T::kind, T::dim, R, kFineTile, 2>;
+          sm = fwd_smem<T, R>(kFineTile);
+          a.n_tiles = npad / kFineTile;
+          a.tiles_per_split = (int)((a.n_tiles + L.split - 1) / L.split);
+        }
+      }
       INTI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      dim3 grid((unsigned)((L.m + kBlock * L.tpt - 1) / (kBlock * L.tpt)), (unsigned)L.split);
+      const int64_t rows = fwd_rows(L.precision, L.tpt);
+      dim3 grid((unsigned)((L.m + rows - 1) / rows), (unsigned)L.split);
       ProfScope pp(ctx, "pair");
       launch_pdl(ctx->stream, grid, kBlock, sm, fn, a);
       launches = 2;
@@ -1987,8 +2087,7 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
   e.br = beta ? beta[0] : 0.0;
   e.bi = beta ? beta[1] : 0.0;
   e.beta_zero = (e.br == 0.0 && e.bi == 0.0);
-  const int tb = 256;
-  const unsigned gb = (unsigned)((L.m + tb - 1) / tb);
+  const EpiShape es = epi_shape(L.symm ? 1 : L.split);
   const bool cplx = L.pde == HELMHOLTZ;
   ProfScope pe(ctx, "epilogue");
   if (L.symm && L.sym_npanels > 1) {
@@ -1996,9 +2095,9 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
     e.partial = L.sym_acc;
     e.split = 1;
     if (cplx)
-      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double2, true>, e);
+      launch_pdl(ctx->stream, es.blocks(L.m), es.threads(), es.smem(), &pair_epilogue_kernel<double2, true>, e, es.nodes);
     else
-      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double, false>, e);
+      launch_pdl(ctx->stream, es.blocks(L.m), es.threads(), es.smem(), &pair_epilogue_kernel<double, false>, e, es.nodes);
     INTI_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return 1;
@@ -2031,14 +2130,14 @@ int pair_epilogue(inti_ctx* ctx, const PairLaunch& L, const inti_csr* corr, cons
   }
   if (L.precision == INTI_FP32C) {
     if (cplx)
-      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<float4, true>, e);
+      launch_pdl(ctx->stream, es.blocks(L.m), es.threads(), es.smem(), &pair_epilogue_kernel<float4, true>, e, es.nodes);
     else
-      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<float2, false>, e);
+      launch_pdl(ctx->stream, es.blocks(L.m), es.threads(), es.smem(), &pair_epilogue_kernel<float2, false>, e, es.nodes);
   } else {
     if (cplx)
-      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double2, true>, e);
+      launch_pdl(ctx->stream, es.blocks(L.m), es.threads(), es.smem(), &pair_epilogue_kernel<double2, true>, e, es.nodes);
     else
-      launch_pdl(ctx->stream, gb, tb, 0, &pair_epilogue_kernel<double, false>, e);
+      launch_pdl(ctx->stream, es.blocks(L.m), es.threads(), es.smem(), &pair_epilogue_kernel<double, false>, e, es.nodes);
   }
   INTI_CUDA(cudaGetLastError());
   ctx->launches += 1;
@@ -2219,7 +2318,7 @@ int apply_noalloc(int pde, int kind, int dim, double k, int precision, int64_t m
                                 " MiB scratch of inti_apply_noalloc: needs " +
                                 std::to_string(packed_bytes + pbytes) + " bytes (use inti_op_apply)");
   // source chunks: enough CTAs for ~2 waves, bounded by the scratch and the tiles
-  const int64_t blocks = (m + kBlock * kTPT - 1) / (kBlock * kTPT);
+  const int64_t blocks = (m + fwd_rows(precision, kTPT) - 1) / fwd_rows(precision, kTPT);
   int64_t split = std::max<int64_t>(1, (2LL * D.num_sms * 4 + blocks - 1) / blocks);
   split = std::min<int64_t>({split, n_tiles, 64, (int64_t)((room - packed_bytes) / pbytes)});
   const int64_t tps = (n_tiles + split - 1) / split;
@@ -2275,18 +2374,18 @@ int apply_noalloc(int pde, int kind, int dim, double k, int precision, int64_t m
   e.bi = beta ? beta[1] : 0.0;
   e.beta_zero = (e.br == 0.0 && e.bi == 0.0);
   e.err = flag;
-  const unsigned gb = (unsigned)((m + 255) / 256);
+  const EpiShape es = epi_shape((int)split);
   const bool cplx = pde == HELMHOLTZ;
   if (precision == INTI_FP32C) {
     if (cplx)
-      pair_epilogue_kernel<float4, true><<<gb, 256, 0, stream>>>(e);
+      pair_epilogue_kernel<float4, true><<<es.blocks(m), es.threads(), es.smem(), stream>>>(e, es.nodes);
     else
-      pair_epilogue_kernel<float2, false><<<gb, 256, 0, stream>>>(e);
+      pair_epilogue_kernel<float2, false><<<es.blocks(m), es.threads(), es.smem(), stream>>>(e, es.nodes);
   } else {
     if (cplx)
-      pair_epilogue_kernel<double2, true><<<gb, 256, 0, stream>>>(e);
+      pair_epilogue_kernel<double2, true><<<es.blocks(m), es.threads(), es.smem(), stream>>>(e, es.nodes);
     else
-      pair_epilogue_kernel<double, false><<<gb, 256, 0, stream>>>(e);
+      pair_epilogue_kernel<double, false><<<es.blocks(m), es.threads(), es.smem(), stream>>>(e, es.nodes);
   }
   INTI_CUDA(cudaGetLastError());
   if (synchronize) {
