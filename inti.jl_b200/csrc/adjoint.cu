@@ -29,17 +29,31 @@ namespace inti {
 
 constexpr int kAdjBlock = 128;
 constexpr int kAdjTile = 128;
-constexpr int kAdjSpt = 2;  // sources per thread: each staged target serves two pairs
+constexpr int kAdjSpt = 2;     // sources per thread: each staged target serves two pairs
+constexpr int kAdjSlices = 4;  // the warps of a CTA: the same sources, a quarter of the targets each
+constexpr int kAdjRows = kAdjBlock / kAdjSlices * kAdjSpt;  // sources per CTA
 
+// One CTA: 64 sources (two per lane), a chunk of the targets staged 128 at a
+// time, each warp a quarter of a stage; the warps' sums are added in a fixed
+// order.  Bound by the FP64 pipe (26 operations per pair for DL in 3D, 79% of
+// it at 51,894 sources x 4,096 targets); with one warp per source block and a
+// thread per source in the reduction, few sources or targets left SMs idle.
+// Back to back, DL in 3D: 51,894 x 4,096 396 -> 381 us, x 1,000 119 -> 102,
+// 12,150 x 4,096 122 -> 101, 3,456 x 1,000 28 -> 16.5; SL 51,894 x 4,096
+// 315 -> 279.  One source per lane 400, three 385; 96 and 80 registers (the
+// compiler's choice without a bound on the CTAs per SM, and six) 401 and 405.
 // partial layout per (split, source): [s, a_0..a_{D-1}, b_0..b_{D-1}, pad]
 template <int KIND, int DIM, int SPT>
-__global__ void __launch_bounds__(kAdjBlock) adjoint_sources(
+__global__ void __launch_bounds__(kAdjBlock, 1) adjoint_sources(
     int64_t m, int64_t n, const double* __restrict__ tx, const double* __restrict__ g,
-    const double* __restrict__ sx, const double* __restrict__ sn, int tiles_per_split,
+    const double* __restrict__ sx, const double* __restrict__ sn, int64_t per_split,
     double* __restrict__ partial) {
-  constexpr int W = 2 * DIM + 2;
-  __shared__ double stx[kAdjTile * DIM], sg[kAdjTile];
-  const int64_t j0 = blockIdx.x * (int64_t)(kAdjBlock * SPT) + threadIdx.x;
+  constexpr int W = 2 * DIM + 2, NV = KIND == DL ? 2 * DIM + 1 : DIM + 1, L = kAdjBlock / kAdjSlices;
+  constexpr int R = DIM == 3 ? 4 : 3;  // staged target: coordinates, cotangent
+  __shared__ __align__(16) double st[kAdjTile * R];
+  __shared__ double red[kAdjSlices - 1][SPT][NV][L];
+  const int lane = threadIdx.x % L, slice = threadIdx.x / L;
+  const int64_t j0 = blockIdx.x * (int64_t)(L * SPT) + lane;
   double y[SPT][DIM], ny[SPT][DIM];
   // DL: the source's own normal factors out of two sums, accumulated as
   // scalars and applied at the end: s = n_y . a, and b = P*h - n_y*G with
@@ -47,7 +61,7 @@ __global__ void __launch_bounds__(kAdjBlock) adjoint_sources(
   double s[SPT], G[SPT], a[SPT][DIM], b[SPT][DIM];
 #pragma unroll
   for (int u = 0; u < SPT; ++u) {
-    const int64_t jj = min(j0 + u * kAdjBlock, n - 1);
+    const int64_t jj = min(j0 + u * L, n - 1);
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
       y[u][c] = sx[DIM * jj + c];
@@ -56,25 +70,22 @@ __global__ void __launch_bounds__(kAdjBlock) adjoint_sources(
     }
     s[u] = G[u] = 0.0;
   }
-  const int64_t ntile = (m + kAdjTile - 1) / kAdjTile;
-  const int64_t t0 = (int64_t)blockIdx.y * tiles_per_split;
-  const int64_t t1 = min(ntile, t0 + tiles_per_split);
-  for (int64_t t = t0; t < t1; ++t) {
+  const int64_t t0 = (int64_t)blockIdx.y * per_split, t1 = min(m, t0 + per_split);
+  for (int64_t t = t0; t < t1; t += kAdjTile) {
+    const int cnt = (int)min((int64_t)kAdjTile, t1 - t);
     __syncthreads();
-    for (int q = threadIdx.x; q < kAdjTile; q += kAdjBlock) {
-      const int64_t i = t * kAdjTile + q;
-      const bool in = i < m;
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) stx[q * DIM + c] = in ? tx[DIM * i + c] : 0.0;
-      sg[q] = in ? g[i] : 0.0;
+    for (int q = threadIdx.x; q < cnt * R; q += kAdjBlock) {
+      const int i = q / R, c = q - i * R;
+      st[q] = c < DIM ? tx[DIM * (t + i) + c] : g[t + i];
     }
     __syncthreads();
+    const int share = (cnt + kAdjSlices - 1) / kAdjSlices, q1 = min(cnt, (slice + 1) * share);
 #pragma unroll 2
-    for (int q = 0; q < kAdjTile; ++q) {
+    for (int q = slice * share; q < q1; ++q) {
       double xt[DIM];
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) xt[c] = stx[q * DIM + c];
-      const double gi = sg[q];
+      for (int c = 0; c < DIM; ++c) xt[c] = st[q * R + c];
+      const double gi = st[q * R + DIM];
 #pragma unroll
       for (int u = 0; u < SPT; ++u) {
         double r[DIM];
@@ -127,6 +138,24 @@ __global__ void __launch_bounds__(kAdjBlock) adjoint_sources(
       }
     }
   }
+  // the slices' sums, in a fixed order
+  auto value = [&](int u, int c) -> double& {
+    return c < DIM ? b[u][c] : KIND == SL ? s[u] : c < 2 * DIM ? a[u][c - DIM] : G[u];
+  };
+  if (slice > 0) {
+#pragma unroll
+    for (int u = 0; u < SPT; ++u)
+#pragma unroll
+      for (int c = 0; c < NV; ++c) red[slice - 1][u][c][lane] = value(u, c);
+  }
+  __syncthreads();
+  if (slice > 0) return;
+#pragma unroll
+  for (int u = 0; u < SPT; ++u)
+#pragma unroll
+    for (int c = 0; c < NV; ++c)
+#pragma unroll
+      for (int q = 0; q < kAdjSlices - 1; ++q) value(u, c) += red[q][u][c][lane];
 #pragma unroll
   for (int u = 0; u < SPT; ++u) {
     if (KIND == DL) {
@@ -137,7 +166,7 @@ __global__ void __launch_bounds__(kAdjBlock) adjoint_sources(
 #pragma unroll
       for (int c = 0; c < DIM; ++c) b[u][c] = fma(P, b[u][c], -G[u] * ny[u][c]);
     }
-    const int64_t j = j0 + u * kAdjBlock;
+    const int64_t j = j0 + u * L;
     if (j < n) {
       double* o = partial + ((int64_t)blockIdx.y * n + j) * W;
       o[0] = s[u];
@@ -150,33 +179,32 @@ __global__ void __launch_bounds__(kAdjBlock) adjoint_sources(
   }
 }
 
+// One thread per value of a source: its chunks' sums and the outputs that
+// they give.
 template <int KIND, int DIM>
 __global__ void adjoint_reduce(int64_t n, int split, const double* __restrict__ partial,
                                const double* __restrict__ w, const double* __restrict__ sigma,
                                double* dsigma, double* dcoords, double* dnormals, double* dweights) {
   constexpr int W = 2 * DIM + 2;
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  double acc[W - 1];
-#pragma unroll
-  for (int c = 0; c < W - 1; ++c) acc[c] = 0.0;
-  for (int s = 0; s < split; ++s) {
-    const double* p = partial + ((int64_t)s * n + j) * W;
-#pragma unroll
-    for (int c = 0; c < W - 1; ++c) acc[c] += p[c];
-  }
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, j = t / W;
+  const int c = (int)(t - j * W);
+  if (j >= n || c == W - 1) return;  // the last value is padding
+  double acc = 0.0;
+#pragma unroll 4
+  for (int s = 0; s < split; ++s) acc += partial[(int64_t)s * n * W + t];
   const double c0 = DIM == 3 ? 1.0 / (4 * kPi) : 1.0 / (2 * kPi);
-  // SL 2D value term is log(d^2) = 2 log(d): K = -log(d)/(2 pi) = -log(d^2)/(4 pi)
-  const double cs = (DIM == 2 && KIND == SL) ? -1.0 / (4 * kPi) : c0;
-  const double sv = cs * acc[0];
-  const double wj = w[j], sj = sigma[j];
-  if (dsigma) dsigma[j] = wj * sv;
-  if (dweights) dweights[j] = sj * sv;
-  const double ws = wj * sj * c0;
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) {
-    if (dnormals) dnormals[DIM * j + c] = KIND == DL ? ws * acc[1 + c] : 0.0;
-    if (dcoords) dcoords[DIM * j + c] = ws * acc[1 + DIM + c];
+  if (c == 0) {
+    // SL 2D value term is log(d^2) = 2 log(d): K = -log(d)/(2 pi) = -log(d^2)/(4 pi)
+    const double sv = ((DIM == 2 && KIND == SL) ? -1.0 / (4 * kPi) : c0) * acc;
+    if (dsigma) dsigma[j] = w[j] * sv;
+    if (dweights) dweights[j] = sigma[j] * sv;
+    return;
+  }
+  const double ws = w[j] * sigma[j] * c0;
+  if (c <= DIM) {
+    if (dnormals) dnormals[DIM * j + c - 1] = KIND == DL ? ws * acc : 0.0;
+  } else if (dcoords) {
+    dcoords[DIM * j + c - 1 - DIM] = ws * acc;
   }
 }
 
@@ -205,12 +233,15 @@ void grad_sources(inti_op* op, const double* g, const double* sigma, double* dsi
     if (dnormals) { o_n.ensure(sizeof(double) * dim * n); DN = o_n.as<double>(); }
     if (dweights) { o_w.ensure(sizeof(double) * n); DW = o_w.as<double>(); }
   }
-  const int64_t blocks = (n + kAdjBlock * kAdjSpt - 1) / (kAdjBlock * kAdjSpt);
-  const int64_t ntile = (m + kAdjTile - 1) / kAdjTile;
-  const int64_t want = (int64_t)ctx->num_sms * 8;
-  int split = (int)std::max<int64_t>(1, std::min<int64_t>(ntile, (want + blocks - 1) / blocks));
-  const int tps = (int)((ntile + split - 1) / split);
-  split = (int)((ntile + tps - 1) / tps);
+  const int64_t blocks = (n + kAdjRows - 1) / kAdjRows;
+  // 12 CTAs per SM, but chunks of 64 targets and more: below that the partial
+  // sums cost more than the SMs gain (3,456 sources x 1,000 targets: chunks of
+  // 64 targets 16.5 us, with a limit of 32 and 16 targets 2 and 3 to 5 us more;
+  // 51,894 x 4,096: 381 us at 12 per SM, 389 at 20, 383 at 40)
+  const int64_t want = (int64_t)ctx->num_sms * 12 / blocks;
+  const int64_t chunks = std::max<int64_t>(1, std::min((m + 63) / 64, want));
+  const int64_t per = ((m + chunks - 1) / chunks + kAdjSlices - 1) / kAdjSlices * kAdjSlices;
+  const int split = (int)((m + per - 1) / per);
   const int W = 2 * dim + 2;
   op->gpartial.ensure(sizeof(double) * (size_t)split * n * W);
   double* part = op->gpartial.as<double>();
@@ -224,9 +255,9 @@ void grad_sources(inti_op* op, const double* g, const double* sigma, double* dsi
     {
       ProfScope pa(ctx, "adjoint");
       adjoint_sources<K, D, kAdjSpt><<<dim3((unsigned)blocks, (unsigned)split), kAdjBlock, 0, ctx->stream>>>(
-          m, n, TX, G, SX, SN, tps, part);
+          m, n, TX, G, SX, SN, per, part);
     }
-    adjoint_reduce<K, D><<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(
+    adjoint_reduce<K, D><<<(unsigned)((n * W + 255) / 256), 256, 0, ctx->stream>>>(
         n, split, part, SW, SG, DS, DC, DN, DW);
     ctx->launches += 2;
   };

@@ -7,6 +7,7 @@ its FP64 sums: at most about n eps of the sum of magnitudes (3e-12 at the
 norm as for every FP64 product."""
 import numpy as np
 import pytest
+import torch
 
 import inti_b200 as inti
 import oracle as O
@@ -58,3 +59,29 @@ def test_launch_shapes(tiled, case, m, n):
         y = A.mul(y0.copy(), x, alpha=alpha, beta=beta)
         assert relerr(y[rows], ref) < 1e-12, kname
         assert np.array_equal(A.mul(y0.copy(), x, alpha=alpha, beta=beta), y)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("m,n", [(1, 1), (3, 65), (64, 63), (130, 64), (513, 129), (4100, 300)])
+def test_source_gradients(tiled, dim, m, n):
+    """Source gradients at the edges of their blocks (64 sources, 128 staged
+    targets, four shares of a stage) against automatic differentiation of the
+    dense product; the sums are over at most 4,100 targets."""
+    src, tgt = _points(n, dim, 3 + m), inti.points(_points(m, dim, 5 + n).coords)
+    g, sig = density(m, False, 2), density(n, False, 4)
+    for K in (inti.SingleLayerKernel, inti.DoubleLayerKernel):
+        A = inti.GpuOperator(K(inti.Laplace(dim=dim)), tgt, src, None, "fp64", tiled)
+        got = A.grad_sources(g, sig)
+        s, y, ny, w = (torch.tensor(np.array(v), requires_grad=True)
+                       for v in (sig, src.coords, src.normals, src.weights))
+        r = torch.tensor(np.array(tgt.coords))[:, None, :] - y[None]
+        d2 = (r * r).sum(-1)
+        if K is inti.SingleLayerKernel:
+            M = -torch.log(d2) / (4 * np.pi) if dim == 2 else d2 ** -0.5 / (4 * np.pi)
+        else:
+            rn = (r * ny[None]).sum(-1)
+            M = rn / (2 * np.pi * d2) if dim == 2 else rn * d2 ** -1.5 / (4 * np.pi)
+        (torch.tensor(g) @ (M @ (w * s))).backward()
+        for name, v in (("sigma", s), ("coords", y), ("normals", ny), ("weights", w)):
+            want = np.zeros(tuple(v.shape)) if v.grad is None else v.grad.numpy()
+            assert np.linalg.norm(got[name] - want) <= 1e-12 * np.linalg.norm(want), (K, name)
