@@ -382,8 +382,31 @@ struct FwdArgs {
   int* err;
 };
 
+// CTAs per SM that the FP64 pair kernels ask the compiler for: one lets it
+// take the registers that keep more pairs in flight, zero leaves its own
+// choice (more CTAs).  Which is faster depends on the arithmetic of a pair,
+// so it is measured per kernel.  Symmetric form, 19,200 nodes, zero -> as
+// below, us: Laplace 3D SL 219 -> 200, HS 406 -> 391; 2D ADL 245 -> 234,
+// HS 301 -> 278; Helmholtz SL 522 -> 488, ADL 711 -> 698, HS 806 -> 786, CF
+// 857 -> 854 (two targets per thread 899 -> 854).  Slower with one, so left at
+// zero: Laplace 3D DL 318 (347), ADL 342 (369), CF 344 (351), 2D SL 662
+// (683), Helmholtz DL 725 (741).  One-sided, 3,888 targets x 12,288 sources:
+// Laplace 3D SL 54 -> 49, HS 100 -> 96, 2D DL 47 -> 43, ADL 49 -> 47, HS 71 ->
+// 67, Helmholtz SL 124 -> 116, DL 155 -> 153, ADL 153 -> 144.
+template <int PDE, int KIND, int DIM, class R>
+constexpr int fwd_min_ctas() {
+  if (std::is_same<R, float>::value || KIND == CF) return 0;
+  return PDE == HELMHOLTZ || (DIM == 3 ? KIND == SL || KIND == HS : KIND != SL) ? 1 : 0;
+}
+template <int PDE, int KIND, int DIM, class R>
+constexpr int symm_min_ctas() {
+  if (std::is_same<R, float>::value) return 0;
+  if (PDE == HELMHOLTZ) return KIND == DL ? 0 : KIND == CF ? 3 : 1;
+  return fwd_min_ctas<PDE, KIND, DIM, R>();
+}
+
 template <int PDE, int KIND, int DIM, class R, int TILE, int TPT = kTPT>
-__global__ void __launch_bounds__(kBlock) pair_forward(FwdArgs a) {
+__global__ void __launch_bounds__(kBlock, (fwd_min_ctas<PDE, KIND, DIM, R>())) pair_forward(FwdArgs a) {
   using RC = Rec<PDE, KIND, DIM, R>;
   constexpr bool CPLX = RC::cplx;
   using P = typename PartialT<R, CPLX>::T;
@@ -1037,7 +1060,7 @@ __device__ __forceinline__ void put_partial(float4* p, float r, float i) { *p = 
 // tile length is a constant: made a variable it cost 4% at 62,208 nodes, and
 // up to 38 registers.
 template <int PDE, int KIND, int DIM, class R, int TILE, int TPT, bool SUB>
-__global__ void __launch_bounds__(kBlock) pair_symm(SymArgs a) {
+__global__ void __launch_bounds__(kBlock, (symm_min_ctas<PDE, KIND, DIM, R>())) pair_symm(SymArgs a) {
   using RC = SymRec<PDE, KIND, DIM, R>;
   constexpr bool CPLX = RC::cplx;
   using P = typename PartialT<R, CPLX>::T;
