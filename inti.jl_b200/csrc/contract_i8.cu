@@ -119,17 +119,21 @@ struct FxConst {
 };
 
 // e^{i d k}, kT = k FX_TAB / (2 pi): the table value of the nearest multiple
-// of delta = 2 pi / FX_TAB times the Taylor series of the rest (|f delta| <=
-// pi/128: sin to r^7, cos to r^6, truncation below 4e-18).
+// of delta = 2 pi / FX_TAB times series of the rest (|r| = |f delta| <= H =
+// pi/128): cos to r^6 (truncation below 4e-18), sin to r^5 with the r^7 term
+// economised, x^7 ~ (112 x^5 - 56 x^3 + 7 x)/64 for x = r/H, which leaves
+// H^7/5040/64 = 1.7e-17.
 __device__ __forceinline__ void fx_expi(double d, double kT, const double2* __restrict__ tab, double& c, double& s) {
   constexpr double D = 2.0 * kPi / FX_TAB, D2 = D * D;
   constexpr double C2 = -D2 / 2, C4 = D2 * D2 / 24, C6 = -D2 * D2 * D2 / 720;
-  constexpr double S3 = -D2 * D / 6, S5 = D2 * D2 * D / 120, S7 = -D2 * D2 * D2 * D / 5040;
+  constexpr double H2 = D2 / 4;
+  constexpr double S1 = D * (1.0 - 7 * H2 * H2 * H2 / (64 * 5040.0)), S3 = D2 * D * (-1.0 / 6 + 56 * H2 * H2 / (64 * 5040.0)),
+                   S5 = D2 * D2 * D * (1.0 / 120 - 112 * H2 / (64 * 5040.0));
   const double t = fma(d, kT, kRoundShift);
   const double f = fma(d, kT, -(t - kRoundShift));
   const double f2 = f * f;
   const double cp = fma(f2, fma(f2, fma(f2, C6, C4), C2), 1.0);
-  const double sp = f * fma(f2, fma(f2, fma(f2, S7, S5), S3), D);
+  const double sp = f * fma(f2, fma(f2, S5, S3), S1);
   const double2 e = tab[(__double2loint(t) & (FX_TAB - 1)) * FX_REP];
   c = fma(cp, e.x, -sp * e.y);
   s = fma(sp, e.x, cp * e.y);
@@ -211,10 +215,12 @@ __device__ __forceinline__ void fx_values(const double (&x)[3], const double (&n
       v[0] = fma(cp, wr, -sp * wi);
       v[1] = fma(cp, wi, sp * wr);
     } else if constexpr (KIND == FX_THETA) {
-      const double pri = pr * ri;
+      // D = (r.n)/d^2 (1 - ikd) S
+      const double pri = pr * ri, kd = c.k * d, q = rny * id2;
       v[0] = pri * cs;
       v[1] = pri * sn;
-      layer(pr * rny, v[2], v[3]);
+      v[2] = q * fma(kd, v[1], v[0]);
+      v[3] = q * fma(-kd, v[0], v[1]);
     } else {
       layer(-rnx, v[0], v[1]);
       hyper(v[2], v[3]);
@@ -424,7 +430,7 @@ template <int PDE, int KIND, int CL>
 __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
   using SH = FxShape<PDE, KIND>;
   extern __shared__ __align__(1024) unsigned char sm[];
-  __shared__ __align__(8) uint64_t fullS[FX_NS], fullB[2], aFull[2], aPeer[2], mmaDone[FX_ND], drainBar;
+  __shared__ __align__(8) uint64_t fullS[FX_NS], fullB[2], aReady[2], aFull[2], aPeer[2], mmaDone[FX_ND], drainBar;
   __shared__ uint32_t tmem_base_sh;
   __shared__ int item_sh, fail_sh;
   if (*a.flag) return;  // densities or kernel values out of range: the FP64 kernels run
@@ -439,6 +445,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
     for (int q = 0; q < FX_ND; ++q) mbar_init(&mmaDone[q], CL);
     for (int q = 0; q < 2; ++q) {
       mbar_init(&fullB[q], 1);
+      mbar_init(&aReady[q], FX_GEN);
       mbar_init(&aFull[q], FX_GEN);
       mbar_init(&aPeer[q], 1);
     }
@@ -488,7 +495,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
         for (uint32_t t = 0; t < T; ++t) {
           const uint32_t gg = g + t, bb = gg & 1;
           ok = mbar_wait_bounded(&aFull[bb], (gg >> 1) & 1) && mbar_wait_bounded(&fullB[bb], (gg >> 1) & 1) &&
-               (CL == 1 || fx_wait<CL>(&aPeer[bb], (gg >> 1) & 1));
+               (CL == 1 || fx_wait<CL>(&aPeer[bb], (gg >> 1) & 1)) &&
+               (t + 1 == T || mbar_wait_bounded(&aReady[bb ^ 1], ((gg + 1) >> 1) & 1));
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
@@ -585,8 +593,6 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
         for (uint32_t t = 0; t < T; ++t) {
           const uint32_t gg = g + t, sb = gg % FX_NS;
           bool w = mbar_wait_bounded(&fullS[sb], (gg / FX_NS) & 1);
-          // A buffer gg & 1 was last read by MMA group gg-2
-          if (w && t >= 2) w = fx_wait<CL>(&mmaDone[(gg - 2) % FX_ND], ((gg - 2) / FX_ND) & 1);
           if (!__all_sync(0xffffffffu, w)) {
             ok = false;
             break;
@@ -598,29 +604,44 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
           unsigned char* A = sm + (gg & 1) * FX_A_BYTES + chunk * (FX_M * 16) + r * 16;
           // Groups of four sources, NA words each.  The octets of a warp take
           // them in rotated order, so that their stores of NA words at a
-          // stride of 16 bytes fall on distinct banks; storing each group at
-          // once keeps the registers for evaluations in flight.
+          // stride of 16 bytes fall on distinct banks.
           constexpr int G = SH::JT / 4, GQ = G / CL;  // of a chunk; of this thread
           static_assert(GQ >= 1, "a group per thread");
-          const int g0 = CL == 2 ? (quarter & 1) * GQ : 0;
+          const int g0 = (CL == 2 ? (quarter & 1) * GQ : 0) + (lane >> 3);
+          uint2 dg[GQ][SH::NA][4];
 #pragma unroll
           for (int q = 0; q < GQ; ++q) {
-            const int grp = (q + g0 + (lane >> 3)) & (G - 1);
-            const double* Sg = S + grp * (4 * FX_REC);
-            uint2 dg[SH::NA][4];
-            {
-              double v[4][SH::NA];
+            const double* Sg = S + ((q + g0) & (G - 1)) * (4 * FX_REC);
+            double v[4][SH::NA];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) fx_values<PDE, KIND>(x, nx, scale, Sg + e * FX_REC, a.c, tab, v[e]);
+            for (int e = 0; e < 4; ++e) fx_values<PDE, KIND>(x, nx, scale, Sg + e * FX_REC, a.c, tab, v[e]);
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
+            for (int e = 0; e < 4; ++e)
 #pragma unroll
-                for (int n = 0; n < SH::NA; ++n) dg[n][e] = fx_bytes(v[e][n]);
-            }
+              for (int n = 0; n < SH::NA; ++n) dg[q][n][e] = fx_bytes(v[e][n]);
+          }
+          // FP64 work of the stage done: the MMAs of the one before may run,
+          // beside the packing of this one
+#pragma unroll
+          for (int q = 0; q < GQ; ++q)
+#pragma unroll
+            for (int n = 0; n < SH::NA; ++n)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) asm volatile("" : "+r"(dg[q][n][e].x), "+r"(dg[q][n][e].y));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&aReady[gg & 1]);
+          // A buffer gg & 1 was last read by MMA group gg-2
+          if (t >= 2) w = fx_wait<CL>(&mmaDone[(gg - 2) % FX_ND], ((gg - 2) / FX_ND) & 1);
+          if (!__all_sync(0xffffffffu, w)) {
+            ok = false;
+            break;
+          }
+#pragma unroll
+          for (int q = 0; q < GQ; ++q) {
             uint32_t wd[SH::NA][FX_D];
 #pragma unroll
-            for (int n = 0; n < SH::NA; ++n) fx_pack4(dg[n], wd[n]);
-            unsigned char* Ag = A + grp * (4 * SH::NA);
+            for (int n = 0; n < SH::NA; ++n) fx_pack4(dg[q][n], wd[n]);
+            unsigned char* Ag = A + ((q + g0) & (G - 1)) * (4 * SH::NA);
 #pragma unroll
             for (int p = 0; p < FX_D; ++p) {
               if constexpr (SH::NA == 1)
