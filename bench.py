@@ -25,7 +25,7 @@ gmres   (extra key) time to ||b - Lx|| <= 1e-10 ||b|| for the 3D Laplace
 
 Other workloads (--workload): c2_dl, c2_adl, c2_hs, c3_dl_fp64, c3_dl_fp32c, c3_sl_fp64, c1
 (single operators); c4 (batched surfaces x 64 right-hand sides, TF32 tensor
-cores and FP64 MMA, --nsurf surfaces); c5 (adjoint); csr (correction SpMV
+cores and FP64, --nsurf surfaces); c5 (adjoint); csr (correction SpMV
 bandwidth); dim_c2, dim_c3 (GPU construction of the DIM correction).
 
 --impl reference times the reference's CPU algorithm for the same step
@@ -435,8 +435,8 @@ def bench_dim(args, ctx, peaks, torch) -> dict:
     """GPU construction of the on-surface DIM correction (bdim_correction,
     src/bdim.jl:50-196) of the C2 operator (Helmholtz k = 10, P2 sphere,
     N = 62,208, ns = 18) or the C3 operator (Laplace, ellipsoid, N = 200,934,
-    ns = 27): traces, the Θ pair product over all node pairs on the FP64 MMA
-    path, per-element least squares, CSR assembly.  value = seconds per
+    ns = 27): traces, the Θ pair product over all node pairs as fixed-point
+    products on the INT8 tensor path, per-element least squares, CSR assembly.  value = seconds per
     construction (wall clock around the call, synchronised)."""
     import inti_b200 as inti
 
@@ -469,7 +469,9 @@ def bench_dim(args, ctx, peaks, torch) -> dict:
             "vs_baseline": None, "dtype": "c128" if isinstance(op, inti.Helmholtz) else "f64", "data": "synthetic",
             "config": {"workload": work, "n": n, "nnz_per_row": dS.nnz // n, "l2": "inputs (traces, partials) "
                        "larger than L2 are not flushed: each step rebuilds everything"},
-            "roofline": {"bound": "fp64", "kernel": "dim_theta_mma + dim_theta_reduce", "kernel_ms": theta_ms,
+            "roofline": {"bound": "fp64", "kernel": "fx_contract_kernel with its plan and reductions", "kernel_ms": theta_ms,
+                         "form": "the columns are multiplied as exact 8-bit digit products on the INT8 tensor path; "
+                                 "flops are counted as FP64, so frac can pass 1",
                          "achieved": achieved, "peak": fp64, "unit": "TFLOP/s", "frac": achieved / fp64,
                          "flops_per_pair": flops_pair, "traffic": None,
                          "peak_source": "FP64 FMA throughput measured in this run (inti_measure_peaks), of measured"},
@@ -1016,7 +1018,7 @@ def main() -> None:
                 "flops_per_pair": FLOPS_PER_PAIR[fkey],
                 "form": ("symmetric: one kernel evaluation per unordered pair serves both products; achieved "
                          "counts the metric's M*N ordered pairs" if sym else
-                         "single launch: one cluster kernel per product builds the source records, sums the pairs, adds the "
+                         "single launch: one kernel per product builds the source records, sums the pairs, adds the "
                          "correction rows and applies alpha/beta; kernel_ms is the step's own CUDA-event time "
                          "(the step is that one launch)" if small else
                          "one-sided"),

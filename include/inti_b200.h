@@ -166,11 +166,11 @@ int inti_op_info(const inti_op* op, int64_t* m, int64_t* n, int* dtype);
 /* Y = alpha*(A*X + C*X) + beta*Y for nrhs columns (leading dimensions ldx,
  * ldy in elements).  alpha, beta: 2 doubles each (re, im); NULL means 1, 0.
  * beta = 0 does not read Y.  FP64 3D operators (every kernel) apply 8 or
- * more columns in one pass that evaluates each kernel value once
- * per 64 columns (16 complex / 32 real when all columns fit), the pair tile
- * multiplied with the columns on the FP64 MMA path; other operators and
- * fewer columns run one pair product per column.  Results agree to rounding
- * (the summation order differs). */
+ * more columns in one pass that evaluates each kernel value once for up to
+ * 64 columns, multiplied with them as exact fixed-point products on the INT8
+ * tensor path (from 2e6 pairs, outside stream capture) or on the FP64 MMA
+ * path; other operators and fewer columns run one pair product per column.
+ * Results agree to rounding (the summation order differs). */
 int inti_op_apply(inti_op* op, const double* x, int64_t ldx, double* y, int64_t ldy,
                   int32_t nrhs, const double* alpha, const double* beta, int on_device);
 /* Y = alpha*(A^T*X + C^T*X) + beta*Y: the transpose (not conjugate) apply,

@@ -8,7 +8,9 @@
 // on-the-fly Nystrom operator of surface s.  Densities are column-major
 // (node, rhs) over the concatenated nodes.
 //
-// Two arithmetic forms of the pair product:
+// Arithmetic forms of the pair product:
+//  * FP64 from 2e6 pairs: exact fixed-point products on the INT8 tensor path
+//    (contract_i8.cu), with the next form standing by.
 //  * FP64 (mrhs_mma): a CTA owns 64 targets and 64 right-hand sides; per
 //    source tile the CUDA cores evaluate each kernel value once into shared
 //    memory and the warps multiply that tile with the staged densities on

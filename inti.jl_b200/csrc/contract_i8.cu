@@ -40,28 +40,31 @@
 //     accumulators: eight diagonals of NC columns, all 512 tensor-memory
 //     columns for NC = 64.  Reading each A digit once per 256 columns keeps
 //     the operand traffic of shared memory below the MMA time.
-// Generation of one stage runs beside the MMAs of the one before (two A
-// buffers), but only its integer, memory and conversion instructions overlap
-// them: on the B200 FP64 FMAs make no progress while INT8 MMAs are in flight
-// (16 warps of independent FMAs next to an MMA loop: 1.5% of their rate
-// alone, and the MMAs at 92% of theirs).  A stage therefore costs about the
-// sum of both: DL with 64 columns 2,333 cycles of MMAs (the full INT8 rate)
-// and 4,250 of generation, of which 2,500 are FP64 issue.  The 32-bit sums
+// Only the integer, memory and conversion instructions of the generators
+// overlap MMAs: on the B200 FP64 FMAs make no progress while INT8 MMAs are in
+// flight (16 warps of independent FMAs next to an MMA loop: 1.5% of their rate
+// alone, and the MMAs at 92% of theirs).  The MMAs of a stage therefore start
+// once the values of the next stage are evaluated (aReady), and its packing
+// and stores run beside them (two A buffers); starting them at once left the
+// evaluation stalled and the packing alone (64 columns 1.92 -> 1.87 ms).  A
+// stage costs about the sum: Theta with 18 complex columns 2,010 cycles of
+// MMAs and stores (1,490 of operand reads), 1,990 of evaluation (1,353 of FP64
+// issue) and 290 of hand-over.  The 32-bit sums
 // hold 127 stages (8 * 255 * 128 * 8,128 < 2^31); then, or at the end of the
 // item, the generators read the diagonals and add them up in FP64.
 //
 // More than 64 real columns go to pairs of CTAs that share the evaluation.
 //
 // Measured (B200, against the FP64 MMA kernels, device time): 64 complex
-// columns of a Helmholtz DL at 13,872 nodes 5.63 -> 1.91 ms (2.48 without
+// columns of a Helmholtz DL at 13,872 nodes 5.63 -> 1.87 ms (2.48 without
 // pairs); eight surfaces of 2,646 .. 21,600 nodes, combined field, 64 columns
-// 26.9 -> 11.4 ms (15.7); the correction of a 43,200-node surface (18 complex
+// 26.9 -> 11.1 ms (15.7); the correction of a 43,200-node surface (18 complex
 // columns) 33.6 -> 16.0 ms.
 //
 // e^{ikd} comes from a 128-entry table in eight copies, one per lane of a
 // quarter-warp, so the gathers never conflict (a shared 1024-entry table
 // costs about 12 wavefronts a warp, and shared memory is as busy here as the
-// FP64 pipe), with one more term in each series.
+// FP64 pipe), with one more term in the cosine.
 //
 // Every wait is bounded, as in mrhs_tc.cu.
 #include <cuda_runtime.h>

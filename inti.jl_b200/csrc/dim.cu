@@ -8,7 +8,8 @@
 //  2. traces g0[j,k] = G(y_j, xs_k), g1[j,k] = ADL(y_j, xs_k) (bdim.jl:94-103).
 //  3. Theta = mu*B(x) + S*g1 - D*g0 (bdim.jl:104-118): a multi-right-hand-side
 //     pair product over all node pairs, S and D being the uncorrected Nystrom
-//     operators (entries K*w), evaluated on the fly and never stored.
+//     operators (entries K*w), evaluated on the fly and never stored (large
+//     3D surfaces on the INT8 tensor path, contract_i8.cu).
 //  4. per element: Householder QR of M^T = [g0[el,:]; g1[el,:]]^T (ns x 2nq)
 //     and least squares for each of the element's nq nodes (bdim.jl:154-185);
 //     one warp per element, lane l owning row l.
