@@ -155,6 +155,7 @@ __global__ void axpby(int64_t n, double ar, double ai, const double* x, double b
 
 constexpr int kArnoldiThreads = 1024;
 constexpr int kArnoldiBatch = 4;
+constexpr int kSmallMaxRestart = 1000;
 
 // Device state of a small-system Arnoldi cycle: the rotated Hessenberg
 // matrix R ((restart+1) x restart, column-major), the Givens rotations, the
@@ -433,7 +434,7 @@ struct Solver {
     return std::sqrt(std::max(v.x, 0.0));
   }
 
-  bool small_cycle(int restart) const { return n <= ctx->krylov_small && restart <= 1000; }
+  bool small_cycle(int restart) const { return n <= ctx->krylov_small && restart <= kSmallMaxRestart; }
 
   // One Arnoldi cycle of a small system with v_0 = V[0] normalised and
   // g = (beta, 0, ...): steps of one operator application and one
@@ -462,7 +463,10 @@ struct Solver {
     INTI_CUDA(cudaMemcpyAsync(st.g, &g0, sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
     const size_t smem = sizeof(double2) * 6 * (restart + 1);
     const auto step = C ? &arnoldi_small_step<true> : &arnoldi_small_step<false>;
-    INTI_CUDA(cudaFuncSetAttribute(step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The limit belongs to the kernel on the device, whose other contexts may
+    // be solving with other restarts: always the largest restart's.
+    INTI_CUDA(cudaFuncSetAttribute(step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(sizeof(double2) * 6 * (kSmallMaxRestart + 1))));
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = n > 4096 ? 8 : n > 2048 ? 4 : n > 1024 ? 2 : 1;
