@@ -928,40 +928,42 @@ constexpr int kMaxRun = 8;  // stages per warp
 template <bool CPLX>
 __global__ void fx_colmax(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
                           const double* __restrict__ x, int64_t ldx, int ncol, unsigned long long* colmax) {
-  const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, c = blockIdx.y;
+  const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int s0 = run * kMaxRun, s1 = min(nstages, s0 + kMaxRun);
-  unsigned long long best = 0;
-  int surf = -1;
-  auto flush = [&]() {
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-      best = other > best ? other : best;
-    }
-    if (lane == 0 && surf >= 0) atomicMax(&colmax[(int64_t)surf * ncol + c], best);
-    best = 0;
-  };
-  for (int s = s0; s < s1; ++s) {
-    const FxStage st = stages[s];
-    if (st.surf != surf) {
-      flush();
-      surf = st.surf;
-    }
-    for (int j = lane; j < st.count; j += 32) {
-      const int64_t i = st.src0 + j;
-      const int64_t q = (int64_t)c * ldx + i;
-      double m;
-      if (CPLX) {
-        const double2 v = reinterpret_cast<const double2*>(x)[q];
-        const double re = fabs(w[i] * v.x), im = fabs(w[i] * v.y);
-        m = re > im || re != re ? re : im;
-      } else {
-        m = fabs(w[i] * x[q]);
+  for (int c = blockIdx.y; c < ncol; c += gridDim.y) {  // (a grid dimension holds 65,535)
+    unsigned long long best = 0;
+    int surf = -1;
+    auto flush = [&]() {
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
       }
-      const unsigned long long b = (unsigned long long)__double_as_longlong(m);
-      best = b > best ? b : best;
+      if (lane == 0 && surf >= 0) atomicMax(&colmax[(int64_t)surf * ncol + c], best);
+      best = 0;
+    };
+    for (int s = s0; s < s1; ++s) {
+      const FxStage st = stages[s];
+      if (st.surf != surf) {
+        flush();
+        surf = st.surf;
+      }
+      for (int j = lane; j < st.count; j += 32) {
+        const int64_t i = st.src0 + j;
+        const int64_t q = (int64_t)c * ldx + i;
+        double m;
+        if (CPLX) {
+          const double2 v = reinterpret_cast<const double2*>(x)[q];
+          const double re = fabs(w[i] * v.x), im = fabs(w[i] * v.y);
+          m = re > im || re != re ? re : im;
+        } else {
+          m = fabs(w[i] * x[q]);
+        }
+        const unsigned long long b = (unsigned long long)__double_as_longlong(m);
+        best = b > best ? b : best;
+      }
     }
+    flush();
   }
-  flush();
 }
 
 // Sets the flag when a row or column bound does not fit (one block).
@@ -1450,7 +1452,7 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
   auto by_type = [&](auto cc) {
     constexpr bool C = decltype(cc)::value;
     const int runs = (plan.nstages + kMaxRun - 1) / kMaxRun;
-    fx_colmax<C><<<dim3((runs + 7) / 8, nrhs), 256, 0, ctx->stream>>>(plan.nstages, st, p.weights, x, ldx, nrhs, colmax);
+    fx_colmax<C><<<dim3((runs + 7) / 8, std::min(nrhs, 65535)), 256, 0, ctx->stream>>>(plan.nstages, st, p.weights, x, ldx, nrhs, colmax);
     fx_check<<<1, 256, 0, ctx->stream>>>(plan.nsurf * nrhs, colmax, meta, flag);
     ctx->launches += 2;
     int pass = 0;

@@ -1,0 +1,225 @@
+"""Entry-wise accuracy of multi-column FP64 products whose magnitudes vary
+within a row of the operator or within a density: refined surfaces, targets
+close to a surface, unit vectors, narrow Gaussians, densities on one part of
+a surface.
+
+The reference is the sum in extended precision (64-bit significands) of the
+kernel at the nodes' FP64 coordinates.  An entry's allowance is
+
+    (4 m + 64 + 4 k d) eps sum_j S_ij |w_j x_j|,   eps = 2^-52,
+
+m nonzero densities, S the modulus that the kernel's evaluation works with
+(|n| d for |r.n|: the products in r.n are rounded at that size).  The parts:
+rounding of a kernel value and of w x, under 32 operations of eps/2 each,
+doubled; the phase k d (relative rounding of d and of the product, and the
+table's, under 4 eps k d); the sum of m complex products in any order, at
+most 2 m real ones, each rounded at eps/2 of the sum of moduli, twice for
+m complex densities whose parts are summed apart.
+"""
+import numpy as np
+import pytest
+import torch
+
+import inti_b200 as inti
+
+pytestmark = pytest.mark.gpu
+
+KERNEL = {"SL": inti.SingleLayerKernel, "DL": inti.DoubleLayerKernel, "ADL": inti.AdjointDoubleLayerKernel,
+          "HS": inti.HyperSingularKernel}
+LD = np.longdouble
+EPS = 2.0**-52
+
+
+def graded_sphere(levels=12, cells=5):
+    """The unit sphere as six patches of cells x cells (odd), the middle cell of
+    one refined towards its centre by `levels` halvings, 3 x 3 Gauss nodes."""
+    g, w = np.polynomial.legendre.leggauss(3)
+    h = 2.0 / cells
+    rect = []
+    for face in range(6):
+        for i in range(cells):
+            for j in range(cells):
+                if face == 0 and i == j == cells // 2:
+                    continue
+                rect.append((face, -1 + i * h, -1 + j * h, h))
+    s = h
+    for _ in range(levels):  # the square (-s/2, s/2)^2 without its middle ninth: eight cells
+        for i in range(3):
+            for j in range(3):
+                if not i == j == 1:
+                    rect.append((0, -s / 2 + i * s / 3, -s / 2 + j * s / 3, s / 3))
+        s /= 3
+    rect.append((0, -s / 2, -s / 2, s))
+    X, W = [], []
+    for face, u0, v0, c in rect:
+        u, v = np.meshgrid(u0 + c * (g + 1) / 2, v0 + c * (g + 1) / 2, indexing="ij")
+        u, v, ww = u.ravel(), v.ravel(), (np.outer(w, w) * c * c / 4).ravel()
+        p = np.stack([np.ones(9), np.tan(np.pi / 4 * u), np.tan(np.pi / 4 * v)], 1)
+        r = np.linalg.norm(p, axis=1)
+        jac = (np.pi / 4) ** 2 * (p[:, 1] ** 2 + 1) * (p[:, 2] ** 2 + 1) / r**3
+        p /= r[:, None]
+        sign = 1 if face < 3 else -1
+        X.append(sign * np.roll(p, face % 3, axis=1))
+        W.append(ww * jac)
+    X = np.concatenate(X)
+    return inti.Quadrature(X, X.copy(), np.concatenate(W), 9)
+
+
+def reference(pde, kind, k, tgt, rows, src, X):
+    """(K w X)[rows] in extended precision, and sum S |w x|."""
+    x, y = tgt.coords[rows].astype(LD), src.coords.astype(LD)
+    ny = src.normals.astype(LD)
+    b = src.weights.astype(LD)[:, None] * X.astype(np.clongdouble if pde == "helmholtz" else LD)
+    r = x[:, None, :] - y[None]
+    d2 = (r * r).sum(-1)
+    same = d2 <= LD(1e-28)
+    d = np.sqrt(np.where(same, LD(1), d2))
+    one = LD(1)
+    nx = tgt.normals[rows].astype(LD) if tgt.normals is not None else None
+    rny = (r * ny[None]).sum(-1)
+    lnx = np.sqrt((nx * nx).sum(-1))[:, None] if nx is not None else None
+    lny = np.sqrt((ny * ny).sum(-1))[None]
+    f = one / d + k  # |1/d - ik| at most
+    if kind == "SL":
+        v, S = one / d, one / d
+    elif kind == "DL":
+        v, S = rny / d**2 * (one / d - 1j * LD(k) if k else one / d), f / d * lny
+    else:
+        rnx = (r * nx[:, None]).sum(-1)
+        if kind == "ADL":
+            v, S = -rnx / d**2 * (one / d - 1j * LD(k) if k else one / d), f / d * lnx
+        else:
+            nn = (nx[:, None] * ny[None]).sum(-1)
+            kd = LD(k) * d
+            v = nn / d**2 * (one / d - 1j * LD(k) if k else one / d)
+            v = v + ((kd * kd - 3 + 3j * kd) if k else -3 * one) * rnx * rny / d**5
+            S = (f / d**2 + (kd * kd + 3 * kd + 3) / d**3) * lnx * lny
+    if pde == "helmholtz":
+        v = v * (np.cos(LD(k) * d) + 1j * np.sin(LD(k) * d))
+    c = one / (4 * LD(np.pi).__class__("3.14159265358979323846264338327950288"))
+    v, S = np.where(same, 0, v) * c, np.where(same, 0, S) * c
+    return v @ b, S @ abs(b), float(d.max())
+
+
+def check(A, pde, kind, k, tgt, src, X, rows):
+    Y = A @ X
+    ref, T, dmax = reference(pde, kind, k, tgt, rows, src, X)
+    m = (X != 0).sum(0)[None, :]
+    allow = (4.0 * m + 64 + 4 * k * dmax) * EPS * T
+    err = np.abs(Y[rows] - ref)
+    assert (err <= allow).all(), float((err / np.maximum(allow, LD(1e-300))).max())
+    return Y
+
+
+def waves(q, n, cplx, seed):
+    v = np.random.default_rng(seed).standard_normal((n, 3))
+    p = q.coords @ v.T
+    return np.exp(1j * p) if cplx else np.cos(p + 0.3)
+
+
+def columns(q, family, cplx, seed=1):
+    """(n, 8) densities of a family."""
+    r = np.random.default_rng(seed)
+    n = len(q)
+    W = waves(q, 8, cplx, seed)
+    if family == "smooth":
+        return W
+    if family == "unit":
+        X = np.zeros_like(W)
+        X[np.concatenate([[n - 1, n - 5], r.choice(n, 6, replace=False)]), np.arange(8)] = 1.0
+        return X
+    c = np.concatenate([[n - 1], r.choice(n, 7, replace=False)])
+    d2 = ((q.coords[:, None] - q.coords[None, c]) ** 2).sum(-1)
+    if family == "gauss":
+        return np.exp(-d2 / (2 * 0.05**2)) * W
+    X = W.copy()  # "part": only farther than 0.5 from a node
+    X[d2 < 0.25] = 0.0
+    return X
+
+
+def operator(pde, kind, k, tgt, src, ctx):
+    return inti.GpuOperator(KERNEL[kind](inti.Helmholtz(k=k, dim=3) if k else inti.Laplace(dim=3)), tgt, src, None,
+                            "fp64", ctx)
+
+
+@pytest.mark.parametrize("pde,k", [("laplace", 0.0), ("helmholtz", 4.0)])
+@pytest.mark.parametrize("kind", ["SL", "DL", "ADL", "HS"])
+@pytest.mark.parametrize("shape", ["graded", "uniform"])
+def test_on_a_surface(ctx, pde, k, kind, shape):
+    q = graded_sphere() if shape == "graded" else inti.p2_sphere_quadrature(7)
+    n = len(q)
+    assert n * n >= 2e6
+    A = operator(pde, kind, k, q, q, ctx)
+    rows = np.unique(np.concatenate([np.arange(0, n, 97), np.arange(n - 20, n)]))
+    for family in ("smooth", "unit", "gauss", "part"):
+        check(A, pde, kind, k, q, q, columns(q, family, bool(k)), rows)
+
+
+@pytest.mark.parametrize("pde,k", [("laplace", 0.0), ("helmholtz", 4.0)])
+@pytest.mark.parametrize("kind", ["DL", "HS"])
+@pytest.mark.parametrize("off", [1e-3, 1e-6])
+def test_close_to_a_surface(ctx, pde, k, kind, off):
+    """Targets at a small distance from nodes, among targets farther away."""
+    q = inti.p2_sphere_quadrature(7)
+    d = np.random.default_rng(5).standard_normal((900, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    t = np.concatenate([q.coords[::50] * (1 + off), 1.5 * d])
+    tgt = inti.Quadrature(t, t / np.linalg.norm(t, axis=1, keepdims=True), np.ones(len(t)), 0)
+    A = operator(pde, kind, k, tgt, q, ctx)
+    rows = np.concatenate([np.arange(0, 48, 3), np.arange(100, 900, 80)])
+    for family in ("smooth", "unit", "gauss", "part"):
+        check(A, pde, kind, k, tgt, q, columns(q, family, bool(k)), rows)
+
+
+def _captured(A, X, c, s):
+    """The product in a captured graph, which keeps the FP64 MMA kernel."""
+    x = torch.from_numpy(X.T.copy()).cuda()
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        A.apply_device(x.data_ptr(), y.data_ptr(), X.shape[1])
+    g.replay()
+    torch.cuda.synchronize()
+    out = y.cpu().numpy().T
+    del g
+    return out
+
+
+@pytest.mark.parametrize("pde,k", [("laplace", 0.0), ("helmholtz", 4.0)])
+@pytest.mark.parametrize("kind", ["SL", "DL", "ADL"])
+def test_which_form_takes_a_density(pde, k, kind):
+    """Smooth densities keep the fixed-point form (other last bits than the
+    FP64 MMA kernel), unit vectors and an otherwise smooth block with one
+    unit vector get the FP64 MMA kernel's own bits."""
+    s = torch.cuda.Stream()
+    c = inti.Context(0, stream=s.cuda_stream)
+    q = inti.p2_sphere_quadrature(7)
+    A = operator(pde, kind, k, q, q, c)
+    smooth, unit = columns(q, "smooth", bool(k)), columns(q, "unit", bool(k))
+    mixed = smooth.copy()
+    mixed[:, 5] = unit[:, 2]
+    assert not np.array_equal(A @ smooth, _captured(A, smooth, c, s))
+    for X in (unit, mixed):
+        assert np.array_equal(A @ X, _captured(A, X, c, s))
+
+
+def test_no_digit_product_is_missing(ctx):
+    """A sum of positive terms whose largest kernel value is about 2^5 times
+    the mean of n = 1,536: the reference is met to 8 roundings of a term and
+    what the dropped digits may take, n 2^-53.  One of the eight digit
+    products of the lowest kept order is worth 127 * 85 * 2^-70 per pair of the
+    two scales here (digits of 1/3), some 1e-12 of the sum."""
+    n = 1536
+    r = np.random.default_rng(3)
+    d = r.standard_normal((n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    src = inti.Quadrature(d, d.copy(), np.full(n, 1.0 / 3.0), 0)
+    tgt = inti.points(np.concatenate([1.02 * d[:64], 1.5 * r.standard_normal((1400, 3))]))
+    A = operator("laplace", "SL", 0.0, tgt, src, ctx)
+    X = np.ones((n, 8))
+    X *= 2.0 ** np.arange(8)
+    Y = A @ X
+    rows = np.arange(0, 64)
+    ref, T, _ = reference("laplace", "SL", 0.0, tgt, rows, src, X)
+    assert (np.abs(Y[rows] - ref) <= (8 + n / 16) * 2.0**-53 * T).all()
