@@ -768,6 +768,9 @@ __global__ void fx_plan_sources(int nstages, int J, const FxStage* __restrict__ 
   }
 }
 
+// The larger value; a NaN (of a coefficient that is not finite) stays.
+__device__ __forceinline__ double fx_max(double a, double b) { return b > a || b != b ? b : a; }
+
 // Bound of |K(x, y)| over the NA values from the modulus of the kernel (no
 // phase), with the distance d, id = 1/d, |r.n_x|, |r.n_y| and |n_x.n_y| given.
 template <int PDE, int KIND>
@@ -782,8 +785,8 @@ __device__ __forceinline__ double fx_modulus(double d, double id, double rnx, do
   if (KIND == ADL) return f * rnx;
   if (KIND == HS) return h;
   if (KIND == CF) return (fabs(c.c1r) + fabs(c.c1i)) * f * rny + (fabs(c.c2r) + fabs(c.c2i)) * id;
-  if (KIND == FX_THETA) return fmax(id, f * rny);
-  return fmax(f * rnx, h);
+  if (KIND == FX_THETA) return fx_max(id, f * rny);
+  return fx_max(f * rnx, h);
 }
 
 // Scale of each target row: a bound of its kernel values.  One warp per eight
@@ -847,7 +850,7 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
         const double id = rsqrt_fast(d2);
         const double rnx = fabs(a * t[3] + b * t[4] + e * t[5]), rny = fabs(a * n0 + b * n1 + e * n2);
         const double nn = fabs(t[3] * n0 + t[4] * n1 + t[5] * n2);
-        best[p] = fmax(best[p], fx_modulus<PDE, KIND>(d2 * id, id, rnx, rny, nn, c));
+        best[p] = fx_max(best[p], fx_modulus<PDE, KIND>(d2 * id, id, rnx, rny, nn, c));
       }
     }
   };
@@ -856,7 +859,7 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
 #pragma unroll
     for (int p = 0; p < NP; ++p)
       if (p == q / RP && lane / JL == q % RP) v = best[p];
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(kAll, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = fx_max(v, __shfl_xor_sync(kAll, v, o));
     return v;
   };
   int last = -1;

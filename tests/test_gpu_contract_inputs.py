@@ -34,3 +34,19 @@ def test_more_columns_than_a_grid_dimension_holds(ctx):
     ctx.synchronize()
     d = y.view(nrhs // 8, 8, n).sub_(ref)
     assert (d.norm(dim=2).amax(0) <= 1e-13 * ref.norm(dim=1)).all()
+
+
+@pytest.mark.parametrize("pde", ["laplace", "helmholtz"])
+@pytest.mark.parametrize("coefs", [(np.nan, 1.0), (1.0, np.nan), (np.inf, 1.0)])
+def test_coefficients_that_are_not_finite(ctx, pde, coefs):
+    """A combined field with such a coefficient: no entry of the block of
+    columns is finite, as in products of one column."""
+    cplx = pde == "helmholtz"
+    op = inti.Helmholtz(k=3.0, dim=3) if cplx else inti.Laplace(dim=3)
+    q = _points(1500, 2)
+    S = inti.GpuOperator(inti.SingleLayerKernel(op), q, q, None, "fp64", ctx)
+    D = inti.GpuOperator(inti.DoubleLayerKernel(op), q, q, None, "fp64", ctx)
+    A = inti.CombinedFieldOperator(D, S, *coefs)
+    X = np.stack([density(1500, cplx, c) for c in range(9)], axis=1)
+    assert not np.isfinite(A @ X[:, 0]).any()
+    assert not np.isfinite(A @ X).any()
