@@ -167,10 +167,14 @@ int inti_op_info(const inti_op* op, int64_t* m, int64_t* n, int* dtype);
  * ldy in elements).  alpha, beta: 2 doubles each (re, im); NULL means 1, 0.
  * beta = 0 does not read Y.  FP64 3D operators (every kernel) apply 8 or
  * more columns in one pass that evaluates each kernel value once for up to
- * 64 columns, multiplied with them as exact fixed-point products on the INT8
- * tensor path (from 2e6 pairs, outside stream capture) or on the FP64 MMA
- * path; other operators and fewer columns run one pair product per column.
- * Results agree to rounding (the summation order differs). */
+ * 64 columns.  From 2e6 pairs, outside stream capture, the values are
+ * multiplied with them as 64-bit fixed-point numbers on the INT8 tensor path
+ * while every entry's error stays below n 2^-52.8 times its sum of moduli (n
+ * real products; the a priori bound of an FP64 sum), which the device checks
+ * for each product; other blocks of columns (unit vectors, narrow bumps,
+ * refined surfaces, targets close to a surface) and smaller products take the
+ * FP64 MMA path.  Other operators and fewer columns run one pair product per
+ * column.  Results agree within those bounds (the summation order differs). */
 int inti_op_apply(inti_op* op, const double* x, int64_t ldx, double* y, int64_t ldy,
                   int32_t nrhs, const double* alpha, const double* beta, int on_device);
 /* Y = alpha*(A^T*X + C^T*X) + beta*Y: the transpose (not conjugate) apply,

@@ -115,7 +115,7 @@ struct FxStage {
 // lists, source records and row scales, all functions of the geometry, the
 // kernel and its coefficients.
 struct FxPlan {
-  DevBuf tables, records, tiles, rowscale, meta;
+  DevBuf tables, records, tiles, least_normal, rowscale, meta;
   const FxRows* rows = nullptr;  // in tables
   const FxStage* stages = nullptr;
   const FxItem* items = nullptr;
@@ -185,11 +185,11 @@ struct inti_ctx {
     inti::FxPlan plan;
   } dimwork;
   // Buffers of the multi-column contractions (contract_i8.cu): phase table,
-  // digit blocks of the densities, partial sums, and [flag, counters, column
-  // bounds].  Shared by the context's operators like the symmetric form's
+  // digit blocks of the densities, partial sums, [flag, counters, column
+  // bounds, digit sums], and the densities' mass per stage.  Shared by the context's operators like the symmetric form's
   // partials: live only within one product, on the context's one stream.
   struct {
-    inti::DevBuf tab, bdig, partial, work;
+    inti::DevBuf tab, bdig, partial, work, mass;
   } fx;
 };
 

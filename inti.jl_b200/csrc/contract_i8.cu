@@ -14,15 +14,23 @@
 // evaluation per pair and column group and four instructions per value that
 // cut it into digits.
 //
-// Accuracy.  Row i of A = K is scaled by a power of two that puts a bound of
-// |K_i.| just below 2^63, column c of B = diag(w) X by one for max |w x_c|;
-// both are rounded to integers (error 1/2 in 2^62..2^63) and the digit
-// products with p + q <= 7 are kept (p, q = 0 the leading digits; what is
-// dropped is below 2^-61 of the product of the two bounds per pair).  Sums
-// carry no rounding.  An FP64 accumulation of n terms rounds n times at
-// 2^-53 of the running sum, so the result is closer to the exact product of
-// the FP64 kernel values than the FP64 MMA's (measured against 64-bit
-// references in tests/test_gpu_contract.py).
+// Accuracy.  Row i of A = K is scaled by a power of two pa that takes a bound
+// of |K_i.| to 2^61.9 .. 2^62.9, column c of B = diag(w) X by one (pb) for max
+// |w x_c|; both are rounded to integers (error 1/2), the digit products with
+// p + q <= 7 are kept (p, q = 0 the leading digits) and the mean of the others
+// is added at the end (fx_mean).  Sums carry no rounding.  What is missing is at
+// most 2^65.2 / (pa pb) per real product, whatever the product's own size: one
+// scale serves a whole row and a whole column.  fx_guard therefore measures
+// each result's sum of moduli T against that unit, and the products in which
+// an entry would come out worse than n 2^-52.8 T, the a priori bound of an FP64
+// sum of n terms, are left to the FP64 kernels: unit vectors, narrow bumps,
+// densities on one part of a surface, refined surfaces, targets close to a
+// surface.  With smooth densities on uniform meshes the single and double
+// layers and Theta lie 2^7 to 2^16 above the limit, the hypersingular kernel
+// mostly below it.  Far above, the result is closer to the exact product of the
+// FP64 kernel values than an FP64 accumulation, which rounds n times at 2^-53
+// of the running sum (64 columns, 13,872 nodes: 1.9e-15 from 64-bit values).  tests/test_gpu_contract_accuracy.py
+// holds each entry to these bounds in extended precision.
 //
 // Work.  A persistent CTA per SM takes items (128 targets, a run of source
 // stages) from a counter, the longest first.  A stage is 64 K elements: NA
@@ -245,17 +253,17 @@ __device__ __forceinline__ bool fx_fits(double cur) { return cur == 0.0 || (cur 
 
 // Digits of A: the bytes of v rounded to a 64-bit integer, the leading one
 // signed, the others unsigned (the MMA takes the signedness of A per
-// instruction, so nothing has to be balanced).  The conversion runs on the
-// otherwise idle conversion unit; cutting v with rounding additions took four
-// FP64 instructions.
+// instruction, so nothing has to be balanced: that took 2% of a product and
+// 4% of Theta, and the mean of the dropped products is added in the end,
+// fx_mean).  The conversion runs on the otherwise idle conversion unit;
+// cutting v with rounding additions took four FP64 instructions.
 __device__ __forceinline__ uint2 fx_bytes(double v) {
   const long long w = __double2ll_rn(v);
   return make_uint2((uint32_t)w, (uint32_t)(w >> 32));
 }
 
 // Digits of B are balanced (-128 .. 127): the bytes of the integer plus 0x80
-// in every byte, each minus 128.  Their mean is zero, and so is that of what
-// is dropped.
+// in every byte, each minus 128.
 __device__ __forceinline__ uint2 fx_digits(double v) {
   const unsigned long long w = ((unsigned long long)__double2ll_rn(v) + 0x8080808080808080ULL) ^ 0x8080808080808080ULL;
   return make_uint2((uint32_t)w, (uint32_t)(w >> 32));
@@ -729,16 +737,17 @@ done:
 // ---------------------------------------------------------------------------
 // plan kernels
 // ---------------------------------------------------------------------------
-// Centre and radius of each stage's sources (double4) and their records; the
-// largest normal of all sources (bits in meta[0]).
+// Centre and radius of each stage's sources (double4), their least normal and
+// their records; the largest normal of all sources (bits in meta[0]).
 __global__ void fx_plan_sources(int nstages, int J, const FxStage* __restrict__ stages,
                                 const double* __restrict__ coords, const double* __restrict__ normals,
                                 double* __restrict__ records, double4* __restrict__ tiles,
-                                unsigned long long* __restrict__ meta) {
+                                double* __restrict__ least_normal, unsigned long long* __restrict__ meta) {
   const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (s >= nstages) return;
   const FxStage st = stages[s];
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY}, n2 = 0.0;
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY}, n2 = 0.0,
+         least = INFINITY;
   for (int j = lane; j < J; j += 32) {
     double v[FX_REC] = {0, 0, 0, 0, 0, 0};
     if (j < st.count) {
@@ -749,7 +758,9 @@ __global__ void fx_plan_sources(int nstages, int J, const FxStage* __restrict__ 
         hi[c] = fmax(hi[c], v[c]);
         if (normals) v[3 + c] = normals[3 * i + c];
       }
-      n2 = fmax(n2, v[3] * v[3] + v[4] * v[4] + v[5] * v[5]);
+      const double q2 = v[3] * v[3] + v[4] * v[4] + v[5] * v[5];
+      n2 = fmax(n2, q2);
+      least = fmin(least, q2);
     }
     for (int c = 0; c < FX_REC; ++c) records[((int64_t)s * J + j) * FX_REC + c] = v[c];
   }
@@ -759,8 +770,10 @@ __global__ void fx_plan_sources(int nstages, int J, const FxStage* __restrict__ 
       hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
     }
     n2 = fmax(n2, __shfl_xor_sync(0xffffffffu, n2, o));
+    least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
   }
   if (lane == 0) {
+    least_normal[s] = sqrt(least);
     const double a = hi[0] - lo[0], b = hi[1] - lo[1], c = hi[2] - lo[2];
     tiles[s] = make_double4((lo[0] + hi[0]) / 2, (lo[1] + hi[1]) / 2, (lo[2] + hi[2]) / 2,
                             0.5 * sqrt(a * a + b * b + c * c) * (1 + 1e-12));
@@ -926,21 +939,23 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
 // ---------------------------------------------------------------------------
 // colmax[surf * ncol + c]: bits of max |w x| over the (Re, Im) parts of column c.  Non-negative doubles
 // order as their bits; a NaN's exceed every number's.
+// mass[stage * ncol + c]: at most the sum of |w x| (the larger part) over the
+// stage without its largest term, so that it holds for a target that is one
+// of the stage's nodes, too.
 constexpr int kMaxRun = 8;  // stages per warp
+
+__device__ __forceinline__ double fx_mass(double sum, double top) { return fmax(0.0, (sum - top) - 1e-14 * sum); }
 
 template <bool CPLX>
 __global__ void fx_colmax(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
-                          const double* __restrict__ x, int64_t ldx, int ncol, unsigned long long* colmax) {
+                          const double* __restrict__ x, int64_t ldx, int ncol, unsigned long long* colmax,
+                          double* __restrict__ mass) {
   const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int s0 = run * kMaxRun, s1 = min(nstages, s0 + kMaxRun);
   for (int c = blockIdx.y; c < ncol; c += gridDim.y) {  // (a grid dimension holds 65,535)
     unsigned long long best = 0;
     int surf = -1;
     auto flush = [&]() {
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other > best ? other : best;
-      }
       if (lane == 0 && surf >= 0) atomicMax(&colmax[(int64_t)surf * ncol + c], best);
       best = 0;
     };
@@ -950,6 +965,8 @@ __global__ void fx_colmax(int nstages, const FxStage* __restrict__ stages, const
         flush();
         surf = st.surf;
       }
+      double sum = 0.0;
+      unsigned long long top = 0;
       for (int j = lane; j < st.count; j += 32) {
         const int64_t i = st.src0 + j;
         const int64_t q = (int64_t)c * ldx + i;
@@ -961,20 +978,210 @@ __global__ void fx_colmax(int nstages, const FxStage* __restrict__ stages, const
         } else {
           m = fabs(w[i] * x[q]);
         }
+        sum += m;
         const unsigned long long b = (unsigned long long)__double_as_longlong(m);
-        best = b > best ? b : best;
+        top = b > top ? b : top;
       }
+      for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, top, o);
+        top = other > top ? other : top;
+      }
+      if (lane == 0) mass[(int64_t)s * ncol + c] = fx_mass(sum, __longlong_as_double((long long)top));
+      best = top > best ? top : best;
     }
     flush();
   }
 }
 
-// Sets the flag when a row or column bound does not fit (one block).
-__global__ void fx_check(int count, const unsigned long long* __restrict__ colmax,
-                         const unsigned long long* __restrict__ meta, int* flag) {
-  bool bad = meta[1] != 0;
-  for (int q = threadIdx.x; q < count; q += blockDim.x) bad |= !fx_fits(__longlong_as_double((long long)colmax[q]));
-  if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
+// ---------------------------------------------------------------------------
+// what the fixed-point form may take
+// ---------------------------------------------------------------------------
+// At most the modulus of the kernel's values (FX_THETA, FX_THETA_D: of the two
+// kernels) at distance d, without the cosines of r with the normals: the size
+// at which their evaluation rounds, |n| d in the place of |r.n|.  Falls with d.
+template <int PDE, int KIND>
+__device__ __forceinline__ double2 fx_least(double d, double nx, double ny, const FxConst& c) {
+  const double id = 1.0 / d;
+  const double f = (PDE == HELMHOLTZ ? sqrt(fma(c.k, c.k, id * id)) : id) * id;  // |1/d - ik|/d
+  if (KIND == SL) return make_double2(id, 0.0);
+  if (KIND == DL) return make_double2(f * ny, 0.0);
+  if (KIND == ADL) return make_double2(f * nx, 0.0);
+  if (KIND == HS) return make_double2(f * id * nx * ny, 0.0);
+  if (KIND == CF) return make_double2(hypot(c.c1r, c.c1i) * f * ny + hypot(c.c2r, c.c2i) * id, 0.0);
+  if (KIND == FX_THETA) return make_double2(id, f * ny);
+  return make_double2(f * nx, f * id * nx * ny);
+}
+
+struct FxGuard {
+  const FxRows* rows;
+  const double4* tiles;
+  const double* least_normal;
+  const double* tcoords;
+  const double* tnormals;
+  const double* rowscale;
+  const double* mass;   // Theta: of g1, then of g0
+  int64_t mass_stride;  // between the two
+  const unsigned long long* colmax;
+  const unsigned long long* meta;
+  int ncol;
+  FxConst c;
+  int* flag;
+};
+
+// Sets the flag when a row or column bound does not fit, and when a result
+// would not come out as well as an FP64 sum.  What the digits leave out and
+// the rounding to integers is at most 2^65.2 units per real product, a unit
+// being 1/(pa pb) for the scales of the row and the column (seven products of
+// order 8 of at most 2^14 each, and half a unit of either factor), so it stays
+// below n 2^-52.8 T for n products while
+//
+//     T = sum_j |K_ij| |w_j x_jc| >= 2^-8 2^126 / (pa pb)
+//
+// (2^63/pa and 2^63/pb lie between one and 2.1 times the largest |K_ij| and
+// |w_j x_jc|).  As terms of mean zero they come to about sqrt(n) 2^-56 T at that
+// limit.
+//
+// T is bounded from below stage by stage: the stage's mass times the kernel's
+// modulus at the largest distance between its sources and the 16 rows of a
+// group, from the nearest 64 stages on; a block is done when its rows and
+// columns (128 x 64) have what they need.  Smooth densities need one round:
+// 16 us of 1,880 at 13,872 nodes and 64 complex columns, 30 of 16,000 for the
+// Theta of 43,200 nodes.
+constexpr double kFxFloor = 1.0 / 256;
+constexpr int kGuardRows = 16, kGuardGroups = FX_M / kGuardRows;
+
+template <int PDE, int KIND>
+__global__ void __launch_bounds__(256) fx_guard(FxGuard a) {
+  using SH = FxShape<PDE, KIND>;
+  constexpr int NM = SH::theta ? 2 : 1, CH = 64;
+  constexpr double kDown = 1.0 / 9223372036854775808.0;  // 2^-63
+  __shared__ double grp[kGuardGroups][6];                // centre, radius, scale (0: nothing to check), least |n_x|
+  __shared__ float m[NM][kGuardGroups][CH];
+  __shared__ unsigned long long near;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const FxRows rb = a.rows[blockIdx.x];
+  if (tid == 0) near = ~0ULL;
+  if (tid < FX_M) {
+    const bool in = tid < rb.nrows;
+    const int64_t row = rb.row0 + min(tid, rb.nrows - 1);
+    double lo[3], hi[3], n2 = 0.0, p = in ? a.rowscale[row] : 0.0;
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = hi[c] = a.tcoords[3 * row + c];
+      if (SH::tnormal) n2 += a.tnormals[3 * row + c] * a.tnormals[3 * row + c];
+    }
+    if (p == 0.0) p = INFINITY;  // a row of zeros (or past the end)
+    for (int o = kGuardRows / 2; o > 0; o >>= 1) {
+      for (int c = 0; c < 3; ++c) {
+        lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+        hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+      }
+      n2 = fmin(n2, __shfl_xor_sync(0xffffffffu, n2, o));
+      p = fmin(p, __shfl_xor_sync(0xffffffffu, p, o));
+    }
+    if (lane % kGuardRows == 0) {
+      const double x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
+      double* g = grp[tid / kGuardRows];
+      for (int c = 0; c < 3; ++c) g[c] = (lo[c] + hi[c]) / 2;
+      g[3] = 0.5 * sqrt(x * x + y * y + z * z);
+      g[4] = p < INFINITY ? p : 0.0;
+      g[5] = sqrt(n2);
+    }
+  }
+  const int c = blockIdx.y * CH + (tid & (CH - 1)), g0 = tid / CH * 2;  // this thread's column and two groups
+  double pb = 0.0;
+  bool bad = a.meta[1] != 0;
+  if (c < a.ncol) {
+    const double top = __longlong_as_double((long long)a.colmax[(int64_t)rb.surf * a.ncol + c]);
+    bad |= !fx_fits(top);
+    if (!bad) pb = fx_scale(top);
+  }
+  const bool stop = tid == 0 && *(volatile int*)a.flag != 0;  // another block's finding
+  if (__syncthreads_or(bad || stop)) {
+    if (bad) *a.flag = 1;
+    return;
+  }
+  const int nch = (rb.nstages + CH - 1) / CH;
+  unsigned long long mine = ~0ULL;
+  for (int s = tid; s < rb.nstages; s += 256) {  // the stage nearest to the first group
+    const double4 t = a.tiles[rb.stage0 + s];
+    const float x = (float)(grp[0][0] - t.x), y = (float)(grp[0][1] - t.y), z = (float)(grp[0][2] - t.z);
+    mine = min(mine, (unsigned long long)__float_as_uint(x * x + y * y + z * z) << 32 | (unsigned)s);
+  }
+  for (int o = 16; o > 0; o >>= 1) mine = min(mine, __shfl_xor_sync(0xffffffffu, mine, o));
+  if (lane == 0) atomicMin(&near, mine);
+  __syncthreads();
+  const int first = (int)((unsigned)near / CH);
+  const bool need[2] = {pb > 0.0 && grp[g0][4] > 0.0, pb > 0.0 && grp[g0 + 1][4] > 0.0};
+  float t[2] = {0.f, 0.f};
+  for (int q = 0; q < nch; ++q) {
+    const int s0 = (first + q) % nch * CH, cnt = min(CH, rb.nstages - s0);
+    __syncthreads();
+    for (int e = tid; e < kGuardGroups * cnt; e += 256) {
+      const int g = e / cnt, s = e - g * cnt;
+      const double4 tl = a.tiles[rb.stage0 + s0 + s];
+      const double x = grp[g][0] - tl.x, y = grp[g][1] - tl.y, z = grp[g][2] - tl.z;
+      const double d = (sqrt(x * x + y * y + z * z) + tl.w + grp[g][3]) * (1 + 1e-9);
+      const double2 v = fx_least<PDE, KIND>(d, grp[g][5], a.least_normal[rb.stage0 + s0 + s], a.c);
+      m[0][g][s] = (float)fmin(v.x * grp[g][4] * kDown, 1e30);
+      if (SH::theta) m[NM - 1][g][s] = (float)fmin(v.y * grp[g][4] * kDown, 1e30);
+    }
+    __syncthreads();
+    if (need[0] || need[1]) {
+      const double* ms = a.mass + (int64_t)(rb.stage0 + s0) * a.ncol + c;
+#pragma unroll 16
+      for (int s = 0; s < cnt; ++s) {
+        const float w = (float)(ms[(int64_t)s * a.ncol] * (pb * kDown));
+        t[0] = fmaf(m[0][g0][s], w, t[0]);
+        t[1] = fmaf(m[0][g0 + 1][s], w, t[1]);
+        if (SH::theta) {
+          const float u = (float)(ms[a.mass_stride + (int64_t)s * a.ncol] * (pb * kDown));
+          t[0] = fmaf(m[NM - 1][g0][s], u, t[0]);
+          t[1] = fmaf(m[NM - 1][g0 + 1][s], u, t[1]);
+        }
+      }
+    }
+    const bool pass = (!need[0] || t[0] >= (float)(kFxFloor * 1.001)) && (!need[1] || t[1] >= (float)(kFxFloor * 1.001));
+    if (__syncthreads_and(pass)) return;
+  }
+  if (tid == 0) *a.flag = 1;
+}
+
+// Mean of the digit products that are dropped, p + q > 7, of a column in units
+// of 256^7: A's lower digits are about 127.5 on average, so it is 1/2 times the
+// sum of B's digits 1 to 7 (fx_pack), and what is left has mean zero.  Without
+// it they add up where B's digits are alike: the sum of 1,536 terms of a
+// constant density, largest kernel value 50 times the mean, 1.8e-16 -> 8e-18 of
+// the sum (from the digits in exact arithmetic).  A sum that is exactly zero
+// (kernel values of zero) stays.
+__device__ __forceinline__ double fx_mean(double sum, long long digits) {
+  return sum != 0.0 ? fma(0.5, (double)digits, sum) : 0.0;
+}
+// Sum of the digits 1 to 7 of four values.
+__device__ __forceinline__ int fx_low(const uint32_t (&w)[FX_D]) {
+  int s = 0;
+#pragma unroll
+  for (int q = 1; q < FX_D; ++q) s = __dp4a((int)w[q], 0x01010101, s);
+  return s;
+}
+// Adds a thread's sums for column c (r, and i of complex columns) to the
+// columns' totals of its surface: integers, in any order.  The threads of the
+// block's first surface meet in shared memory (zero at the start).
+template <int COMPS>
+__device__ __forceinline__ void fx_add(int* block, bool live, int surf, int surf0, int64_t stride, int c, int r, int i,
+                                       int columns, long long* total) {
+  auto global = [&](int64_t at, int v) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(total + at), (unsigned long long)(long long)v);
+  };
+  if (live && surf == surf0) {
+    atomicAdd(block + COMPS * c, r);
+    if (COMPS == 2) atomicAdd(block + COMPS * c + 1, i);
+  } else if (live) {
+    global(surf * stride + COMPS * c, r);
+    if (COMPS == 2) global(surf * stride + COMPS * c + 1, i);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < COMPS * columns) global(surf0 * stride + threadIdx.x, block[threadIdx.x]);
 }
 
 // Digit blocks: stage s, digit q of column n at [chunk][q * nc + n][16 bytes].
@@ -985,7 +1192,7 @@ template <bool CPLX>
 __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
                         const double* __restrict__ x, int64_t ldx, int c0, int ncol, int half, int nall, int nc,
                         const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
-                        unsigned char* __restrict__ out) {
+                        unsigned char* __restrict__ out, long long* __restrict__ digits) {
   constexpr int JT = CPLX ? 8 : 16;  // sources of a chunk
   // plane blockIdx.y: columns c0 + y * half and on
   c0 += blockIdx.y * half;
@@ -995,9 +1202,13 @@ __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const d
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int c = (int)(id % per), chunk = (int)(id / per % 4);
   const int64_t s = id / per / 4;
-  if (s >= nstages || *flag) return;
-  const FxStage st = stages[s];
-  const bool live = c < ncol;
+  if (*flag) return;
+  __shared__ int low[FX_NMAX];
+  if (threadIdx.x < FX_NMAX) low[threadIdx.x] = 0;
+  __syncthreads();
+  const bool in = s < nstages;
+  const FxStage st = stages[in ? s : nstages - 1];
+  const bool live = in && c < ncol;
   const double p =
       live ? fx_scale(__longlong_as_double((long long)colmax[(int64_t)st.surf * nall + c0 + c])) : 0.0;
   uint4* o = reinterpret_cast<uint4*>(out + s * ((int64_t)nc * FX_D * FX_K) + (int64_t)chunk * (nc * FX_D * 16));
@@ -1031,6 +1242,19 @@ __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const d
       fx_pack4(m, mi[h]);
     }
   }
+  int lr = 0, li = 0, lm = 0;
+#pragma unroll
+  for (int h = 0; h < JT / 4; ++h) {
+    lr += fx_low(re[h]);
+    if constexpr (CPLX) {
+      li += fx_low(im[h]);
+      lm += fx_low(mi[h]);
+    }
+  }
+  constexpr int COMPS = CPLX ? 2 : 1;
+  fx_add<COMPS>(low, live, st.surf, stages[blockIdx.x * (int64_t)blockDim.x / per / 4].surf, (int64_t)nall * COMPS, c,
+                lr + lm, li + lr, ncol, digits + (int64_t)c0 * COMPS);
+  if (!in) return;
 #pragma unroll
   for (int q = 0; q < FX_D; ++q) {
     if constexpr (CPLX) {
@@ -1043,24 +1267,37 @@ __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const d
 }
 
 // Theta: column bounds over the traces (both arrays share a column's scale,
-// since their products share the accumulators).
-__global__ void fx_theta_max(int64_t n, int ns, bool cplx, const double* __restrict__ w, const double2* __restrict__ g0,
-                             const double2* __restrict__ g1, unsigned long long* colmax) {
-  // a block takes 256 consecutive nodes; thread t the entries t, t + 256, ... of their rows
+// since their products share the accumulators) and the masses of g1 and g0.
+// One thread per (stage, column).
+__global__ void fx_theta_max(int nstages, const FxStage* __restrict__ stages, int ns, bool cplx,
+                             const double* __restrict__ w, const double2* __restrict__ g0,
+                             const double2* __restrict__ g1, unsigned long long* colmax, double* __restrict__ mass) {
   __shared__ unsigned long long best[32];
   if (threadIdx.x < 32) best[threadIdx.x] = 0;
   __syncthreads();
-  const int64_t j0 = blockIdx.x * (int64_t)256, j1 = min(n, j0 + 256);
-  for (int64_t e = j0 * ns + threadIdx.x; e < j1 * ns; e += blockDim.x) {
-    const int64_t j = e / ns;
-    const double2 a = g0[e], b = g1[e];
-    const double v[4] = {a.x, b.x, cplx ? a.y : 0.0, cplx ? b.y : 0.0};
-    unsigned long long m = 0;
-    for (int q = 0; q < 4; ++q) {
-      const unsigned long long t = (unsigned long long)__double_as_longlong(fabs(w[j] * v[q]));
-      m = t > m ? t : m;
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int s = (int)(id / ns), k = (int)(id - (int64_t)s * ns);
+  if (s < nstages) {
+    const FxStage st = stages[s];
+    double sum[2] = {0.0, 0.0};
+    unsigned long long top[2] = {0, 0};
+    for (int j = 0; j < st.count; ++j) {
+      const int64_t i = st.src0 + j, e = i * ns + k;
+      const double wj = w[i];
+      const double2 v[2] = {g1[e], g0[e]};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double re = fabs(wj * v[q].x), im = cplx ? fabs(wj * v[q].y) : 0.0;
+        const double mx = re > im || re != re ? re : im;
+        const unsigned long long b = (unsigned long long)__double_as_longlong(mx);
+        sum[q] += mx;
+        top[q] = b > top[q] ? b : top[q];
+      }
     }
-    atomicMax(&best[(int)(e - j * ns)], m);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      mass[(int64_t)q * nstages * ns + id] = fx_mass(sum[q], __longlong_as_double((long long)top[q]));
+    atomicMax(&best[k], top[0] > top[1] ? top[0] : top[1]);
   }
   __syncthreads();
   if ((int)threadIdx.x < ns) atomicMax(&colmax[threadIdx.x], best[threadIdx.x]);
@@ -1073,15 +1310,19 @@ template <bool CPLX>
 __global__ void fx_theta_pack(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
                               const double2* __restrict__ g0, const double2* __restrict__ g1, int ns, int nc,
                               const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
-                              unsigned char* __restrict__ out) {
+                              unsigned char* __restrict__ out, long long* __restrict__ digits) {
   constexpr int JT = CPLX ? 4 : 8;
   const int per = CPLX ? nc / 2 : nc;
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int c = (int)(id % per), chunk = (int)(id / per % 4);
   const int64_t s = id / per / 4;
-  if (s >= nstages || *flag) return;
-  const FxStage st = stages[s];
-  const bool live = c < ns;
+  if (*flag) return;
+  __shared__ int low[FX_NMAX];
+  if (threadIdx.x < FX_NMAX) low[threadIdx.x] = 0;
+  __syncthreads();
+  const bool in = s < nstages;
+  const FxStage st = stages[in ? s : nstages - 1];
+  const bool live = in && c < ns;
   const double p = live ? fx_scale(__longlong_as_double((long long)colmax[c])) : 0.0;
   uint4* o = reinterpret_cast<uint4*>(out + s * ((int64_t)nc * FX_D * FX_K) + (int64_t)chunk * (nc * FX_D * 16));
   double2 a[JT], b[JT];
@@ -1111,6 +1352,9 @@ __global__ void fx_theta_pack(int nstages, const FxStage* __restrict__ stages, c
     pack([&](int e) { return -a[e].x; }, wd[3]);
     pack([&](int e) { return -a[e].y; }, wd[4]);
     pack([&](int e) { return a[e].y; }, wd[5]);
+    fx_add<2>(low, live, 0, 0, 0, c, fx_low(wd[0]) + fx_low(wd[2]) + fx_low(wd[3]) + fx_low(wd[5]),
+              fx_low(wd[1]) + fx_low(wd[0]) + fx_low(wd[4]) + fx_low(wd[3]), ns, digits);
+    if (!in) return;
 #pragma unroll
     for (int q = 0; q < FX_D; ++q) {
       o[q * nc + 2 * c] = make_uint4(wd[0][q], wd[2][q], wd[3][q], wd[5][q]);
@@ -1121,6 +1365,8 @@ __global__ void fx_theta_pack(int nstages, const FxStage* __restrict__ stages, c
     pack([&](int e) { return b[e + 4].x; }, wd[1]);
     pack([&](int e) { return -a[e].x; }, wd[2]);
     pack([&](int e) { return -a[e + 4].x; }, wd[3]);
+    fx_add<1>(low, live, 0, 0, 0, c, fx_low(wd[0]) + fx_low(wd[1]) + fx_low(wd[2]) + fx_low(wd[3]), 0, ns, digits);
+    if (!in) return;
 #pragma unroll
     for (int q = 0; q < FX_D; ++q) o[q * nc + c] = make_uint4(wd[0][q], wd[2][q], wd[1][q], wd[3][q]);
   }
@@ -1149,6 +1395,7 @@ struct FxOut {
   const double* partial;
   const double* rowscale;
   const unsigned long long* colmax;
+  const long long* digits;
   const int* flag;
   const int64_t* rowptr;  // correction, null when there is none
   const int32_t* col;
@@ -1174,11 +1421,12 @@ __global__ void __launch_bounds__(FX_M) fx_finish(FxOut o) {
   const double* partial = o.partial + (size_t)(c / o.half) * o.nslots * o.nc * FX_M;
   const int cp = c % o.half;
   double sr, si = 0.0;
+  const long long* d = o.digits + ((int64_t)rb.surf * o.nall + cg) * (CPLX ? 2 : 1);
   if (CPLX) {
-    sr = u * fx_total(rb, partial, o.nc, 2 * cp, r);
-    si = u * fx_total(rb, partial, o.nc, 2 * cp + 1, r);
+    sr = u * fx_mean(fx_total(rb, partial, o.nc, 2 * cp, r), d[0]);
+    si = u * fx_mean(fx_total(rb, partial, o.nc, 2 * cp + 1, r), d[1]);
   } else {
-    sr = u * fx_total(rb, partial, o.nc, cp, r);
+    sr = u * fx_mean(fx_total(rb, partial, o.nc, cp, r), d[0]);
   }
   if (o.rowptr) {
     for (int64_t p = o.rowptr[row]; p < o.rowptr[row + 1]; ++p) {
@@ -1213,7 +1461,8 @@ template <bool CPLX>
 __global__ void __launch_bounds__(FX_M) fx_theta_finish(const FxRows* __restrict__ rows,
                                                         const double* __restrict__ partial,
                                                         const double* __restrict__ rowscale,
-                                                        const unsigned long long* __restrict__ colmax, int ns, int nc,
+                                                        const unsigned long long* __restrict__ colmax,
+                                                        const long long* __restrict__ digits, int ns, int nc,
                                                         const int* __restrict__ flag, double2* __restrict__ out) {
   if (*flag) return;
   const FxRows rb = rows[blockIdx.x];
@@ -1224,10 +1473,10 @@ __global__ void __launch_bounds__(FX_M) fx_theta_finish(const FxRows* __restrict
                    fx_inverse(fx_scale(__longlong_as_double((long long)colmax[c]))) * (1.0 / (4 * kPi) * kFxUnit);
   double2 v = make_double2(0.0, 0.0);
   if (CPLX) {
-    v.x = u * fx_total(rb, partial, nc, 2 * c, r);
-    v.y = u * fx_total(rb, partial, nc, 2 * c + 1, r);
+    v.x = u * fx_mean(fx_total(rb, partial, nc, 2 * c, r), digits[2 * c]);
+    v.y = u * fx_mean(fx_total(rb, partial, nc, 2 * c + 1, r), digits[2 * c + 1]);
   } else {
-    v.x = u * fx_total(rb, partial, nc, c, r);
+    v.x = u * fx_mean(fx_total(rb, partial, nc, c, r), digits[c]);
   }
   out[row * ns + c] = v;
 }
@@ -1290,10 +1539,11 @@ static FxPass fx_pass(int left, int comps) {
   p.nc = fx_width(p.half * comps);
   return p;
 }
-// work: [flag, counter per pass (up to 63) | column bounds]
+// work: [flag, counter per pass (up to 63) | column bounds | digit sums of the
+// columns' one or two components]
 constexpr int FX_COUNTERS = 64;
-static size_t fx_work_bytes(int nsurf, int ncols) {
-  return sizeof(int) * FX_COUNTERS + sizeof(unsigned long long) * (size_t)nsurf * ncols;
+static size_t fx_work_bytes(const FxProblem& p, int nsurf, int ncols) {
+  return sizeof(int) * FX_COUNTERS + sizeof(long long) * (size_t)nsurf * ncols * (p.pde == HELMHOLTZ ? 3 : 2);
 }
 
 static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
@@ -1347,12 +1597,13 @@ static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
   plan.items = reinterpret_cast<const FxItem*>(plan.tables.as<unsigned char>() + b_rows + b_stages);
   plan.records.ensure(sizeof(double) * FX_REC * J * stages.size());
   plan.tiles.ensure(sizeof(double4) * stages.size());
+  plan.least_normal.ensure(sizeof(double) * stages.size());
   plan.rowscale.ensure(sizeof(double) * std::max<int64_t>(plan.ntargets, 1));
   plan.meta.ensure(sizeof(unsigned long long) * 2);
   INTI_CUDA(cudaMemsetAsync(plan.meta.p, 0, sizeof(unsigned long long) * 2, ctx->stream));
   fx_plan_sources<<<(plan.nstages + 7) / 8, 256, 0, ctx->stream>>>(
       plan.nstages, J, plan.stages, p.coords, p.normals, plan.records.as<double>(),
-      plan.tiles.as<double4>(), plan.meta.as<unsigned long long>());
+      plan.tiles.as<double4>(), plan.least_normal.as<double>(), plan.meta.as<unsigned long long>());
   fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
     constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
     fx_plan_rows<P, K><<<(unsigned)plan.nrows * (FX_M / kPlanRows / 8), 256, 0, ctx->stream>>>(
@@ -1387,7 +1638,8 @@ bool fx_prepare(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, int ncols) {
     if (!plan.ready) fx_plan(ctx, p, plan);
     ctx->fx.bdig.ensure(digits());
     ctx->fx.partial.ensure(partial());
-    ctx->fx.work.ensure(fx_work_bytes(plan.nsurf, ncols));
+    ctx->fx.work.ensure(fx_work_bytes(p, plan.nsurf, ncols));
+    ctx->fx.mass.ensure(sizeof(double) * (size_t)plan.nstages * ncols * (p.kind >= FX_THETA ? 2 : 1));
   } catch (const Error& e) {
     if (e.code != INTI_E_NOMEM) throw;
     return false;
@@ -1397,6 +1649,32 @@ bool fx_prepare(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, int ncols) {
 
 static unsigned long long* fx_colmax_ptr(inti_ctx* ctx) {
   return reinterpret_cast<unsigned long long*>(ctx->fx.work.as<int>() + FX_COUNTERS);
+}
+
+static long long* fx_digits_ptr(inti_ctx* ctx, const FxPlan& plan, int ncols) {
+  return reinterpret_cast<long long*>(fx_colmax_ptr(ctx)) + (size_t)plan.nsurf * ncols;
+}
+
+static void fx_guard_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int ncol) {
+  FxGuard a;
+  a.rows = plan.rows;
+  a.tiles = plan.tiles.as<double4>();
+  a.least_normal = plan.least_normal.as<double>();
+  a.tcoords = p.tcoords;
+  a.tnormals = p.tnormals;
+  a.rowscale = plan.rowscale.as<double>();
+  a.mass = ctx->fx.mass.as<double>();
+  a.mass_stride = (int64_t)plan.nstages * ncol;
+  a.colmax = fx_colmax_ptr(ctx);
+  a.meta = plan.meta.as<unsigned long long>();
+  a.ncol = ncol;
+  a.c = fx_const(p);
+  a.flag = ctx->fx.work.as<int>();
+  fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
+    constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
+    fx_guard<P, K><<<dim3((unsigned)plan.nrows, (unsigned)((ncol + 63) / 64)), 256, 0, ctx->stream>>>(a);
+  });
+  ctx->launches++;
 }
 
 static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc, int planes, int* counter) {
@@ -1447,17 +1725,17 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
               int64_t ldx, double* y, int64_t ldy, int nrhs, const double* alpha, const double* beta) {
   const bool cplx = p.pde == HELMHOLTZ;
   const int comps = cplx ? 2 : 1;
-  INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(plan.nsurf, nrhs), ctx->stream));
+  INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(p, plan.nsurf, nrhs), ctx->stream));
   int* flag = ctx->fx.work.as<int>();
   unsigned long long* colmax = fx_colmax_ptr(ctx);
   const FxStage* st = plan.stages;
-  const unsigned long long* meta = plan.meta.as<unsigned long long>();
   auto by_type = [&](auto cc) {
     constexpr bool C = decltype(cc)::value;
     const int runs = (plan.nstages + kMaxRun - 1) / kMaxRun;
-    fx_colmax<C><<<dim3((runs + 7) / 8, std::min(nrhs, 65535)), 256, 0, ctx->stream>>>(plan.nstages, st, p.weights, x, ldx, nrhs, colmax);
-    fx_check<<<1, 256, 0, ctx->stream>>>(plan.nsurf * nrhs, colmax, meta, flag);
-    ctx->launches += 2;
+    fx_colmax<C><<<dim3((runs + 7) / 8, std::min(nrhs, 65535)), 256, 0, ctx->stream>>>(plan.nstages, st, p.weights, x, ldx, nrhs, colmax,
+                                                                 ctx->fx.mass.as<double>());
+    ctx->launches++;
+    fx_guard_run(ctx, p, plan, nrhs);
     int pass = 0;
     FxPass w;
     for (int c0 = 0; c0 < nrhs; c0 += w.cols, ++pass) {
@@ -1465,7 +1743,7 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
       const int64_t threads = (int64_t)plan.nstages * 4 * (w.nc / comps);
       fx_pack<C><<<dim3((unsigned)((threads + 127) / 128), w.planes), 128, 0, ctx->stream>>>(
           plan.nstages, st, p.weights, x, ldx, c0, w.cols, w.half, nrhs, w.nc, colmax, flag,
-          ctx->fx.bdig.as<unsigned char>());
+          ctx->fx.bdig.as<unsigned char>(), fx_digits_ptr(ctx, plan, nrhs));
       ctx->launches++;
       const int slot = 1 + pass % (FX_COUNTERS - 1);
       if (pass >= FX_COUNTERS - 1) INTI_CUDA(cudaMemsetAsync(flag + slot, 0, sizeof(int), ctx->stream));
@@ -1475,6 +1753,7 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
       o.partial = ctx->fx.partial.as<double>();
       o.rowscale = plan.rowscale.as<double>();
       o.colmax = colmax;
+      o.digits = fx_digits_ptr(ctx, plan, nrhs);
       o.flag = flag;
       o.rowptr = corr ? corr->rowptr.as<int64_t>() : nullptr;
       o.col = corr ? corr->col.as<int32_t>() : nullptr;
@@ -1510,27 +1789,28 @@ void fx_theta(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const doubl
               double2* out) {
   const bool cplx = p.pde == HELMHOLTZ;
   const int nc = fx_width(ns * (cplx ? 2 : 1));
-  INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(plan.nsurf, ns), ctx->stream));
+  INTI_CUDA(cudaMemsetAsync(ctx->fx.work.p, 0, fx_work_bytes(p, plan.nsurf, ns), ctx->stream));
   int* flag = ctx->fx.work.as<int>();
   unsigned long long* colmax = fx_colmax_ptr(ctx);
-  const int64_t n = p.nsrc[0];
-  fx_theta_max<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(n, ns, cplx, p.weights, g0, g1, colmax);
-  fx_check<<<1, 32, 0, ctx->stream>>>(ns, colmax, plan.meta.as<unsigned long long>(), flag);
+  fx_theta_max<<<(unsigned)(((int64_t)plan.nstages * ns + 255) / 256), 256, 0, ctx->stream>>>(
+      plan.nstages, plan.stages, ns, cplx, p.weights, g0, g1, colmax, ctx->fx.mass.as<double>());
+  fx_guard_run(ctx, p, plan, ns);
   const int64_t threads = (int64_t)plan.nstages * 4 * (cplx ? nc / 2 : nc);
   auto by_type = [&](auto cc) {
     constexpr bool C = decltype(cc)::value;
     fx_theta_pack<C><<<(unsigned)((threads + 127) / 128), 128, 0, ctx->stream>>>(
         plan.nstages, plan.stages, p.weights, g0, g1, ns, nc, colmax, flag,
-        ctx->fx.bdig.as<unsigned char>());
+        ctx->fx.bdig.as<unsigned char>(), fx_digits_ptr(ctx, plan, ns));
     fx_run(ctx, p, plan, nc, 1, flag + 1);
     fx_theta_finish<C><<<dim3(plan.nrows, ns), FX_M, 0, ctx->stream>>>(
-        plan.rows, ctx->fx.partial.as<double>(), plan.rowscale.as<double>(), colmax, ns, nc, flag, out);
+        plan.rows, ctx->fx.partial.as<double>(), plan.rowscale.as<double>(), colmax,
+        fx_digits_ptr(ctx, plan, ns), ns, nc, flag, out);
   };
   if (cplx)
     by_type(std::true_type());
   else
     by_type(std::false_type());
-  ctx->launches += 4;
+  ctx->launches += 3;
   INTI_CUDA(cudaGetLastError());
 }
 

@@ -37,8 +37,10 @@ bool fx_pays(int pde, int kind, double pairs);
 bool fx_prepare(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, int ncols);
 // Y = alpha*(scale*A X + C X) + beta*Y, column-major X and Y (complex
 // interleaved).  A product whose densities or kernel values do not fit the
-// fixed-point form (not finite, or of extreme magnitude) leaves Y alone and
-// sets *fx_flag(ctx), which the caller's FP64 kernels then run on.
+// fixed-point form (not finite, of extreme magnitude, or of magnitudes that
+// differ so much within a row or column that an entry would come out worse
+// than an FP64 sum) leaves Y alone and sets *fx_flag(ctx), which the caller's
+// FP64 kernels then run on.
 void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_csr* corr, const double* x,
               int64_t ldx, double* y, int64_t ldy, int nrhs, const double* alpha, const double* beta);
 // Theta products S g1 - D g0 of the targets (out: m x ns complex, row-major)

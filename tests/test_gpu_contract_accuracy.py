@@ -204,22 +204,65 @@ def test_which_form_takes_a_density(pde, k, kind):
         assert np.array_equal(A @ X, _captured(A, X, c, s))
 
 
-def test_no_digit_product_is_missing(ctx):
-    """A sum of positive terms whose largest kernel value is about 2^5 times
-    the mean of n = 1,536: the reference is met to 8 roundings of a term and
-    what the dropped digits may take, n 2^-53.  One of the eight digit
-    products of the lowest kept order is worth 127 * 85 * 2^-70 per pair of the
-    two scales here (digits of 1/3), some 1e-12 of the sum."""
+def _scale(top):
+    """The power of two that takes top to (1.9, 3.8) 2^61: the splitting's unit is its inverse."""
+    m, e = np.frexp(top)
+    return 2.0 ** ((61 if 2 * m > 1.9 else 62) - (e - 1))
+
+
+@pytest.mark.parametrize("near,heavy", [(64, 64), (1024, 8), (8, 1024)])
+def test_no_digit_product_is_missing(ctx, near, heavy):
+    """1,534 equal terms, so that the digits of the products add up: sources on
+    a sphere about the first target, one of them `near` times closer and one of
+    `heavy` times the weight, which set the scales.  Each of the eight lowest
+    products that are kept is worth 9e-15 of the sum or more in one of the three
+    cases (8.8e-15 the least, computed from the digits in exact arithmetic).
+    Allowed: what is dropped and rounded, 2^65.2 units of the two scales per
+    term, and four roundings of a term, twice: 5.2e-15 to 6.4e-15 of the sum."""
     n = 1536
     r = np.random.default_rng(3)
     d = r.standard_normal((n, 3))
     d /= np.linalg.norm(d, axis=1, keepdims=True)
-    src = inti.Quadrature(d, d.copy(), np.full(n, 1.0 / 3.0), 0)
-    tgt = inti.points(np.concatenate([1.02 * d[:64], 1.5 * r.standard_normal((1400, 3))]))
+    y, w = 1.5 * d, np.full(n, 1.0 / 3.0)
+    y[9] /= near
+    w[700] *= heavy
+    src = inti.Quadrature(y, d, w, 0)
+    far = r.standard_normal((1400, 3))
+    far *= 4.0 / np.linalg.norm(far, axis=1, keepdims=True)
+    tgt = inti.points(np.concatenate([np.zeros((1, 3)), far]))
     A = operator("laplace", "SL", 0.0, tgt, src, ctx)
-    X = np.ones((n, 8))
-    X *= 2.0 ** np.arange(8)
+    X = np.ones((n, 8)) * 2.0 ** np.arange(8)
     Y = A @ X
-    rows = np.arange(0, 64)
-    ref, T, _ = reference("laplace", "SL", 0.0, tgt, rows, src, X)
-    assert (np.abs(Y[rows] - ref) <= (8 + n / 16) * 2.0**-53 * T).all()
+    ref, T, _ = reference("laplace", "SL", 0.0, tgt, np.arange(1), src, X)
+    K = 1.0 / np.linalg.norm(y, axis=1)
+    units = _scale(K.max()) * np.array([_scale(w.max() * c) for c in 2.0 ** np.arange(8)])
+    allow = n * 2.0**65.2 / units / (4 * np.pi) + 8 * 2.0**-53 * T[0]
+    assert (allow <= 7e-15 * T[0]).all()
+    assert (np.abs(Y[0] - ref[0]) <= allow).all(), np.abs(Y[0] - ref[0]) / T[0]
+
+
+@pytest.mark.parametrize("pde,k", [("laplace", 0.0), ("helmholtz", 4.0)])
+@pytest.mark.parametrize("derivative", [False, True])
+def test_theta_of_a_refined_surface(ctx, pde, k, derivative):
+    """The density interpolation of targets on a refined surface: with one
+    target more the product is large enough for the fixed-point form.  Its
+    kernel values and traces do not fit it, so every other row keeps the FP64
+    kernel's bits (rows are summed apart, in chunks that depend on the number
+    of 128-row blocks only); on a uniform surface the rows without derivative
+    change theirs."""
+    limit = 2e7 if k else 5e7
+    op = inti.Helmholtz(k=k, dim=3) if k else inti.Laplace(dim=3)
+    for q, same in ((graded_sphere(12, 9 if k else 13), True), (inti.p2_sphere_quadrature(10 if k else 14), False)):
+        n = len(q)
+        m = int(np.ceil(limit / n)) - 1
+        assert m < n and (m + 127) // 128 == (m + 128) // 128
+        pick = np.random.default_rng(2).permutation(n)
+        pick = np.concatenate([np.arange(n - 30, n), pick[pick < n - 30]])  # the refined corner first
+        rows = []
+        for count in (m, m + 1):
+            t = inti.Quadrature(q.coords[pick[:count]], q.normals[pick[:count]], np.ones(count), 0)
+            dS, dD = inti.bdim_correction(op, t, q, green_multiplier=-0.5, derivative=derivative, ctx=ctx)
+            rows.append([c.arrays()[2][: m * q.nq] for c in (dS, dD)])
+        equal = all(np.array_equal(a, b) for a, b in zip(*rows))
+        if same or not derivative:
+            assert equal == same
