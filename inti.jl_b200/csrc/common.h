@@ -116,6 +116,7 @@ struct FxStage {
 // kernel and its coefficients.
 struct FxPlan {
   DevBuf tables, records, tiles, least_normal, rowscale, meta;
+  DevBuf cut2, near_idx, near_val;  // sources taken apart (hypersingular kernels)
   const FxRows* rows = nullptr;  // in tables
   const FxStage* stages = nullptr;
   const FxItem* items = nullptr;

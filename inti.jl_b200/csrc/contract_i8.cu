@@ -26,8 +26,9 @@
 // sum of n terms, are left to the FP64 kernels: unit vectors, narrow bumps,
 // densities on one part of a surface, refined surfaces, targets close to a
 // surface.  With smooth densities on uniform meshes the single and double
-// layers and Theta lie 2^7 to 2^16 above the limit, the hypersingular kernel
-// mostly below it.  Far above, the result is closer to the exact product of the
+// layers and Theta lie 2^7 to 2^16 above the limit; the hypersingular kernel
+// lies 2^2 to 2^7 above it with the 40 nearest sources of a target taken apart
+// (fx_plan_near), and mostly below it without.  Far above, the result is closer to the exact product of the
 // FP64 kernel values than an FP64 accumulation, which rounds n times at 2^-53
 // of the running sum (64 columns, 13,872 nodes: 1.9e-15 from 64-bit values).  tests/test_gpu_contract_accuracy.py
 // holds each entry to these bounds in extended precision.
@@ -112,6 +113,7 @@ struct FxShape {
   static constexpr int J = FX_K / NA;        // sources per stage
   static constexpr int JT = J / 4;           // sources per generator thread and stage
   static constexpr bool tnormal = KIND == ADL || KIND == HS || KIND == FX_THETA_D;
+  static constexpr bool near = KIND == HS || KIND == FX_THETA_D;  // nearest sources apart (fx_plan_near)
   static constexpr int S_BYTES = J * FX_REC * 8;
   static constexpr int OFF_B = 2 * FX_A_BYTES;
   static constexpr int OFF_T = OFF_B + 2 * FX_B_BYTES;
@@ -150,19 +152,26 @@ __device__ __forceinline__ void fx_expi(double d, double kT, const double2* __re
   s = fma(sp, e.x, cp * e.y);
 }
 
+// The squared distance that decides which pairs are taken apart: rounded the
+// same way wherever it is asked for.
+__device__ __forceinline__ double fx_dist2(double r0, double r1, double r2) {
+  return __fma_rn(r2, r2, __fma_rn(r1, r1, __dmul_rn(r0, r0)));
+}
+
 // The NA values of one pair without the 1/(4 pi), times the row's scale p:
 // (Re, Im) of the kernel, Theta: the S value(s), then the D value(s).  nx is
 // the target normal times p.  rec = x y z nx ny nz of the
 // source; e^{ikd}(1/d - ik)(r.n)/d^2 is formed as e^{ikd}(Q - ik P) with
-// P = (r.n)/d^2, Q = P/d.
+// P = (r.n)/d^2, Q = P/d.  Pairs of a squared distance up to `cut` (bits; the
+// self pair's, or that of the sources taken apart) are zero.
 template <int PDE, int KIND>
 __device__ __forceinline__ void fx_values(const double (&x)[3], const double (&nx)[3], double pr,
                                           const double* __restrict__ rec, const FxConst& c, const double2* __restrict__ tab,
-                                          double (&v)[FxShape<PDE, KIND>::NA]) {
+                                          long long cut, double (&v)[FxShape<PDE, KIND>::NA]) {
   const double2 s01 = reinterpret_cast<const double2*>(rec)[0], s23 = reinterpret_cast<const double2*>(rec)[1];
   const double r0 = x[0] - s01.x, r1 = x[1] - s01.y, r2 = x[2] - s23.x;
-  const double d2 = fma(r2, r2, fma(r1, r1, r0 * r0));
-  const double ri = pair_keep(d2) ? rsqrt_fast(d2) : 0.0;  // self pair: every value 0
+  const double d2 = fx_dist2(r0, r1, r2);
+  const double ri = __double_as_longlong(d2) > cut ? rsqrt_fast(d2) : 0.0;  // every value 0
   double rny = 0.0, rnx = 0.0, nn = 0.0;
   if (KIND != SL) {
     const double2 s45 = reinterpret_cast<const double2*>(rec)[2];
@@ -382,6 +391,7 @@ struct FxArgs {
   const double* tcoords;
   const double* tnormals;
   const double* rowscale;   // per target
+  const double* cut2;       // per target, for kernels with sources apart
   const double* records;    // source records, J per stage
   const unsigned char* bdig;  // digit blocks, nc * 512 bytes per stage, one plane per CTA of a pair
   int nstages;                // stages of a plane
@@ -600,6 +610,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
           for (int c = 0; c < 3; ++c) nx[c] = a.tnormals[3 * row + c] * a.rowscale[row];
         }
         const double scale = a.rowscale[row];
+        const long long cut = __double_as_longlong(SH::near ? a.cut2[row] : kSamePointTol2);
         const double2* tab = reinterpret_cast<const double2*>(sm + SH::OFF_T) + (lane & (FX_REP - 1));
         for (uint32_t t = 0; t < T; ++t) {
           const uint32_t gg = g + t, sb = gg % FX_NS;
@@ -625,7 +636,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
             const double* Sg = S + ((q + g0) & (G - 1)) * (4 * FX_REC);
             double v[4][SH::NA];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) fx_values<PDE, KIND>(x, nx, scale, Sg + e * FX_REC, a.c, tab, v[e]);
+            for (int e = 0; e < 4; ++e) fx_values<PDE, KIND>(x, nx, scale, Sg + e * FX_REC, a.c, tab, cut, v[e]);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
 #pragma unroll
@@ -802,6 +813,162 @@ __device__ __forceinline__ double fx_modulus(double d, double id, double rnx, do
   return fx_max(f * rnx, h);
 }
 
+// The hypersingular kernel's nearest values, about 1/h^3, set a row's scale
+// while the entry may rest on values far smaller.  The sources about a target
+// are therefore taken apart: cut2 is a squared distance about the target, its
+// entries (pairs closer than that, up to kNear) are kept with their kernel
+// values, multiplied in FP64 (fx_near_add), and zero in the contraction.  The
+// rest of the row is then at most 1/(3.5h)^3: on spheres of 1,728 .. 13,872 and
+// ellipsoids of 1,944 .. 15,606 nodes the least sum of moduli of an entry rises
+// from 2^-13 .. 2^-5 of the two scales to 2^-5 .. 2^-1.  64 complex columns of
+// 13,872 nodes: 5.90 ms on the FP64 MMA path, 2.12 ms here; the derivative
+// correction of 43,200 nodes 34.0 and 17.4 ms.  Plan (once per operator, 0.1 ms
+// there) and entries (40 values per target) pay from the sizes of fx_pays.
+constexpr int kNear = 48;       // entries per target at most
+constexpr double kNearFill = 40.0 / kPi;  // cut2 / the nearest source's weight: some 40 of a surface's sources
+
+struct FxNear {
+  int32_t* count;    // per target
+  int32_t* idx;      // entry e of target r at e * estep + r * rstep
+  double* val;       // there times NV: (Re, Im) of the kernel, FX_THETA_D: of both
+  int64_t estep, rstep;
+};
+
+// One warp per target.
+template <int PDE, int KIND>
+__global__ void __launch_bounds__(256) fx_plan_near(int64_t m, int nstages, const FxStage* __restrict__ stages,
+                                                    const double4* __restrict__ tiles,
+                                                    const double* __restrict__ records,
+                                                    const double* __restrict__ tc, const double* __restrict__ tn,
+                                                    const double* __restrict__ weights, double k,
+                                                    double* __restrict__ cut2, FxNear near) {
+  using SH = FxShape<PDE, KIND>;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int64_t row = blockIdx.x * (int64_t)8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= m) return;
+  const double x0 = tc[3 * row], x1 = tc[3 * row + 1], x2 = tc[3 * row + 2];
+  auto better = [&](double& d, int& i) {  // the least over the warp, the first of equals
+    for (int o = 16; o > 0; o >>= 1) {
+      const double od = __shfl_xor_sync(kAll, d, o);
+      const int oi = __shfl_xor_sync(kAll, i, o);
+      if (od < d || (od == d && oi < i)) {
+        d = od;
+        i = oi;
+      }
+    }
+  };
+  auto source2 = [&](int s, int j) {
+    const double* y = records + ((int64_t)s * SH::J + j) * FX_REC;
+    return fx_dist2(x0 - y[0], x1 - y[1], x2 - y[2]);
+  };
+  double dn = INFINITY;
+  int at = 0;
+  for (int s = lane; s < nstages; s += 32) {
+    const double4 t = tiles[s];
+    const double d = fx_dist2(x0 - t.x, x1 - t.y, x2 - t.z);
+    if (d < dn) {
+      dn = d;
+      at = s;
+    }
+  }
+  better(dn, at);
+  double sn = INFINITY;
+  int js = 0;
+  for (int j = lane; j < stages[at].count; j += 32) {
+    const double d = source2(at, j);
+    if (d < sn) {
+      sn = d;
+      js = j;
+    }
+  }
+  better(sn, js);
+  double cut = kNearFill * weights[stages[at].src0 + js];
+  int total = 0;
+  // where more than kNear sources lie that close: a smaller distance, at last none
+  for (int attempt = 0;; ++attempt) {
+    if (!(cut > kSamePointTol2) || attempt == 8) {
+      cut = kSamePointTol2;
+      total = 0;
+      break;
+    }
+    total = 0;
+    const double r = sqrt(cut);
+    for (int b = 0; b < nstages; b += 32) {
+      bool want = false;
+      if (b + lane < nstages) {
+        const double4 t = tiles[b + lane];
+        const double rr = (r + t.w) * (1 + 1e-9);
+        want = fx_dist2(x0 - t.x, x1 - t.y, x2 - t.z) <= rr * rr;
+      }
+      for (unsigned w = __ballot_sync(kAll, want); w; w &= w - 1) {
+        const int s = b + __ffs(w) - 1, cnt = stages[s].count;
+        for (int j0 = 0; j0 < cnt; j0 += 32) {
+          const int j = j0 + lane;
+          bool take = false;
+          if (j < cnt) {
+            const double d2 = source2(s, j);
+            take = d2 > kSamePointTol2 && d2 <= cut;
+          }
+          const unsigned mask = __ballot_sync(kAll, take);
+          const int e = total + __popc(mask & ((1u << lane) - 1));
+          if (take && e < kNear) near.idx[e * near.estep + row * near.rstep] = (int32_t)(stages[s].src0 + j);
+          total += __popc(mask);
+        }
+      }
+    }
+    if (total <= kNear) break;
+    cut *= 0.8 * kNear / total;
+  }
+  if (lane == 0) {
+    cut2[row] = cut;
+    near.count[row] = total;
+  }
+}
+
+// Kernel values of the entries times the sources' weights, without the
+// 1/(4 pi).
+template <int PDE, int KIND>
+__global__ void fx_near_values(int64_t m, const double* __restrict__ tc, const double* __restrict__ tn,
+                               const double* __restrict__ sc, const double* __restrict__ sn,
+                               const double* __restrict__ weights, double k, FxNear near) {
+  using SH = FxShape<PDE, KIND>;
+  constexpr int NV = SH::NA;
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t row = SH::theta ? id / kNear : id % m;
+  const int e = (int)(SH::theta ? id % kNear : id / m);
+  if (row >= m || e >= kNear || e >= near.count[row]) return;
+  const int64_t o = e * near.estep + row * near.rstep;
+  const int64_t j = near.idx[o];
+  double r[3], d2 = 0.0, rnx = 0.0, rny = 0.0, nn = 0.0;
+  for (int c = 0; c < 3; ++c) {
+    const double nx = tn[3 * row + c], ny = sn[3 * j + c];
+    r[c] = tc[3 * row + c] - sc[3 * j + c];
+    d2 = fma(r[c], r[c], d2);
+    rnx = fma(r[c], nx, rnx);
+    rny = fma(r[c], ny, rny);
+    nn = fma(nx, ny, nn);
+  }
+  const double d = sqrt(d2), id1 = 1.0 / d, id2 = 1.0 / d2;
+  double* v = near.val + o * NV;
+  // e^{ikd} [(1/d - ik) p + (k^2 d^2 - 3 + 3ikd) q], p = nn/d^2, q = rnx rny/d^5
+  const double w = weights[j], p = w * (nn * id2), q = w * (rnx * rny * (id2 * id2 * id1)), a = -w * (rnx * id2);
+  if constexpr (PDE == LAPLACE) {
+    if (SH::theta) v[0] = a * id1;
+    v[NV - 1] = fma(-3.0, q, p * id1);
+  } else {
+    const double kd = k * d;
+    double s, c;
+    sincos(kd, &s, &c);
+    auto put = [&](double wr, double wi, double* o) {
+      o[0] = fma(c, wr, -s * wi);
+      o[1] = fma(c, wi, s * wr);
+    };
+    if (SH::theta) put(a * id1, -k * a, v);
+    put(fma(id1, p, fma(kd, kd, -3.0) * q), fma(-k, p, 3.0 * kd * q), v + NV - 2);
+  }
+}
+
 // Scale of each target row: a bound of its kernel values.  One warp per eight
 // consecutive rows, which lie close together: it takes the values of their
 // nearest tiles, then of every tile whose values may exceed one of the bounds
@@ -816,21 +983,21 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
                                                     const FxStage* __restrict__ stages,
                                                     const double4* __restrict__ tiles,
                                                     const double* __restrict__ records, FxConst c,
-                                                    double* __restrict__ rowscale,
+                                                    const double* __restrict__ cut2, double* __restrict__ rowscale,
                                                     unsigned long long* __restrict__ meta) {
   using SH = FxShape<PDE, KIND>;
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int JL = SH::J < 32 ? SH::J : 32;  // lanes along the sources of a tile
   constexpr int RP = 32 / JL;                  // rows per pass
   constexpr int NP = kPlanRows / RP;           // passes
-  __shared__ double sx[8][kPlanRows][8];       // x, n_x, |n_x| of a warp's rows
+  __shared__ double sx[8][kPlanRows][9];       // x, n_x, |n_x|, reach, cut2 of a warp's rows
   const int wid = blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (wid / (FX_M / kPlanRows) >= nrb) return;
   const FxRows rb = rows[wid / (FX_M / kPlanRows)];
   const int r0 = wid % (FX_M / kPlanRows) * kPlanRows;
   if (r0 >= rb.nrows) return;
   const double snorm = __longlong_as_double((long long)meta[0]);
-  double (*rx)[8] = sx[threadIdx.x >> 5];
+  double (*rx)[9] = sx[threadIdx.x >> 5];
   if (lane < kPlanRows) {
     const int64_t row = rb.row0 + min(r0 + lane, rb.nrows - 1);
     double n2 = 0.0;
@@ -841,6 +1008,7 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
       n2 += nq * nq;
     }
     rx[lane][6] = SH::tnormal ? sqrt(n2) : 1.0;
+    rx[lane][8] = SH::near ? cut2[row] : kSamePointTol2;
   }
   __syncwarp();
   auto centre2 = [&](int q, const double4& t) {  // squared distance of row q to the tile's centre
@@ -859,7 +1027,7 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
         const double* t = rx[RP * p + lane / JL];
         const double a = t[0] - y0, b = t[1] - y1, e = t[2] - y2;
         const double d2 = a * a + b * b + e * e;
-        if (!(d2 > 0.99 * kSamePointTol2)) continue;
+        if (!(d2 > 0.99 * t[8])) continue;
         const double id = rsqrt_fast(d2);
         const double rnx = fabs(a * t[3] + b * t[4] + e * t[5]), rny = fabs(a * n0 + b * n1 + e * n2);
         const double nn = fabs(t[3] * n0 + t[4] * n1 + t[5] * n2);
@@ -877,11 +1045,14 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
   };
   int last = -1;
   for (int q = 0; q < kPlanRows; ++q) {
+    // (the nearest one outside of the sources taken apart, which would give no bound)
     double dn = INFINITY;
     int near = s0;
+    const double inner = rx[q][8] > kSamePointTol2 ? sqrt(rx[q][8]) : -INFINITY;
     for (int s = s0 + lane; s < s1; s += 32) {
-      const double d = centre2(q, tiles[s]);
-      if (d < dn) {
+      const double4 t = tiles[s];
+      const double d = centre2(q, t), out = inner + t.w;
+      if (d < dn && (!SH::near || out < 0.0 || d > out * out)) {
         dn = d;
         near = s;
       }
@@ -1266,6 +1437,96 @@ __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const d
   }
 }
 
+// Y += alpha * (1/(4 pi)) * (sources taken apart) for four columns of a row,
+// four threads per row with a quarter of the entries each.  Bound by the
+// gathers of the densities (13,872 rows, 64 complex columns: 71 us of 2,115);
+// one thread per row left few in flight (1,728 rows 36 us, now 16).
+template <bool CPLX>
+__global__ void fx_near_add(int64_t m, FxNear near, const double* __restrict__ x, int64_t ldx, double* y, int64_t ldy,
+                            int c0, int ncol, double ar, double ai, const int* __restrict__ flag) {
+  constexpr int U = 4;
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, row = min(id / 4, m - 1);
+  const int f = blockIdx.y * U;
+  if (*flag) return;
+  double sr[U] = {}, si[U] = {};
+  const int cnt = near.count[row];
+  const double* xc[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) xc[u] = x + (int64_t)(c0 + min(f + u, ncol - 1)) * ldx * (CPLX ? 2 : 1);
+#pragma unroll 4
+  for (int e = id & 3; e < cnt; e += 4) {
+    const int64_t o = e * near.estep + row * near.rstep, j = near.idx[o];
+    const double2 v = CPLX ? reinterpret_cast<const double2*>(near.val)[o] : make_double2(near.val[o], 0.0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (CPLX) {
+        const double2 t = reinterpret_cast<const double2*>(xc[u])[j];
+        sr[u] = fma(v.x, t.x, fma(-v.y, t.y, sr[u]));
+        si[u] = fma(v.x, t.y, fma(v.y, t.x, si[u]));
+      } else {
+        sr[u] = fma(v.x, xc[u][j], sr[u]);
+      }
+    }
+  }
+  constexpr double kScale = 1.0 / (4 * kPi);
+  double vr = 0.0, vi = 0.0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {  // the row's sum of column u to its thread u
+    double r = sr[u], i = si[u];
+    for (int o = 2; o > 0; o >>= 1) {
+      r += __shfl_xor_sync(0xffffffffu, r, o);
+      if (CPLX) i += __shfl_xor_sync(0xffffffffu, i, o);
+    }
+    if ((id & 3) == u) {
+      vr = kScale * r;
+      vi = kScale * i;
+    }
+  }
+  const int c = f + (int)(id & 3);
+  if (id / 4 >= m || c >= ncol) return;
+  const int64_t q = (int64_t)(c0 + c) * ldy + row;
+  if (CPLX) {
+    double2* Y = reinterpret_cast<double2*>(y);
+    double2 t = Y[q];
+    t.x += ar * vr - ai * vi;
+    t.y += ar * vi + ai * vr;
+    Y[q] = t;
+  } else {
+    y[q] += ar * vr;
+  }
+}
+
+// The same for Theta: out[row, k] += 1/(4 pi) sum (ADL w g1 - HS w g0).
+template <bool CPLX>
+__global__ void fx_near_theta(int64_t m, int ns, FxNear near, const double2* __restrict__ g0,
+                              const double2* __restrict__ g1, double2* out, const int* __restrict__ flag) {
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, row = id / ns;
+  const int k = (int)(id - row * ns);
+  if (row >= m || *flag) return;
+  double sr = 0.0, si = 0.0;
+  const int cnt = near.count[row];
+#pragma unroll 8
+  for (int e = 0; e < cnt; ++e) {
+    const int64_t o = e * near.estep + row * near.rstep, j = near.idx[o];
+    const double2 a = g1[j * ns + k], b = g0[j * ns + k];
+    if (CPLX) {
+      const double2 s = reinterpret_cast<const double2*>(near.val)[2 * o], d = reinterpret_cast<const double2*>(near.val)[2 * o + 1];
+      sr = fma(s.x, a.x, fma(-s.y, a.y, sr));
+      si = fma(s.x, a.y, fma(s.y, a.x, si));
+      sr = fma(-d.x, b.x, fma(d.y, b.y, sr));
+      si = fma(-d.x, b.y, fma(-d.y, b.x, si));
+    } else {
+      sr = fma(near.val[2 * o], a.x, sr);
+      sr = fma(-near.val[2 * o + 1], b.x, sr);
+    }
+  }
+  constexpr double kScale = 1.0 / (4 * kPi);
+  double2 v = out[id];
+  v.x = fma(kScale, sr, v.x);
+  v.y = fma(kScale, si, v.y);
+  out[id] = v;
+}
+
 // Theta: column bounds over the traces (both arrays share a column's scale,
 // since their products share the accumulators) and the masses of g1 and g0.
 // One thread per (stage, column).
@@ -1517,9 +1778,13 @@ const int* fx_flag(const inti_ctx* ctx) { return ctx->fx.work.as<int>(); }
 // columns at 1,200 nodes take 123 us either way, at 1,728 nodes 170 us against
 // 64 us here (64 columns 407 against 125 us).  Theta pays for its plan (row
 // bounds, work lists) every time, about 0.1 ms: real values break even near
-// 5e7 pairs (7,000 nodes), complex ones near 2e7.
+// 5e7 pairs (7,000 nodes), complex ones near 2e7.  The derivative form adds the
+// sources taken apart: real values 0.78 against 0.81 ms at 9,408 nodes and
+// 1.22 against 1.08 at 12,288, complex ones 0.59 against 0.72 at 4,800 and 1.03
+// against 0.97 at 6,912.
 bool fx_pays(int pde, int kind, double pairs) {
   if (kind < FX_THETA) return pairs >= 2e6;
+  if (kind == FX_THETA_D) return pairs >= (pde == HELMHOLTZ ? 4e7 : 1.2e8);
   return pairs >= (pde == HELMHOLTZ ? 2e7 : 5e7);
 }
 
@@ -1544,6 +1809,19 @@ static FxPass fx_pass(int left, int comps) {
 constexpr int FX_COUNTERS = 64;
 static size_t fx_work_bytes(const FxProblem& p, int nsurf, int ncols) {
   return sizeof(int) * FX_COUNTERS + sizeof(long long) * (size_t)nsurf * ncols * (p.pde == HELMHOLTZ ? 3 : 2);
+}
+
+// Kernels with sources taken apart (of one surface: the first target is 0).
+static bool fx_near_kind(int kind) { return kind == HS || kind == FX_THETA_D; }
+static FxNear fx_near(const FxProblem& p, const FxPlan& plan) {
+  const int64_t m = plan.ntargets;
+  FxNear n;
+  n.count = plan.near_idx.as<int32_t>();
+  n.idx = n.count + m;
+  n.val = plan.near_val.as<double>();
+  n.estep = p.kind == HS ? m : 1;  // threads run along the rows, of Theta along a row's columns
+  n.rstep = p.kind == HS ? 1 : kNear;
+  return n;
 }
 
 static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
@@ -1600,15 +1878,30 @@ static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
   plan.least_normal.ensure(sizeof(double) * stages.size());
   plan.rowscale.ensure(sizeof(double) * std::max<int64_t>(plan.ntargets, 1));
   plan.meta.ensure(sizeof(unsigned long long) * 2);
+  if (fx_near_kind(p.kind)) {
+    plan.cut2.ensure(sizeof(double) * plan.ntargets);
+    plan.near_idx.ensure(sizeof(int32_t) * plan.ntargets * (1 + kNear));
+    plan.near_val.ensure(sizeof(double) * plan.ntargets * kNear * fx_na(p.pde, p.kind));
+  }
   INTI_CUDA(cudaMemsetAsync(plan.meta.p, 0, sizeof(unsigned long long) * 2, ctx->stream));
   fx_plan_sources<<<(plan.nstages + 7) / 8, 256, 0, ctx->stream>>>(
       plan.nstages, J, plan.stages, p.coords, p.normals, plan.records.as<double>(),
       plan.tiles.as<double4>(), plan.least_normal.as<double>(), plan.meta.as<unsigned long long>());
   fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
     constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
+    if constexpr (FxShape<P, K>::near) {
+      const int64_t m = plan.ntargets;
+      fx_plan_near<P, K><<<(unsigned)((m + 7) / 8), 256, 0, ctx->stream>>>(
+          m, plan.nstages, plan.stages, plan.tiles.as<double4>(), plan.records.as<double>(), p.tcoords, p.tnormals,
+          p.weights, p.k, plan.cut2.as<double>(), fx_near(p, plan));
+      fx_near_values<P, K><<<(unsigned)((m * kNear + 255) / 256), 256, 0, ctx->stream>>>(
+          m, p.tcoords, p.tnormals, p.coords, p.normals, p.weights, p.k, fx_near(p, plan));
+      ctx->launches += 2;
+    }
     fx_plan_rows<P, K><<<(unsigned)plan.nrows * (FX_M / kPlanRows / 8), 256, 0, ctx->stream>>>(
         plan.nrows, plan.rows, p.tcoords, p.tnormals, plan.stages, plan.tiles.as<double4>(),
-        plan.records.as<double>(), fx_const(p), plan.rowscale.as<double>(), plan.meta.as<unsigned long long>());
+        plan.records.as<double>(), fx_const(p), plan.cut2.as<double>(), plan.rowscale.as<double>(),
+        plan.meta.as<unsigned long long>());
     INTI_CUDA(cudaFuncSetAttribute(fx_contract_kernel<P, K, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    FxShape<P, K>::SMEM));
     if constexpr (!FxShape<P, K>::theta)
@@ -1686,6 +1979,7 @@ static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc
   a.tcoords = p.tcoords;
   a.tnormals = p.tnormals;
   a.rowscale = plan.rowscale.as<double>();
+  a.cut2 = plan.cut2.as<double>();
   a.records = plan.records.as<double>();
   a.bdig = ctx->fx.bdig.as<unsigned char>();
   a.nstages = plan.nstages;
@@ -1776,6 +2070,11 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
       o.beta_zero = o.br == 0.0 && o.bi == 0.0;
       fx_finish<C><<<dim3(plan.nrows, w.cols), FX_M, 0, ctx->stream>>>(o);
       ctx->launches++;
+      if (fx_near_kind(p.kind)) {
+        fx_near_add<C><<<dim3((unsigned)((plan.ntargets + 31) / 32), (unsigned)((w.cols + 3) / 4)), 128, 0,
+                         ctx->stream>>>(plan.ntargets, fx_near(p, plan), x, ldx, y, ldy, c0, w.cols, o.ar, o.ai, flag);
+        ctx->launches++;
+      }
     }
   };
   if (cplx)
@@ -1805,6 +2104,12 @@ void fx_theta(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const doubl
     fx_theta_finish<C><<<dim3(plan.nrows, ns), FX_M, 0, ctx->stream>>>(
         plan.rows, ctx->fx.partial.as<double>(), plan.rowscale.as<double>(), colmax,
         fx_digits_ptr(ctx, plan, ns), ns, nc, flag, out);
+    if (fx_near_kind(p.kind)) {
+      const int64_t m = plan.ntargets;
+      fx_near_theta<C><<<(unsigned)((m * ns + 127) / 128), 128, 0, ctx->stream>>>(m, ns, fx_near(p, plan), g0, g1, out,
+                                                                                flag);
+      ctx->launches++;
+    }
   };
   if (cplx)
     by_type(std::true_type());

@@ -171,6 +171,26 @@ def test_close_to_a_surface(ctx, pde, k, kind, off):
         check(A, pde, kind, k, tgt, q, columns(q, family, bool(k)), rows)
 
 
+@pytest.mark.parametrize("pde,k", [("laplace", 0.0), ("helmholtz", 4.0)])
+@pytest.mark.parametrize("nrhs", [8, 37])
+def test_sources_taken_apart(ctx, pde, k, nrhs):
+    """The hypersingular kernel's nearest sources where they are not the 40 of
+    a smooth surface: 300 nodes of ordinary weight within 0.02 (more than a
+    target keeps), 60 on one point, weights of zero and below it."""
+    q = inti.p2_sphere_quadrature(7)
+    r = np.random.default_rng(8)
+    y = np.concatenate([q.coords, q.coords[100] + 0.02 * r.random((300, 3)), np.repeat(q.coords[900:901], 60, axis=0)])
+    w = np.concatenate([q.weights, np.full(360, q.weights.mean())])
+    w[200:260] = 0.0
+    w[300:360] *= -1.0
+    src = inti.Quadrature(y, y / np.linalg.norm(y, axis=1, keepdims=True), w, 0)
+    A = operator(pde, "HS", k, src, src, ctx)
+    rows = np.concatenate([np.arange(90, 110), np.arange(195, 365, 10), [900, 901, 2000], np.arange(2352, 2652, 30), [2700]])
+    X = np.tile(columns(src, "smooth", bool(k)), (1, 5))[:, :nrhs]
+    check(A, pde, "HS", k, src, src, X, rows)
+    check(A, pde, "HS", k, src, src, columns(src, "unit", bool(k)), rows)
+
+
 def _captured(A, X, c, s):
     """The product in a captured graph, which keeps the FP64 MMA kernel."""
     x = torch.from_numpy(X.T.copy()).cuda()
@@ -187,7 +207,7 @@ def _captured(A, X, c, s):
 
 
 @pytest.mark.parametrize("pde,k", [("laplace", 0.0), ("helmholtz", 4.0)])
-@pytest.mark.parametrize("kind", ["SL", "DL", "ADL"])
+@pytest.mark.parametrize("kind", ["SL", "DL", "ADL", "HS"])
 def test_which_form_takes_a_density(pde, k, kind):
     """Smooth densities keep the fixed-point form (other last bits than the
     FP64 MMA kernel), unit vectors and an otherwise smooth block with one
@@ -248,11 +268,11 @@ def test_theta_of_a_refined_surface(ctx, pde, k, derivative):
     target more the product is large enough for the fixed-point form.  Its
     kernel values and traces do not fit it, so every other row keeps the FP64
     kernel's bits (rows are summed apart, in chunks that depend on the number
-    of 128-row blocks only); on a uniform surface the rows without derivative
-    change theirs."""
-    limit = 2e7 if k else 5e7
+    of 128-row blocks only); on a uniform surface the rows change theirs."""
+    limit = {(False, False): 5e7, (False, True): 2e7, (True, False): 1.2e8, (True, True): 4e7}[derivative, bool(k)]
     op = inti.Helmholtz(k=k, dim=3) if k else inti.Laplace(dim=3)
-    for q, same in ((graded_sphere(12, 9 if k else 13), True), (inti.p2_sphere_quadrature(10 if k else 14), False)):
+    cells, nsub = {5e7: (13, 14), 2e7: (9, 10), 1.2e8: (17, 17), 4e7: (11, 12)}[limit]
+    for q, same in ((graded_sphere(12, cells), True), (inti.p2_sphere_quadrature(nsub), False)):
         n = len(q)
         m = int(np.ceil(limit / n)) - 1
         assert m < n and (m + 127) // 128 == (m + 128) // 128
@@ -264,5 +284,4 @@ def test_theta_of_a_refined_surface(ctx, pde, k, derivative):
             dS, dD = inti.bdim_correction(op, t, q, green_multiplier=-0.5, derivative=derivative, ctx=ctx)
             rows.append([c.arrays()[2][: m * q.nq] for c in (dS, dD)])
         equal = all(np.array_equal(a, b) for a, b in zip(*rows))
-        if same or not derivative:
-            assert equal == same
+        assert equal == same
