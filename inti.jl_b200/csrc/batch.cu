@@ -538,7 +538,9 @@ static void mrhs_mma_launch(inti_ctx* ctx, int pde, int kind, const BatchArgs& a
 // densities that do not fit it; else on the FP64 MMA kernel.
 static void mrhs_fp64(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, const inti_csr* corr, BatchArgs& a,
                       double pairs, int64_t blocks) {
-  if (fx_pays(p.pde, p.kind, pairs) && fx_prepare(ctx, p, plan, a.nrhs)) {
+  double targets = 0.0;
+  for (int64_t n : p.nrow) targets += (double)n;
+  if (fx_pays(p.pde, p.kind, targets, pairs) && fx_prepare(ctx, p, plan, a.nrhs)) {
     const double alpha[2] = {a.ar, a.ai}, beta[2] = {a.br, a.bi};
     fx_apply(ctx, p, plan, corr, a.x, a.ldx, a.y, a.ldy, a.nrhs, alpha, beta);
     a.only_if = fx_flag(ctx);

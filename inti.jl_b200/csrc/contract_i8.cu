@@ -1781,10 +1781,20 @@ const int* fx_flag(const inti_ctx* ctx) { return ctx->fx.work.as<int>(); }
 // 5e7 pairs (7,000 nodes), complex ones near 2e7.  The derivative form adds the
 // sources taken apart: real values 0.78 against 0.81 ms at 9,408 nodes and
 // 1.22 against 1.08 at 12,288, complex ones 0.59 against 0.72 at 4,800 and 1.03
-// against 0.97 at 6,912.
-bool fx_pays(int pde, int kind, double pairs) {
-  if (kind < FX_THETA) return pairs >= 2e6;
-  if (kind == FX_THETA_D) return pairs >= (pde == HELMHOLTZ ? 4e7 : 1.2e8);
+// against 0.97 at 6,912; 2,352 x 20,000 complex 2.39 against 2.54 (4,800 sources
+// 3.01 against 2.95).
+// Few sources leave little of an item next to its hand-over (and a surface's
+// last stage partly empty), while the FP64 MMA kernel's blocks are short then.
+// Ratio of its time to the time here, 8 and 64 columns, sources x targets:
+// Laplace SL 256 x 16,000 0.59 and 0.70, 512 x 8,000 0.73 and 0.76, 768 x 8,000
+// 0.77 and 0.84, 1,024 x 8,000 0.98 and 1.09, 1,024 x 2,000 1.15 and 1.37, 2,048
+// x 8,000 1.34 and 1.42; batches of surfaces of 216 nodes 0.63 .. 0.91, 486
+// nodes 0.87 .. 1.40, 864 nodes 1.31 .. 2.12.  With sources taken apart: HS
+// 1,024 x 8,000 0.76 and 0.85, 1,500 x 8,000 0.88 and 1.01, 1,452 x 1,452 1.12
+// and 1.42.
+bool fx_pays(int pde, int kind, double targets, double pairs) {
+  if (kind < FX_THETA) return pairs >= 2e6 && pairs >= (kind == HS ? 1400.0 : 850.0) * targets;
+  if (kind == FX_THETA_D) return pairs >= (pde == HELMHOLTZ ? 4e7 : 1.2e8) && pairs >= 5000.0 * targets;
   return pairs >= (pde == HELMHOLTZ ? 2e7 : 5e7);
 }
 

@@ -27,9 +27,9 @@ struct FxProblem {
   std::vector<int64_t> row, nrow, src, nsrc;
 };
 
-// Whether the contraction is the faster form for a product of this many pairs
-// (per column, summed over the surfaces).
-bool fx_pays(int pde, int kind, double pairs);
+// Whether the contraction is the faster form for a product of this many targets
+// and pairs (per column, summed over the surfaces).
+bool fx_pays(int pde, int kind, double targets, double pairs);
 // Builds the plan and sizes the buffers of a product of `ncols` columns.
 // False when there is no memory for them, and while the context's stream is
 // being captured: a graph would keep the addresses of buffers that the

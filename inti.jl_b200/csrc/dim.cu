@@ -788,7 +788,7 @@ static void dim_theta_run(inti_ctx* ctx, int pde, double k_re, const inti_quad* 
         fp.nsrc = {n};
         FxPlan& plan = ctx->dimwork.plan;
         plan.ready = false;  // another geometry
-        if (fx_pays(P, fp.kind, (double)m * (double)n) && fx_prepare(ctx, fp, plan, ns)) {
+        if (fx_pays(P, fp.kind, (double)m, (double)m * (double)n) && fx_prepare(ctx, fp, plan, ns)) {
           fx_theta(ctx, fp, plan, wk.g0.as<double2>(), wk.g1.as<double2>(), ns, wk.part.as<double2>());
           only_if = fx_flag(ctx);
         }

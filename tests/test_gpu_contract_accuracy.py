@@ -194,7 +194,8 @@ def test_sources_taken_apart(ctx, pde, k, nrhs):
 def _captured(A, X, c, s):
     """The product in a captured graph, which keeps the FP64 MMA kernel."""
     x = torch.from_numpy(X.T.copy()).cuda()
-    y = torch.zeros_like(x)
+    assert x.shape[1] == A.shape[1]
+    y = torch.zeros((x.shape[0], A.shape[0]), dtype=x.dtype, device="cuda")
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g, stream=s):
@@ -222,6 +223,22 @@ def test_which_form_takes_a_density(pde, k, kind):
     assert not np.array_equal(A @ smooth, _captured(A, smooth, c, s))
     for X in (unit, mixed):
         assert np.array_equal(A @ X, _captured(A, X, c, s))
+
+
+@pytest.mark.parametrize("kind,n,apart", [("SL", 512, True), ("SL", 1024, False), ("HS", 1024, True), ("HS", 1728, False)])
+def test_few_sources_keep_the_fp64_kernel(ctx, kind, n, apart):
+    """8,000 targets: with few sources the FP64 MMA kernel is the faster form
+    (its bits), with more the contraction."""
+    s = torch.cuda.Stream()
+    c = inti.Context(0, stream=s.cuda_stream)
+    full = inti.p2_sphere_quadrature(6)
+    pick = np.linspace(0, len(full) - 1, n).astype(int)
+    q = inti.Quadrature(full.coords[pick], full.normals[pick], full.weights[pick], 0)
+    d = np.random.default_rng(4).standard_normal((8000, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    A = operator("laplace", kind, 0.0, inti.Quadrature(1.4 * d, d, np.ones(8000), 0), q, c)
+    X = columns(q, "smooth", False)
+    assert np.array_equal(A @ X, _captured(A, X, c, s)) == apart
 
 
 def _scale(top):
