@@ -237,6 +237,13 @@ class HyperSingularKernel(_Kernel):
 # ----------------------------------------------------------------------------
 # device handles
 # ----------------------------------------------------------------------------
+def _release(destroy, handle, ctx) -> None:
+    """Finalizer of a handle.  Its arguments hold the context, so that the
+    context is destroyed after every handle also where the garbage collector
+    finds them in one cycle, whose finalizers run in any order."""
+    destroy(handle)
+
+
 def _quad_handle(q: Quadrature, ctx: Context):
     """Device copy of a quadrature, cached on the object per context."""
     cache = q.__dict__.setdefault("_b200", {})
@@ -247,7 +254,7 @@ def _quad_handle(q: Quadrature, ctx: Context):
     nrm = q.normals
     ctx.check(ctx.lib.inti_quad_create(ctx.handle, q.dim, len(q), L.dptr(q.coords), L.dptr(nrm),
                                        L.dptr(q.weights), int(q.nq), C.byref(h)))
-    fin = weakref.finalize(q, ctx.lib.inti_quad_destroy, h)
+    fin = weakref.finalize(q, _release, ctx.lib.inti_quad_destroy, h, ctx)
     cache[key] = (h, fin, ctx)
     return h
 
@@ -275,7 +282,7 @@ class CorrectionMatrix:
         self.shape = (m.value, n.value)
         self.nnz = nnz.value
         self.dtype = np.complex128 if dt.value == L.C128 else np.float64
-        self._fin = weakref.finalize(self, ctx.lib.inti_csr_destroy, handle)
+        self._fin = weakref.finalize(self, _release, ctx.lib.inti_csr_destroy, handle, ctx)
 
     @classmethod
     def from_csr(cls, indptr, indices, data, shape, ctx: Context | None = None):
@@ -484,7 +491,7 @@ class GpuOperator(_Map):
                                                    correction.handle if correction else None, prec,
                                                    C.byref(h)))
         self.handle = h
-        self._fin = weakref.finalize(self, self.ctx.lib.inti_op_destroy, h)
+        self._fin = weakref.finalize(self, _release, self.ctx.lib.inti_op_destroy, h, self.ctx)
         self.shape = (len(target), len(source))
         self.is_complex = op.pde == L.HELMHOLTZ
         self.dtype = np.complex128 if self.is_complex else np.float64
@@ -608,7 +615,7 @@ class CombinedFieldOperator(GpuOperator):
             S.correction.handle if S.correction else None, L.cpair(c_D), L.cpair(c_S), prec, C.byref(h)))
         self.handle = h
         self._keep = (D, S)
-        self._fin = weakref.finalize(self, self.ctx.lib.inti_op_destroy, h)
+        self._fin = weakref.finalize(self, _release, self.ctx.lib.inti_op_destroy, h, self.ctx)
         self.shape = D.shape
         self.is_complex = D.is_complex
         self.dtype = D.dtype
@@ -643,7 +650,7 @@ class BatchOperator:
                                                       C.byref(h)))
         self.handle = h
         self._keep = (corrections,)
-        self._fin = weakref.finalize(self, self.ctx.lib.inti_batch_destroy, h)
+        self._fin = weakref.finalize(self, _release, self.ctx.lib.inti_batch_destroy, h, self.ctx)
         self.n = int(self.ctx.lib.inti_batch_size(h))
         self.offsets = np.cumsum([0] + [len(q) for q in self.quads])
         self.is_complex = op.pde == L.HELMHOLTZ
