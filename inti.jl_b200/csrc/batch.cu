@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mrhs_mma(BatchArgs a) {
   constexpr int XPER = MS::XPER;
   static_assert(Sh::MT == 64 && kMmaThreads % Sh::MT == 0 && kMmaJ % (kMmaThreads / Sh::MT) == 0, "shape");
   extern __shared__ __align__(16) double smem_d[];
+  pdl_wait();
   if (a.only_if && !*a.only_if) return;
   double* As = smem_d;
   double* Bs = As + Sh::MT * Sh::LDA;
@@ -337,6 +338,7 @@ template <bool CPLX>
 __global__ void csr_mrhs(int64_t m, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                         const double* __restrict__ val, const double* __restrict__ x, int64_t ldx, double* y,
                         int64_t ldy, int nrhs, double ar, double ai, const int* only_if) {
+  pdl_wait();
   if (only_if && !*only_if) return;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int c0 = blockIdx.y * kCsrCols;
@@ -507,7 +509,10 @@ static void mrhs_mma_launch(inti_ctx* ctx, int pde, int kind, const BatchArgs& a
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       });
       const dim3 grid((unsigned)(2 * blocks), (unsigned)((a.nrhs + RHS - 1) / RHS));
-      kern<<<grid, kMmaThreads, smem, ctx->stream>>>(a);
+      if (a.only_if)  // the last of a chain of small kernels
+        launch_pdl(ctx->stream, grid, kMmaThreads, smem, kern, a);
+      else
+        kern<<<grid, kMmaThreads, smem, ctx->stream>>>(a);
     };
     if (a.nrhs <= narrow)
       launch(std::integral_constant<int, narrow>());
@@ -537,10 +542,8 @@ static void mrhs_mma_launch(inti_ctx* ctx, int pde, int kind, const BatchArgs& a
 // (the correction rows included), with the FP64 MMA kernel standing by for
 // densities that do not fit it; else on the FP64 MMA kernel.
 static void mrhs_fp64(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, const inti_csr* corr, BatchArgs& a,
-                      double pairs, int64_t blocks) {
-  double targets = 0.0;
-  for (int64_t n : p.nrow) targets += (double)n;
-  if (fx_pays(p.pde, p.kind, targets, pairs) && fx_prepare(ctx, p, plan, a.nrhs)) {
+                      bool pays, int64_t blocks) {
+  if (pays && fx_prepare(ctx, p, plan, a.nrhs)) {
     const double alpha[2] = {a.ar, a.ai}, beta[2] = {a.br, a.bi};
     fx_apply(ctx, p, plan, corr, a.x, a.ldx, a.y, a.ldy, a.nrhs, alpha, beta);
     a.only_if = fx_flag(ctx);
@@ -592,15 +595,17 @@ void batch_apply_device(inti_batch* b, int precision, const double* x, int64_t l
     p.tnormals = p.normals = a.normals;
     p.weights = a.weights;
     double pairs = 0.0;
-    for (size_t s = 0; s + 1 < b->off.size(); ++s) {
-      const int64_t ns = b->off[s + 1] - b->off[s];
-      p.row.push_back(b->off[s]);
-      p.src.push_back(b->off[s]);
-      p.nrow.push_back(ns);
-      p.nsrc.push_back(ns);
-      pairs += (double)ns * (double)ns;
-    }
-    mrhs_fp64(ctx, p, b->fx, b->corr.get(), a, pairs, b->nitems);
+    for (size_t s = 0; s + 1 < b->off.size(); ++s) pairs += std::pow((double)(b->off[s + 1] - b->off[s]), 2);
+    const bool pays = fx_pays(p.pde, p.kind, (double)b->off.back(), pairs);
+    if (pays && !b->fx.ready)  // the plan's lists
+      for (size_t s = 0; s + 1 < b->off.size(); ++s) {
+        const int64_t ns = b->off[s + 1] - b->off[s];
+        p.row.push_back(b->off[s]);
+        p.src.push_back(b->off[s]);
+        p.nrow.push_back(ns);
+        p.nsrc.push_back(ns);
+      }
+    mrhs_fp64(ctx, p, b->fx, b->corr.get(), a, pays, b->nitems);
   } else {
     throw Error(INTI_E_ARG, "batch precision must be FP64 or TF32");
   }
@@ -609,11 +614,11 @@ void batch_apply_device(inti_batch* b, int precision, const double* x, int64_t l
     const int64_t m = b->off.back();
     dim3 grid((unsigned)((m + 255) / 256), (unsigned)((nrhs + kCsrCols - 1) / kCsrCols));
     if (cplx)
-      csr_mrhs<true><<<grid, 256, 0, ctx->stream>>>(m, b->corr->rowptr.as<int64_t>(), b->corr->col.as<int32_t>(),
-                                                    b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
+      launch_pdl(ctx->stream, grid, 256, 0, &csr_mrhs<true>, m, b->corr->rowptr.as<int64_t>(),
+                 b->corr->col.as<int32_t>(), b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     else
-      csr_mrhs<false><<<grid, 256, 0, ctx->stream>>>(m, b->corr->rowptr.as<int64_t>(), b->corr->col.as<int32_t>(),
-                                                     b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
+      launch_pdl(ctx->stream, grid, 256, 0, &csr_mrhs<false>, m, b->corr->rowptr.as<int64_t>(),
+                 b->corr->col.as<int32_t>(), b->corr->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     ctx->launches++;
     INTI_CUDA(cudaGetLastError());
   }
@@ -674,17 +679,17 @@ void op_apply_mrhs(inti_op* op, const double* x, int64_t ldx, double* y, int64_t
     p.row = p.src = {0};
     p.nrow = {a.gm};
     p.nsrc = {a.gn};
-    mrhs_fp64(ctx, p, op->fx, op->corr, a, (double)a.gm * (double)a.gn, blocks);
+    mrhs_fp64(ctx, p, op->fx, op->corr, a, fx_pays(p.pde, p.kind, (double)a.gm, (double)a.gm * (double)a.gn), blocks);
   }
   if (op->corr) {
     const inti_csr* c = op->corr;
     dim3 grid((unsigned)((a.gm + 255) / 256), (unsigned)((nrhs + kCsrCols - 1) / kCsrCols));
     if (cplx)
-      csr_mrhs<true><<<grid, 256, 0, ctx->stream>>>(a.gm, c->rowptr.as<int64_t>(), c->col.as<int32_t>(),
-                                                    c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
+      launch_pdl(ctx->stream, grid, 256, 0, &csr_mrhs<true>, a.gm, c->rowptr.as<int64_t>(), c->col.as<int32_t>(),
+                 c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     else
-      csr_mrhs<false><<<grid, 256, 0, ctx->stream>>>(a.gm, c->rowptr.as<int64_t>(), c->col.as<int32_t>(),
-                                                     c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
+      launch_pdl(ctx->stream, grid, 256, 0, &csr_mrhs<false>, a.gm, c->rowptr.as<int64_t>(), c->col.as<int32_t>(),
+                 c->val.as<double>(), x, ldx, y, ldy, nrhs, a.ar, a.ai, a.only_if);
     ctx->launches++;
     INTI_CUDA(cudaGetLastError());
   }

@@ -449,6 +449,7 @@ __device__ __forceinline__ double fx_sum(const int32_t (&d)[FX_D][4], int e) {
 // the peer's shared memory were twice as slow as evaluating everything twice.)
 template <int PDE, int KIND, int CL>
 __global__ void __launch_bounds__(FX_THREADS, 1) fx_contract_kernel(FxArgs a) {
+  pdl_wait();
   using SH = FxShape<PDE, KIND>;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t fullS[FX_NS], fullB[2], aReady[2], aFull[2], aPeer[2], mmaDone[FX_ND], drainBar;
@@ -834,12 +835,47 @@ struct FxNear {
   int64_t estep, rstep;
 };
 
+// Kernel values of one entry times the source's weight, without the 1/(4 pi):
+// e^{ikd} [(1/d - ik) p + (k^2 d^2 - 3 + 3ikd) q], p = nn/d^2, q = rnx rny/d^5.
+template <int PDE, int KIND>
+__device__ __forceinline__ void fx_near_values(const double (&x)[3], const double (&nx)[3], const double* __restrict__ y,
+                                               const double* __restrict__ ny, double w, double k, double* v) {
+  constexpr bool TH = FxShape<PDE, KIND>::theta;
+  constexpr int NV = FxShape<PDE, KIND>::NA;
+  double d2 = 0.0, rnx = 0.0, rny = 0.0, nn = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double r = x[c] - y[c], n = ny[c];
+    d2 = fma(r, r, d2);
+    rnx = fma(r, nx[c], rnx);
+    rny = fma(r, n, rny);
+    nn = fma(nx[c], n, nn);
+  }
+  const double d = sqrt(d2), id1 = 1.0 / d, id2 = 1.0 / d2;
+  const double p = w * (nn * id2), q = w * (rnx * rny * (id2 * id2 * id1)), a = -w * (rnx * id2);
+  if constexpr (PDE == LAPLACE) {
+    if (TH) v[0] = a * id1;
+    v[NV - 1] = fma(-3.0, q, p * id1);
+  } else {
+    const double kd = k * d;
+    double s, c;
+    sincos(kd, &s, &c);
+    auto put = [&](double wr, double wi, double* o) {
+      o[0] = fma(c, wr, -s * wi);
+      o[1] = fma(c, wi, s * wr);
+    };
+    if (TH) put(a * id1, -k * a, v);
+    put(fma(id1, p, fma(kd, kd, -3.0) * q), fma(-k, p, 3.0 * kd * q), v + NV - 2);
+  }
+}
+
 // One warp per target.
 template <int PDE, int KIND>
 __global__ void __launch_bounds__(256) fx_plan_near(int64_t m, int nstages, const FxStage* __restrict__ stages,
                                                     const double4* __restrict__ tiles,
                                                     const double* __restrict__ records,
                                                     const double* __restrict__ tc, const double* __restrict__ tn,
+                                                    const double* __restrict__ sc, const double* __restrict__ sn,
                                                     const double* __restrict__ weights, double k,
                                                     double* __restrict__ cut2, FxNear near) {
   using SH = FxShape<PDE, KIND>;
@@ -864,6 +900,7 @@ __global__ void __launch_bounds__(256) fx_plan_near(int64_t m, int nstages, cons
   };
   double dn = INFINITY;
   int at = 0;
+#pragma unroll 4
   for (int s = lane; s < nstages; s += 32) {
     const double4 t = tiles[s];
     const double d = fx_dist2(x0 - t.x, x1 - t.y, x2 - t.z);
@@ -873,16 +910,16 @@ __global__ void __launch_bounds__(256) fx_plan_near(int64_t m, int nstages, cons
     }
   }
   better(dn, at);
-  double sn = INFINITY;
+  double ds = INFINITY;
   int js = 0;
   for (int j = lane; j < stages[at].count; j += 32) {
     const double d = source2(at, j);
-    if (d < sn) {
-      sn = d;
+    if (d < ds) {
+      ds = d;
       js = j;
     }
   }
-  better(sn, js);
+  better(ds, js);
   double cut = kNearFill * weights[stages[at].src0 + js];
   int total = 0;
   // where more than kNear sources lie that close: a smaller distance, at last none
@@ -894,6 +931,7 @@ __global__ void __launch_bounds__(256) fx_plan_near(int64_t m, int nstages, cons
     }
     total = 0;
     const double r = sqrt(cut);
+#pragma unroll 4
     for (int b = 0; b < nstages; b += 32) {
       bool want = false;
       if (b + lane < nstages) {
@@ -924,58 +962,23 @@ __global__ void __launch_bounds__(256) fx_plan_near(int64_t m, int nstages, cons
     cut2[row] = cut;
     near.count[row] = total;
   }
-}
-
-// Kernel values of the entries times the sources' weights, without the
-// 1/(4 pi).
-template <int PDE, int KIND>
-__global__ void fx_near_values(int64_t m, const double* __restrict__ tc, const double* __restrict__ tn,
-                               const double* __restrict__ sc, const double* __restrict__ sn,
-                               const double* __restrict__ weights, double k, FxNear near) {
-  using SH = FxShape<PDE, KIND>;
-  constexpr int NV = SH::NA;
-  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t row = SH::theta ? id / kNear : id % m;
-  const int e = (int)(SH::theta ? id % kNear : id / m);
-  if (row >= m || e >= kNear || e >= near.count[row]) return;
-  const int64_t o = e * near.estep + row * near.rstep;
-  const int64_t j = near.idx[o];
-  double r[3], d2 = 0.0, rnx = 0.0, rny = 0.0, nn = 0.0;
-  for (int c = 0; c < 3; ++c) {
-    const double nx = tn[3 * row + c], ny = sn[3 * j + c];
-    r[c] = tc[3 * row + c] - sc[3 * j + c];
-    d2 = fma(r[c], r[c], d2);
-    rnx = fma(r[c], nx, rnx);
-    rny = fma(r[c], ny, rny);
-    nn = fma(nx, ny, nn);
-  }
-  const double d = sqrt(d2), id1 = 1.0 / d, id2 = 1.0 / d2;
-  double* v = near.val + o * NV;
-  // e^{ikd} [(1/d - ik) p + (k^2 d^2 - 3 + 3ikd) q], p = nn/d^2, q = rnx rny/d^5
-  const double w = weights[j], p = w * (nn * id2), q = w * (rnx * rny * (id2 * id2 * id1)), a = -w * (rnx * id2);
-  if constexpr (PDE == LAPLACE) {
-    if (SH::theta) v[0] = a * id1;
-    v[NV - 1] = fma(-3.0, q, p * id1);
-  } else {
-    const double kd = k * d;
-    double s, c;
-    sincos(kd, &s, &c);
-    auto put = [&](double wr, double wi, double* o) {
-      o[0] = fma(c, wr, -s * wi);
-      o[1] = fma(c, wi, s * wr);
-    };
-    if (SH::theta) put(a * id1, -k * a, v);
-    put(fma(id1, p, fma(kd, kd, -3.0) * q), fma(-k, p, 3.0 * kd * q), v + NV - 2);
+  __syncwarp();
+  const double x[3] = {x0, x1, x2}, nx[3] = {tn[3 * row], tn[3 * row + 1], tn[3 * row + 2]};
+  for (int e = lane; e < total; e += 32) {
+    const int64_t o = e * near.estep + row * near.rstep, j = near.idx[o];
+    fx_near_values<PDE, KIND>(x, nx, sc + 3 * j, sn + 3 * j, weights[j], k, near.val + o * SH::NA);
   }
 }
 
-// Scale of each target row: a bound of its kernel values.  One warp per eight
+// Scale of each target row: a bound of its kernel values.  One warp per four
 // consecutive rows, which lie close together: it takes the values of their
 // nearest tiles, then of every tile whose values may exceed one of the bounds
 // so far (|K| from the distance to the tile alone); the others add nothing to
 // the maximum.  (One thread per row left the device almost empty, 4.0 ms at
-// 13,872 rows; one warp per row read the tiles 43,200 times, 2.1 ms there.)
-constexpr int kPlanRows = 8;
+// 13,872 rows; one warp per row read the tiles 43,200 times, 2.1 ms there.
+// Eight, four and two rows per warp, Theta: 43,200 complex rows 704, 668 and
+// 1,121 us, 10,800 real rows of the derivative form 211, 165 and 124.)
+constexpr int kPlanRows = 4;
 
 template <int PDE, int KIND>
 __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __restrict__ rows,
@@ -990,6 +993,7 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
   constexpr int JL = SH::J < 32 ? SH::J : 32;  // lanes along the sources of a tile
   constexpr int RP = 32 / JL;                  // rows per pass
   constexpr int NP = kPlanRows / RP;           // passes
+  static_assert(kPlanRows % RP == 0, "whole passes");
   __shared__ double sx[8][kPlanRows][9];       // x, n_x, |n_x|, reach, cut2 of a warp's rows
   const int wid = blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (wid / (FX_M / kPlanRows) >= nrb) return;
@@ -1113,7 +1117,7 @@ __global__ void __launch_bounds__(256) fx_plan_rows(int nrb, const FxRows* __res
 // mass[stage * ncol + c]: at most the sum of |w x| (the larger part) over the
 // stage without its largest term, so that it holds for a target that is one
 // of the stage's nodes, too.
-constexpr int kMaxRun = 8;  // stages per warp
+constexpr int kMaxRun = 2;  // stages per warp (eight, one after another: 11 us at 1,728 nodes, two 5)
 
 __device__ __forceinline__ double fx_mass(double sum, double top) { return fmax(0.0, (sum - top) - 1e-14 * sum); }
 
@@ -1121,6 +1125,8 @@ template <bool CPLX>
 __global__ void fx_colmax(int nstages, const FxStage* __restrict__ stages, const double* __restrict__ w,
                           const double* __restrict__ x, int64_t ldx, int ncol, unsigned long long* colmax,
                           double* __restrict__ mass) {
+  pdl_trigger();
+  pdl_wait();
   const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int s0 = run * kMaxRun, s1 = min(nstages, s0 + kMaxRun);
   for (int c = blockIdx.y; c < ncol; c += gridDim.y) {  // (a grid dimension holds 65,535)
@@ -1224,6 +1230,8 @@ constexpr int kGuardRows = 16, kGuardGroups = FX_M / kGuardRows;
 
 template <int PDE, int KIND>
 __global__ void __launch_bounds__(256) fx_guard(FxGuard a) {
+  pdl_trigger();
+  pdl_wait();
   using SH = FxShape<PDE, KIND>;
   constexpr int NM = SH::theta ? 2 : 1, CH = 64;
   constexpr double kDown = 1.0 / 9223372036854775808.0;  // 2^-63
@@ -1364,6 +1372,8 @@ __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const d
                         const double* __restrict__ x, int64_t ldx, int c0, int ncol, int half, int nall, int nc,
                         const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
                         unsigned char* __restrict__ out, long long* __restrict__ digits) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int JT = CPLX ? 8 : 16;  // sources of a chunk
   // plane blockIdx.y: columns c0 + y * half and on
   c0 += blockIdx.y * half;
@@ -1444,6 +1454,8 @@ __global__ void fx_pack(int nstages, const FxStage* __restrict__ stages, const d
 template <bool CPLX>
 __global__ void fx_near_add(int64_t m, FxNear near, const double* __restrict__ x, int64_t ldx, double* y, int64_t ldy,
                             int c0, int ncol, double ar, double ai, const int* __restrict__ flag) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int U = 4;
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, row = min(id / 4, m - 1);
   const int f = blockIdx.y * U;
@@ -1500,6 +1512,8 @@ __global__ void fx_near_add(int64_t m, FxNear near, const double* __restrict__ x
 template <bool CPLX>
 __global__ void fx_near_theta(int64_t m, int ns, FxNear near, const double2* __restrict__ g0,
                               const double2* __restrict__ g1, double2* out, const int* __restrict__ flag) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, row = id / ns;
   const int k = (int)(id - row * ns);
   if (row >= m || *flag) return;
@@ -1533,6 +1547,8 @@ __global__ void fx_near_theta(int64_t m, int ns, FxNear near, const double2* __r
 __global__ void fx_theta_max(int nstages, const FxStage* __restrict__ stages, int ns, bool cplx,
                              const double* __restrict__ w, const double2* __restrict__ g0,
                              const double2* __restrict__ g1, unsigned long long* colmax, double* __restrict__ mass) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ unsigned long long best[32];
   if (threadIdx.x < 32) best[threadIdx.x] = 0;
   __syncthreads();
@@ -1572,6 +1588,8 @@ __global__ void fx_theta_pack(int nstages, const FxStage* __restrict__ stages, c
                               const double2* __restrict__ g0, const double2* __restrict__ g1, int ns, int nc,
                               const unsigned long long* __restrict__ colmax, const int* __restrict__ flag,
                               unsigned char* __restrict__ out, long long* __restrict__ digits) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int JT = CPLX ? 4 : 8;
   const int per = CPLX ? nc / 2 : nc;
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1671,6 +1689,8 @@ struct FxOut {
 
 template <bool CPLX>
 __global__ void __launch_bounds__(FX_M) fx_finish(FxOut o) {
+  pdl_trigger();
+  pdl_wait();
   if (*o.flag) return;
   const FxRows rb = o.rows[blockIdx.x];
   const int r = threadIdx.x, c = blockIdx.y, cg = o.c0 + c;
@@ -1725,6 +1745,8 @@ __global__ void __launch_bounds__(FX_M) fx_theta_finish(const FxRows* __restrict
                                                         const unsigned long long* __restrict__ colmax,
                                                         const long long* __restrict__ digits, int ns, int nc,
                                                         const int* __restrict__ flag, double2* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   if (*flag) return;
   const FxRows rb = rows[blockIdx.x];
   const int r = threadIdx.x, c = blockIdx.y;
@@ -1779,10 +1801,10 @@ const int* fx_flag(const inti_ctx* ctx) { return ctx->fx.work.as<int>(); }
 // 64 us here (64 columns 407 against 125 us).  Theta pays for its plan (row
 // bounds, work lists) every time, about 0.1 ms: real values break even near
 // 5e7 pairs (7,000 nodes), complex ones near 2e7.  The derivative form adds the
-// sources taken apart: real values 0.78 against 0.81 ms at 9,408 nodes and
-// 1.22 against 1.08 at 12,288, complex ones 0.59 against 0.72 at 4,800 and 1.03
-// against 0.97 at 6,912; 2,352 x 20,000 complex 2.39 against 2.54 (4,800 sources
-// 3.01 against 2.95).
+// sources taken apart: real values 0.62 against 0.65 ms at 8,112 nodes, 0.78
+// against 0.71 at 9,408, complex ones 0.59 against 0.66 at 4,800, 0.80 against
+// 0.78 at 5,808; with more targets than sources, complex values, 2,352 x 20,000
+// 2.38 both, 3,888 x 20,000 2.73 against 2.57.
 // Few sources leave little of an item next to its hand-over (and a surface's
 // last stage partly empty), while the FP64 MMA kernel's blocks are short then.
 // Ratio of its time to the time here, 8 and 64 columns, sources x targets:
@@ -1794,7 +1816,7 @@ const int* fx_flag(const inti_ctx* ctx) { return ctx->fx.work.as<int>(); }
 // and 1.42.
 bool fx_pays(int pde, int kind, double targets, double pairs) {
   if (kind < FX_THETA) return pairs >= 2e6 && pairs >= (kind == HS ? 1400.0 : 850.0) * targets;
-  if (kind == FX_THETA_D) return pairs >= (pde == HELMHOLTZ ? 4e7 : 1.2e8) && pairs >= 5000.0 * targets;
+  if (kind == FX_THETA_D) return pairs >= (pde == HELMHOLTZ ? 3.3e7 : 8.8e7) && pairs >= 3500.0 * targets;
   return pairs >= (pde == HELMHOLTZ ? 2e7 : 5e7);
 }
 
@@ -1903,10 +1925,8 @@ static void fx_plan(inti_ctx* ctx, const FxProblem& p, FxPlan& plan) {
       const int64_t m = plan.ntargets;
       fx_plan_near<P, K><<<(unsigned)((m + 7) / 8), 256, 0, ctx->stream>>>(
           m, plan.nstages, plan.stages, plan.tiles.as<double4>(), plan.records.as<double>(), p.tcoords, p.tnormals,
-          p.weights, p.k, plan.cut2.as<double>(), fx_near(p, plan));
-      fx_near_values<P, K><<<(unsigned)((m * kNear + 255) / 256), 256, 0, ctx->stream>>>(
-          m, p.tcoords, p.tnormals, p.coords, p.normals, p.weights, p.k, fx_near(p, plan));
-      ctx->launches += 2;
+          p.coords, p.normals, p.weights, p.k, plan.cut2.as<double>(), fx_near(p, plan));
+      ctx->launches++;
     }
     fx_plan_rows<P, K><<<(unsigned)plan.nrows * (FX_M / kPlanRows / 8), 256, 0, ctx->stream>>>(
         plan.nrows, plan.rows, p.tcoords, p.tnormals, plan.stages, plan.tiles.as<double4>(),
@@ -1975,7 +1995,7 @@ static void fx_guard_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, 
   a.flag = ctx->fx.work.as<int>();
   fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
     constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
-    fx_guard<P, K><<<dim3((unsigned)plan.nrows, (unsigned)((ncol + 63) / 64)), 256, 0, ctx->stream>>>(a);
+    launch_pdl(ctx->stream, dim3((unsigned)plan.nrows, (unsigned)((ncol + 63) / 64)), 256, 0, &fx_guard<P, K>, a);
   });
   ctx->launches++;
 }
@@ -2004,20 +2024,22 @@ static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc
   fx_dispatch(p.pde, p.kind, [&](auto pc, auto kc) {
     constexpr int P = decltype(pc)::value, K = decltype(kc)::value;
     if (planes == 1) {
-      fx_contract_kernel<P, K, 1>
-          <<<std::min(ctx->num_sms, plan.nitems), FX_THREADS, FxShape<P, K>::SMEM, ctx->stream>>>(a);
+      launch_pdl(ctx->stream, (unsigned)std::min(ctx->num_sms, plan.nitems), FX_THREADS, FxShape<P, K>::SMEM,
+                 &fx_contract_kernel<P, K, 1>, a);
     } else if constexpr (!FxShape<P, K>::theta) {
-      cudaLaunchAttribute attr[1];
+      cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 2;
       attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(2 * std::min(ctx->num_sms / 2, plan.nitems)));
       cfg.blockDim = dim3(FX_THREADS);
       cfg.dynamicSmemBytes = FxShape<P, K>::SMEM;
       cfg.stream = ctx->stream;
       cfg.attrs = attr;
-      cfg.numAttrs = 1;
+      cfg.numAttrs = 2;
       INTI_CUDA(cudaLaunchKernelEx(&cfg, fx_contract_kernel<P, K, 2>, a));
     }
   });
@@ -2025,6 +2047,10 @@ static void fx_run(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, int nc
   INTI_CUDA(cudaGetLastError());
 }
 
+// The kernels of a product are launched programmatically, each waiting for the
+// one before it at its start: without that the check's launch cost 10 us at
+// 1,728 nodes (8 columns, Laplace SL, back to the host: 66 us without the
+// check, 78 with it, 56 so).
 void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_csr* corr, const double* x,
               int64_t ldx, double* y, int64_t ldy, int nrhs, const double* alpha, const double* beta) {
   const bool cplx = p.pde == HELMHOLTZ;
@@ -2036,8 +2062,8 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
   auto by_type = [&](auto cc) {
     constexpr bool C = decltype(cc)::value;
     const int runs = (plan.nstages + kMaxRun - 1) / kMaxRun;
-    fx_colmax<C><<<dim3((runs + 7) / 8, std::min(nrhs, 65535)), 256, 0, ctx->stream>>>(plan.nstages, st, p.weights, x, ldx, nrhs, colmax,
-                                                                 ctx->fx.mass.as<double>());
+    launch_pdl(ctx->stream, dim3((runs + 7) / 8, std::min(nrhs, 65535)), 256, 0, &fx_colmax<C>, plan.nstages, st,
+               p.weights, x, ldx, nrhs, colmax, ctx->fx.mass.as<double>());
     ctx->launches++;
     fx_guard_run(ctx, p, plan, nrhs);
     int pass = 0;
@@ -2045,9 +2071,9 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
     for (int c0 = 0; c0 < nrhs; c0 += w.cols, ++pass) {
       w = fx_pass(nrhs - c0, comps);
       const int64_t threads = (int64_t)plan.nstages * 4 * (w.nc / comps);
-      fx_pack<C><<<dim3((unsigned)((threads + 127) / 128), w.planes), 128, 0, ctx->stream>>>(
-          plan.nstages, st, p.weights, x, ldx, c0, w.cols, w.half, nrhs, w.nc, colmax, flag,
-          ctx->fx.bdig.as<unsigned char>(), fx_digits_ptr(ctx, plan, nrhs));
+      launch_pdl(ctx->stream, dim3((unsigned)((threads + 127) / 128), w.planes), 128, 0, &fx_pack<C>, plan.nstages, st,
+                 p.weights, x, ldx, c0, w.cols, w.half, nrhs, w.nc, colmax, flag, ctx->fx.bdig.as<unsigned char>(),
+                 fx_digits_ptr(ctx, plan, nrhs));
       ctx->launches++;
       const int slot = 1 + pass % (FX_COUNTERS - 1);
       if (pass >= FX_COUNTERS - 1) INTI_CUDA(cudaMemsetAsync(flag + slot, 0, sizeof(int), ctx->stream));
@@ -2078,11 +2104,11 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
       o.br = beta ? beta[0] : 0.0;
       o.bi = beta ? beta[1] : 0.0;
       o.beta_zero = o.br == 0.0 && o.bi == 0.0;
-      fx_finish<C><<<dim3(plan.nrows, w.cols), FX_M, 0, ctx->stream>>>(o);
+      launch_pdl(ctx->stream, dim3(plan.nrows, w.cols), FX_M, 0, &fx_finish<C>, o);
       ctx->launches++;
       if (fx_near_kind(p.kind)) {
-        fx_near_add<C><<<dim3((unsigned)((plan.ntargets + 31) / 32), (unsigned)((w.cols + 3) / 4)), 128, 0,
-                         ctx->stream>>>(plan.ntargets, fx_near(p, plan), x, ldx, y, ldy, c0, w.cols, o.ar, o.ai, flag);
+        launch_pdl(ctx->stream, dim3((unsigned)((plan.ntargets + 31) / 32), (unsigned)((w.cols + 3) / 4)), 128, 0,
+                   &fx_near_add<C>, plan.ntargets, fx_near(p, plan), x, ldx, y, ldy, c0, w.cols, o.ar, o.ai, flag);
         ctx->launches++;
       }
     }

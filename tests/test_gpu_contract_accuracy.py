@@ -286,9 +286,9 @@ def test_theta_of_a_refined_surface(ctx, pde, k, derivative):
     kernel values and traces do not fit it, so every other row keeps the FP64
     kernel's bits (rows are summed apart, in chunks that depend on the number
     of 128-row blocks only); on a uniform surface the rows change theirs."""
-    limit = {(False, False): 5e7, (False, True): 2e7, (True, False): 1.2e8, (True, True): 4e7}[derivative, bool(k)]
+    limit = {(False, False): 5e7, (False, True): 2e7, (True, False): 8.8e7, (True, True): 3.3e7}[derivative, bool(k)]
     op = inti.Helmholtz(k=k, dim=3) if k else inti.Laplace(dim=3)
-    cells, nsub = {5e7: (13, 14), 2e7: (9, 10), 1.2e8: (17, 17), 4e7: (11, 12)}[limit]
+    cells, nsub = {5e7: (13, 14), 2e7: (9, 10), 8.8e7: (13, 15), 3.3e7: (11, 12)}[limit]
     for q, same in ((graded_sphere(12, cells), True), (inti.p2_sphere_quadrature(nsub), False)):
         n = len(q)
         m = int(np.ceil(limit / n)) - 1
