@@ -14,6 +14,7 @@
 
 #include "batch.h"
 #include "common.h"
+#include "contract_i8.h"
 #include "internal.h"
 
 using inti::DevBuf;
@@ -803,6 +804,7 @@ int inti_op_destroy(inti_op* op) {
   inti_ctx* ctx = op->ctx;
   return guarded(ctx, [&] {
     INTI_CUDA(cudaStreamSynchronize(ctx->stream));
+    fx_drop(ctx, op->fx);
     delete op;
   });
 }
@@ -909,6 +911,7 @@ int inti_batch_destroy(inti_batch* b) {
   inti_ctx* ctx = b->ctx;
   return guarded(ctx, [&] {
     INTI_CUDA(cudaStreamSynchronize(ctx->stream));
+    fx_drop(ctx, b->fx);
     delete b;
   });
 }

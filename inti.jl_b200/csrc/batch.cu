@@ -545,6 +545,7 @@ static void mrhs_fp64(inti_ctx* ctx, const FxProblem& p, FxPlan& plan, const int
                       bool pays, int64_t blocks) {
   if (pays && fx_prepare(ctx, p, plan, a.nrhs)) {
     const double alpha[2] = {a.ar, a.ai}, beta[2] = {a.br, a.bi};
+    fx_hold(ctx, plan);
     fx_apply(ctx, p, plan, corr, a.x, a.ldx, a.y, a.ldy, a.nrhs, alpha, beta);
     a.only_if = fx_flag(ctx);
   }

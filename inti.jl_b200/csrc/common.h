@@ -123,6 +123,7 @@ struct FxPlan {
   int nrows = 0, nitems = 0, nslots = 0, nstages = 0, nsurf = 0;
   int64_t ntargets = 0;
   bool ready = false;
+  bool held = false;  // by an operator or batch that counts in the context's users
 };
 
 }  // namespace inti
@@ -189,8 +190,11 @@ struct inti_ctx {
   // digit blocks of the densities, partial sums, [flag, counters, column
   // bounds, digit sums], and the densities' mass per stage.  Shared by the context's operators like the symmetric form's
   // partials: live only within one product, on the context's one stream.
+  // They grow to the largest product's and are given back with the last
+  // operator or batch that uses them (fx_drop).
   struct {
     inti::DevBuf tab, bdig, partial, work, mass;
+    int users = 0;
   } fx;
 };
 

@@ -1682,7 +1682,7 @@ struct FxOut {
   const double* x;
   double* y;
   int64_t ldx, ldy;
-  int c0, ncol, nall, nc, half, nslots;  // half: columns per plane
+  int c0, nall, nc, half, nslots;  // half: columns per plane
   double scale, ar, ai, br, bi;
   bool beta_zero;
 };
@@ -1794,6 +1794,19 @@ static FxConst fx_const(const FxProblem& p) {
 }
 
 const int* fx_flag(const inti_ctx* ctx) { return ctx->fx.work.as<int>(); }
+
+void fx_hold(inti_ctx* ctx, FxPlan& plan) {
+  if (plan.held) return;
+  plan.held = true;
+  ctx->fx.users++;
+}
+
+void fx_drop(inti_ctx* ctx, FxPlan& plan) {
+  if (!plan.held) return;
+  plan.held = false;
+  if (--ctx->fx.users > 0) return;
+  for (DevBuf* b : {&ctx->fx.bdig, &ctx->fx.partial, &ctx->fx.work, &ctx->fx.mass}) b->release();
+}
 
 // Where the contraction is the faster form.  Below about 2e6 pairs (1,400
 // nodes squared) the FP64 MMA kernel's single launch is as fast: 8 complex
@@ -2093,7 +2106,6 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
       o.ldx = ldx;
       o.ldy = ldy;
       o.c0 = c0;
-      o.ncol = w.cols;
       o.nall = nrhs;
       o.nc = w.nc;
       o.half = w.half;

@@ -48,5 +48,10 @@ void fx_apply(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const inti_
 void fx_theta(inti_ctx* ctx, const FxProblem& p, const FxPlan& plan, const double2* g0, const double2* g1, int ns,
               double2* out);
 const int* fx_flag(const inti_ctx* ctx);
+// An operator or batch takes part in (once) or leaves the users of the
+// context's buffers; the last one to leave, with nothing in flight on the
+// context's stream, gives them back.
+void fx_hold(inti_ctx* ctx, FxPlan& plan);
+void fx_drop(inti_ctx* ctx, FxPlan& plan);
 
 }  // namespace inti
