@@ -27,22 +27,6 @@ namespace inti {
 using cplx = std::complex<double>;
 constexpr int kSegBlock = 1024;
 
-// Warp sums of eight values, reduce-scattered: lane l returns the sum of
-// v[l >> 2] (9 shuffles instead of 40).
-__device__ __forceinline__ double seg_sum8(const double (&v)[8], int lane) {
-  double a[4], b[2];
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    a[q] = (lane & 16 ? v[q + 4] : v[q]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? v[q] : v[q + 4], 16);
-#pragma unroll
-  for (int q = 0; q < 2; ++q)
-    b[q] = (lane & 8 ? a[q + 2] : a[q]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a[q] : a[q + 2], 8);
-  double k = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
-  k += __shfl_xor_sync(0xffffffffu, k, 2);
-  k += __shfl_xor_sync(0xffffffffu, k, 1);
-  return k;
-}
-
 // h[sys*hs + k] = sum_{i in seg(s)} conj(V_k[r][i]) W[r][i], sys = s*R + r.
 // Eight vectors per sweep over W and 1,024 threads: with 256 threads, one
 // vector at a time and a block reduction each, it waited on its reductions
@@ -71,7 +55,7 @@ __global__ void __launch_bounds__(kSegBlock) seg_dots(const int64_t* off, int R,
           ay[u] = fma(v.x, w.y, fma(-v.y, w.x, ay[u]));
         }
     }
-    const double sx = seg_sum8(ax, lane), sy = seg_sum8(ay, lane);
+    const double sx = warp_sum8(ax, lane), sy = warp_sum8(ay, lane);
     if ((lane & 3) == 0) red[warp][lane >> 2] = make_double2(sx, sy);
     __syncthreads();
     if (threadIdx.x < 8 && k0 + (int)threadIdx.x < kcount) {

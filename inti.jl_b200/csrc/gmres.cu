@@ -175,22 +175,6 @@ __device__ __forceinline__ double2 load_c(const double* v, int64_t i) {
   return C ? reinterpret_cast<const double2*>(v)[i] : make_double2(v[i], 0.0);
 }
 
-// Warp sums of eight values, reduce-scattered (as warp_sum4 of the pair
-// kernels): 9 shuffles instead of 40.  Lane l returns the sum of v[l >> 2].
-__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
-  double a[4], b[2];
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    a[q] = (lane & 16 ? v[q + 4] : v[q]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? v[q] : v[q + 4], 16);
-#pragma unroll
-  for (int q = 0; q < 2; ++q)
-    b[q] = (lane & 8 ? a[q + 2] : a[q]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a[q] : a[q + 2], 8);
-  double k = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
-  k += __shfl_xor_sync(0xffffffffu, k, 2);
-  k += __shfl_xor_sync(0xffffffffu, k, 1);
-  return k;
-}
-
 // Step j of a small-system cycle, after w = sum_t coef_t A_t v_j (the shift
 // is added here, w += shift * v_j, saving a launch per step): w is orthogonalised
 // against v_0..v_j twice (CGS2; sums in a fixed order), v_{j+1} = w/|w|,
