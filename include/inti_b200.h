@@ -174,7 +174,13 @@ int inti_op_info(const inti_op* op, int64_t* m, int64_t* n, int* dtype);
  * for each product; other blocks of columns (unit vectors, narrow bumps,
  * refined surfaces, targets close to a surface) and smaller products take the
  * FP64 MMA path.  Other operators and fewer columns run one pair product per
- * column.  Results agree within those bounds (the summation order differs). */
+ * column.  Results agree within those bounds (the summation order differs).
+ * The first product on the INT8 path builds the operator's work lists and row
+ * bounds (0.1 ms at 2,000 nodes, 0.2 to 0.5 ms at 14,000), which it keeps; the
+ * digit blocks and partial sums (about 620 MB for 64 complex columns at
+ * 200,934 nodes, outside the partial budget) belong to the context, grow to the
+ * largest product's and go back with the last operator that used them; without
+ * memory for them the FP64 MMA path runs. */
 int inti_op_apply(inti_op* op, const double* x, int64_t ldx, double* y, int64_t ldy,
                   int32_t nrhs, const double* alpha, const double* beta, int on_device);
 /* Y = alpha*(A^T*X + C^T*X) + beta*Y: the transpose (not conjugate) apply,
@@ -296,7 +302,7 @@ int inti_gmres(inti_ctx* ctx, int32_t nterms, inti_op* const* ops, const double*
                double* history, inti_gmres_stats* stats);
 /* Systems of at most max_unknowns unknowns (default 8192) run each Arnoldi
  * step's orthogonalisation (both Gram-Schmidt passes), the new basis vector
- * and the Givens update in one single-CTA kernel after the operator
+ * and the Givens update in one kernel (a cluster of CTAs) after the operator
  * application, and the host checks the residual once per four steps (the
  * steps enqueued after convergence leave the iterate alone; their operator
  * applications still run and are counted); larger systems use the multi-CTA

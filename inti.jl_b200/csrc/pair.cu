@@ -1788,7 +1788,10 @@ int pair_plan_split(const inti_ctx* ctx, int pde, int kind, int dim, int precisi
 
 // Targets per thread: four, unless whole tiles then give an SM fewer than 12
 // CTAs (Laplace DL, 12,150 sources x 2,000 targets, 10 per SM: 55.4 us with
-// four, 38.6 with two; 51,894 x 1,000, 22 per SM: 70.1 and 71.2).
+// four, 38.6 with two; 51,894 x 1,000, 22 per SM: 70.1 and 71.2).  Transposes
+// of square operators take the same rule, four from about 5,400 nodes on
+// (10,800 nodes, Helmholtz DL, from host arrays: 341 -> 302 us with the slices
+// and chunks above).
 int pair_plan_tpt(const inti_ctx* ctx, int precision, int64_t m, int64_t n) {
   if (precision != INTI_FP64) return 4;
   const int64_t rows = fwd_rows(precision, 4);
