@@ -170,8 +170,8 @@ int inti_op_info(const inti_op* op, int64_t* m, int64_t* n, int* dtype);
  * 64 columns.  From 2e6 pairs, outside stream capture, the values are
  * multiplied with them as 64-bit fixed-point numbers on the INT8 tensor path
  * while every entry's error stays below n 2^-52.8 times its sum of moduli (n
- * real products; the a priori bound of an FP64 sum), which the device checks
- * for each product; other blocks of columns (unit vectors, narrow bumps,
+ * real products, |r||n| in the place of |r.n|; the a priori bound of an FP64
+ * sum), which the device checks for each product; other blocks of columns (unit vectors, narrow bumps,
  * refined surfaces, targets close to a surface) and smaller products take the
  * FP64 MMA path.  Other operators and fewer columns run one pair product per
  * column.  Results agree within those bounds (the summation order differs).

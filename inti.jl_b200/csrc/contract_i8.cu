@@ -21,7 +21,8 @@
 // is added at the end (fx_mean).  Sums carry no rounding.  What is missing is at
 // most 2^65.2 / (pa pb) per real product, whatever the product's own size: one
 // scale serves a whole row and a whole column.  fx_guard therefore measures
-// each result's sum of moduli T against that unit, and the products in which
+// each result's sum of moduli T (with |r||n| in the place of |r.n|) against that
+// unit, and the products in which
 // an entry would come out worse than n 2^-52.8 T, the a priori bound of an FP64
 // sum of n terms, are left to the FP64 kernels: unit vectors, narrow bumps,
 // densities on one part of a surface, refined surfaces, targets close to a
@@ -1213,10 +1214,11 @@ struct FxGuard {
 // order 8 of at most 2^14 each, and half a unit of either factor), so it stays
 // below n 2^-52.8 T for n products while
 //
-//     T = sum_j |K_ij| |w_j x_jc| >= 2^-8 2^126 / (pa pb)
+//     T = sum_j S_ij |w_j x_jc| >= 2^-8 2^126 / (pa pb)
 //
 // (2^63/pa and 2^63/pb lie between one and 2.1 times the largest |K_ij| and
-// |w_j x_jc|).  As terms of mean zero they come to about sqrt(n) 2^-56 T at that
+// |w_j x_jc|; S_ij is |K_ij| with |r||n| in the place of |r.n|, the size at
+// which the evaluation of r.n rounds, in any form of the product).  As terms of mean zero they come to about sqrt(n) 2^-56 T at that
 // limit.
 //
 // T is bounded from below stage by stage: the stage's mass times the kernel's
